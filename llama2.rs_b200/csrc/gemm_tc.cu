@@ -3,41 +3,47 @@
 //
 //   out[m][o] = f[m] * sum_g scale[o][g] * sum_{k in g} (q[o][k] - z[o][g]) * X[m][k]
 //
-// X[m][k] is the activation of token m as a 23-bit signed integer (three balanced base-256 digits, see
-// act_quant_kernel in prefill_kernels.cu), so every product and every sum inside a quantisation
-// group is exact integer arithmetic; f[m] carries the block exponent and the rmsnorm factor.
+// X[m][k] is the activation of token m as a 24-bit signed integer, X = 4096 hi + lo with |hi|, |lo| <= 2048 (see row_quant_kernel in
+// prefill_kernels.cu).  Both digits and q - z are small integers, exact in f16, and so are their products and the sums over a
+// quantisation group (below 2^22) in the f32 accumulators: kind::f16 MMAs do exact integer arithmetic here.  f[m] carries the block
+// exponent and the rmsnorm factor.
+// (The alternative, three 8-bit digits on kind::i8, needs 3/4 of the MMA time but a third more accumulator columns, and their way
+// from s32 columns to f32 sums (one multiply-add, two conversions, the zero-point correction) bounded the kernel at 1110 / 1770 clocks
+// per 128 rows x 64 tokens x group of 64 / 128.  Here the accumulators are f32 already and the zero point is in the operand: two FMAs
+// remain.)
 //
-// One CTA owns 128 output rows and a slice of the quantisation groups (grid.y slices).  Per group:
-//   A  128 rows x GS weights, unpacked from nibbles to unsigned bytes in shared memory (3 bit
-//      operations per 8 weights), K-major with the 128/64/32-byte swizzle the MMA unit expects;
-//   B  N = 3 digits x M tokens rows x GS signed bytes, one bulk copy from the image the quantiser
-//      wrote (already swizzled);
-//   D  128 x N s32 in tensor memory, overwritten by the first MMA of the group (GS/32 MMAs of K = 32).
+// Work.  One launch covers up to three matrices that share an input length (wq/wk/wv, w1/w3).  A tile is RT x 128 output
+// rows by up to 64 tokens; a K step is 128 inputs (1, 2 or 4 quantisation groups).  The (tile, K step) pairs of the launch
+// form one line that is cut into equal pieces, one per SM: no tail wave, and the pipeline of a CTA fills once per launch.
+// A tile that a cut goes through leaves several partial results (slices); whoever reads the output adds them in slice
+// order, which costs nothing where the reader is a kernel that walks the rows anyway (row_quant_kernel, rope_append_kernel).
+// RT = 2: two weight tiles share every digit block (32 KB per K step at 64 tokens, from the L2).
+//
+// Per K step and weight tile:
+//   A  128 rows x 128 weights as f16 q - z in TENSOR MEMORY (64 columns, lane = row): written by the loaders with tcgen05.st and read by
+//      the MMAs from there.  In shared memory the unpacked weights would cost 64 KB of write + read traffic per tile of a bandwidth
+//      of 128 bytes per clock.
+//   B  2 digits x tq tokens rows x 128 f16, one bulk copy of the block the quantiser wrote (two 128-byte-swizzled halves of 64 inputs);
+//   D  per group: 128 x 2 tq f32 in one of three tensor-memory accumulators (GS / 16 MMAs of K = 16).
+//      The way of an accumulator (MMAs, wake the drain, read, wake the issuer) takes about 1200 clocks beside the MMAs' own 256
+//      or 512: with two accumulators that chain bounded the kernel, so the A slots are one per weight tile and D has three.
 //
 // Roles (they meet only through mbarriers):
-//   warps 0-3   loaders.  A thread owns four 16-byte pieces of a group's packed weights (GS = 128): it asks for the
-//               pieces of group g + 7 (cp.async into a ring of raw slots) and unpacks those of group g into one
-//               of three A stages.
-//   warps 4-11  drain: tcgen05.ld of the finished accumulator (a warp reads the 32 tensor-memory lanes of its
-//               quadrant and half of the token columns), zero point through the tokens' digit sums, one f32 FMA
-//               per (row, token) with the scale.  The group's scales, zero points and digit sums arrive in a side
-//               ring that the drain warps fill themselves, seven groups ahead.
-//   warp 12     one thread issues the MMAs of a group into one of two accumulators and commits once: the
-//               commit frees the A and B stages and tells the drain that the accumulator is complete.
-//   warp 13     one thread keeps three B stages filled, up to three groups ahead.
-// While the drain works on group g the tensor cores work on group g + 1 and the loaders on group g + 2.  The kernel
-// is bound by instruction issue, so ring positions are carried along instead of being computed from the group
-// number, and the work is cut so that the bookkeeping of a group is paid by few warps.
-// Split K: the CTAs of a tile whose groups are divided among several (grid.y) store partial results, which
-// ksum_kernel adds in slice order (measured: letting the last CTA of a tile add them cost more than the extra launch).
-// The kernel is launched programmatically behind the activation quantiser: everything that does not read the quantiser's
-// output (set-up, tensor-memory allocation, the loaders' first requests) runs while that kernel still does.  Extending the
-// chain (slice sum behind this kernel, the next quantiser behind the slice sum) was measured slower: the early-resident
-// kernels of the next projection take issue slots and bandwidth from the one that is running (1.13 -> 1.32 ms for eight
-// 7B layers at 30 tokens).
+//   warps 0-7    loaders, four warps per weight tile: a thread turns the 128 weights of one row into f16 (per 8 weights: a shift, four
+//                and-or, four half2 operations).  Thread to row: the 8 threads of a shared-memory phase
+//                read 8 different records, whose starts lie an odd number of 16-byte units apart: no bank conflicts.
+//   warps 8-15   drain, four warps per weight tile: a warp reads the 32 tensor-memory lanes of its quadrant, 16 tokens at a time with
+//                the next 16 in flight; packed f32 FMAs.
+//                (Few warps with much work per hand-over: every wait, fence and arrival is issued by each warp of a role, and with the
+//                weights or the tokens of a tile cut over twice as many warps those outnumbered the useful instructions.)
+//   warp 16      raw weights: one bulk copy per 16-row record run (contiguous in memory), a ring as deep as shared memory allows.
+//   warp 17      digit blocks.     warp 18  one thread issues the MMAs.
+// The kernel is launched programmatically behind the quantiser: everything that does not read the quantiser's output (set-up,
+// tensor-memory allocation, weight requests) runs while that kernel still does.
 // Every wait on an mbarrier is bounded; a wait that gives up raises a flag that ends every loop.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "kernels.cuh"
@@ -46,20 +52,14 @@ namespace l2 {
 
 namespace {
 
-constexpr int TC_LOAD_WARPS = 4, TC_DRAIN_WARPS = 8;
-constexpr int TC_LOADERS = 32 * TC_LOAD_WARPS;     // 128
-constexpr int TC_DRAINERS = 32 * TC_DRAIN_WARPS;   // 256
-constexpr int TC_THREADS = TC_LOADERS + TC_DRAINERS + 64;  // + the MMA warp and the B warp: 448
-constexpr int TC_MMA_WARP = TC_LOAD_WARPS + TC_DRAIN_WARPS;
-constexpr int TC_STAGES = 3;     // A and B stages
-constexpr int TC_RING = 4;       // barrier ring of groups in flight (full / done)
-constexpr int TC_RAW = 8;        // raw ring: groups whose packed weight words are in shared memory or on their way there
-constexpr int TC_SIDE = 12;      // side ring (scales, zero points, digit sums)
-constexpr int TC_AHEAD = TC_RAW - 1;  // groups between a request and the step that makes it (both rings)
-constexpr int MAX_TOKENS = 64;   // tokens of one pass (N = 3 * tokens <= 192 columns)
-constexpr int TC_HALF = MAX_TOKENS / 2;   // tokens a drain thread holds at most
-constexpr int TC_META = 8 * 80;  // bytes of a group's scales and zero points: 20 words of each of the 8 records
-constexpr uint32_t TC_WAIT_LIMIT = 1u << 20;
+constexpr int TC_LOAD_WARPS = 8, TC_DRAIN_WARPS = 8;
+constexpr int TC_RAW_WARP = TC_LOAD_WARPS + TC_DRAIN_WARPS, TC_B_WARP = TC_RAW_WARP + 1, TC_MMA_WARP = TC_RAW_WARP + 2;
+constexpr int TC_THREADS = 640;   // the last warp has no work: register counts are set per group of four warps
+constexpr int TC_KSTEP = 128;     // inputs per K step
+constexpr int TC_B_SLOTS = 3, TC_D_SLOTS = 3, TC_MAX_RAW = 12;
+constexpr uint32_t TC_D_COLS = 128, TC_A_COL0 = 384, TC_A_COLS = 64;  // tensor memory (512 columns): three accumulators, one A slot per weight tile
+constexpr int TC_MAX_SLICES = 8;
+constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -72,96 +72,247 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-// One poll of a barrier phase with a time hint: the hardware parks the thread until the phase completes or the time has
-// passed.  A warp that polls in a tight loop instead takes issue slots and shared-memory bandwidth from the warps that
-// share its scheduler, and this kernel's warps wait a lot (measured: every role ran three to four times slower).
+// One poll of a barrier phase; the hardware parks the thread for a short time of its own choice if the phase is not complete.  (An
+// explicit time hint of 2 microseconds, or a sleep between polls, made every hand-over between roles several hundred clocks longer.)
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity), "r"(2000u) : "memory");
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-// bounded: gives up after TC_WAIT_LIMIT polls or as soon as another thread has given up.  A poll that fails is followed
-// by a short sleep: barrier polls share the shared-memory pipe with every store, copy and MMA issue of the CTA, and
-// hundreds of waiting threads polling back to back made each of those take 200 to 300 cycles (measured).
+// bounded: gives up after TC_WAIT_LIMIT polls or soon after another thread has given up
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
 #pragma unroll 1
     for (uint32_t i = 0; i < TC_WAIT_LIMIT; i++) {
         if (mbar_try_wait(bar, parity)) return true;
-        if (*failed) return false;
-        __nanosleep(40);
+        if ((i & 63) == 63 && *failed) return false;
     }
     return false;
 }
-// the same for a whole warp: lane 0 polls, the others sleep at the shuffle and then look at the barrier once themselves
-// (one successful poll each, which also orders their reads behind the arrivals)
+// the same for a whole warp (every lane polls: its reads are ordered behind the arrivals)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
-    bool ok = true;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, failed);
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    return ok && mbar_try_wait(bar, parity);
+    const bool ok = mbar_wait(bar, parity, failed);
+    return __all_sync(0xffffffffu, ok);
 }
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
 }
 __device__ __forceinline__ void commit_to(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-
-// (float)i for |i| < 2^22 without a conversion instruction: 1.5 * 2^23 + i is exact in f32
-__device__ __forceinline__ float magic_float(int i) { return __int_as_float(0x4B400000 + i) - 12582912.0f; }
-
-// K-major operand descriptor: rows of GS bytes, 8-row swizzle atoms of 8*GS bytes
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t gs) {
-    const uint64_t layout = gs == 128 ? 2 : (gs == 64 ? 4 : 6);  // SWIZZLE_128B / 64B / 32B
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)((8u * gs) >> 4) << 32) | (1ull << 46) | (layout << 61);
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
 }
-// byte offset of (row, k) inside a K-major tile with rows of gs bytes, swizzled
-__device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t kbyte, uint32_t gs) {
-    const uint32_t off = row * gs + kbyte;
-    return off ^ (((off >> 7) & ((gs >> 4) - 1)) << 4);
+// K-major operand descriptor: rows of 128 bytes, 128-byte swizzle, 8-row atoms of 1024 bytes.  Low word: start address (16-byte units)
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+// D (+)= A (tensor memory) * B (shared memory), 128 x N x 16
+template <bool ACC>
+__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc) {
+    asm volatile("{\n.reg .pred p;\n.reg .b64 db;\nsetp.ne.b32 p, %5, 0;\nmov.b64 db, {%2, %3};\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
+                 ::"r"(d), "r"(a), "r"(b_lo), "n"(UMMA_DESC_HI), "r"(idesc), "n"(ACC ? 1 : 0) : "memory");
+}
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long d) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(d));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// 8 weights of a row -> four f16 pairs q - z, inputs (0,4) (1,5) (2,6) (3,7).  0x6400 | n is 1024 + n in f16, 0x6400 | n << 4 is 1024 + 16 n;
+// c1 = -(1024 + z), c2 = -(64 + z): every step is exact.
+__device__ __forceinline__ void unpack8(uint32_t v, uint32_t c1, uint32_t c2, uint32_t* out) {
+    constexpr uint32_t LO = 0x000F000Fu, HI = 0x00F000F0u, ONE = 0x64006400u, SIXTEENTH = 0x2C002C00u;
+    const uint32_t w = v >> 8;
+    out[0] = hadd2(and_or(v, LO, ONE), c1);
+    out[1] = hfma2(and_or(v, HI, ONE), SIXTEENTH, c2);
+    out[2] = hadd2(and_or(w, LO, ONE), c1);
+    out[3] = hfma2(and_or(w, HI, ONE), SIXTEENTH, c2);
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+                   "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+                   "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Register split: the launch gives every thread 96; drain warps keep 64 tensor-memory words in flight beside 64 sums.
+// 8 warps x 80 + 8 warps x 136 + 4 warps x 40 = 60,416 of the launch's 61,440 registers.
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Bytes between record runs in shared memory: the run's records, padded so that runs start an odd number of 16-byte units apart (modulo 8)
+__host__ __device__ constexpr uint32_t tc_run_bytes(int W) { return (uint32_t)(4 / W) * (256u * W + 80u) + (W == 4 ? 0u : 16u); }
+
+// A CTA's piece of the line of (tile, K step) pairs, one tile at a time.
+struct Seg { int mat, pair, tb, k0, k1, slice; };
+struct Walk {
+    int w, w1;
+    __device__ __forceinline__ explicit Walk(const TcParams& P) : w((int)blockIdx.x * P.q), w1(min(P.total, ((int)blockIdx.x + 1) * P.q)) {}
+    __device__ __forceinline__ bool next(const TcParams& P, Seg& s) {
+        if (w >= w1) return false;
+        const int T = w / P.KS;
+        s.k0 = w - T * P.KS;
+        s.k1 = min(P.KS, s.k0 + (w1 - w));
+        s.slice = (int)blockIdx.x - (T * P.KS) / P.q;
+        int begin = 0;
+        s.mat = 0;
+        while (s.mat + 1 < P.nmat && T >= P.mat[s.mat].tile_end) begin = P.mat[s.mat++].tile_end;
+        s.pair = (T - begin) / P.ntb;
+        s.tb = (T - begin) - s.pair * P.ntb;
+        w += s.k1 - s.k0;
+        return true;
+    }
+};
+
+struct Drain {
+    uint64_t *mma_done, *acc_free;
+    volatile int* failed;
+    uint32_t tmem_base;
+    int warp, lane;
+};
+
+__device__ __forceinline__ void tmem_fetch(uint32_t (&c)[2][16], uint32_t col, int tq) {  // both digit columns of 16 tokens
+    tmem_ld16(c[0], col);
+    tmem_ld16(c[1], col + (uint32_t)tq);
+}
+// 16 tokens: scale * (4096 hi + lo), the digit sums being exact integers
+__device__ __forceinline__ void add16(const uint32_t (&c)[2][16], unsigned long long* sum, unsigned long long s2, unsigned long long k4096) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const unsigned long long hi = pack2(__uint_as_float(c[0][2 * j]), __uint_as_float(c[0][2 * j + 1]));
+        const unsigned long long lo = pack2(__uint_as_float(c[1][2 * j]), __uint_as_float(c[1][2 * j + 1]));
+        sum[j] = fma2(s2, fma2(hi, k4096, lo), sum[j]);
+    }
 }
 
-
-// the same, first with one poll by every lane (the usual case: the phase is complete or completes while the hardware parks the warp)
-__device__ __forceinline__ bool mbar_wait_fast(uint64_t* bar, uint32_t parity, volatile int* failed) {
-    if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_warp(bar, parity, failed);
+// The drain role of one warp: NT steps of 16 tokens per group.  A warp may read the 32 tensor-memory lanes of the quadrant given by its
+// index in the CTA modulo 4; the first four drain warps take the first weight tile's accumulator, the others the second's.
+template <int W, int NT>
+__device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, Walk& walk) {
+    constexpr int RT = 2, tq = 16 * NT, GPS = 4 / W;
+    constexpr uint32_t UB = 256u * W + 80u;
+    const int quad = D.warp & 3, rec16 = D.lane & 7, rr = 4 * quad + (D.lane >> 3), rt = (D.warp - TC_LOAD_WARPS) >> 2;
+    const uint32_t tquad = D.tmem_base + ((uint32_t)(32 * quad) << 16);
+    const unsigned long long k4096 = pack2(4096.0f, 4096.0f);
+    unsigned long long acc[8 * NT];                        // pairs of tokens
+    uint32_t ca[2][16], cb[2][16];                         // digit columns of a step and of the next
+    uint32_t d = rt, dph = 0;                              // accumulator of the next unit (every other unit is this warp's) and its parity
+    while (walk.w < walk.w1) {
+        Walk w0 = walk;
+        Seg sg;
+        walk.next(P, sg);
+        const TcMat& X = P.mat[sg.mat];
+        const int g0 = sg.k0 * GPS;
+        int n = min(sg.k1 * GPS, P.G) - g0;                // groups of this tile
+        // The row's scales come straight from its records in global memory (the L2 has them: the raw copies pass through it), three
+        // groups ahead.  Read from shared memory when a group was ready they cost 200 clocks of every group: the memory is busy.
+        const char* sp = reinterpret_cast<const char*>(X.rec) + ((size_t)min((sg.pair * RT + rt) * 8 + rec16, X.tiles16 - 1) * P.G + g0) * UB + 256 * W + 4 * rr;
+        auto scale = [&](int ahead) { return __ldg(reinterpret_cast<const float*>(sp + (size_t)min(ahead, n - 1) * UB)); };
+        float s_a = scale(0), s_b = scale(1), s_c = scale(2);
+#pragma unroll
+        for (int i = 0; i < 8 * NT; i++) acc[i] = 0ull;
+#pragma unroll 1
+        for (; n > 0; n--) {
+            const uint32_t tcol = tquad + d * TC_D_COLS;   // column of digit p, token t: p * tq + t
+            if (!mbar_wait_warp(D.mma_done + d, dph, D.failed)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_fetch(ca, tcol, tq);
+            const unsigned long long s2 = pack2(s_a, s_a);
+            s_a = s_b; s_b = s_c; s_c = scale(3);
+            sp += UB;
+#pragma unroll
+            for (int st = 0; st < NT; st++) {
+                tmem_wait_ld();
+                if (st + 1 < NT) {
+                    if (st & 1) tmem_fetch(ca, tcol + 16 * (st + 1), tq); else tmem_fetch(cb, tcol + 16 * (st + 1), tq);
+                } else {  // everything has been read: the accumulator is free again
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (D.lane == 0) mbar_arrive(D.acc_free + d);
+                }
+                add16(st & 1 ? cb : ca, acc + 8 * st, s2, k4096);
+            }
+            d += RT;
+            if (d >= TC_D_SLOTS) { d -= TC_D_SLOTS; dph ^= 1u; }
+        }
+        w0.next(P, sg);  // (worked out again: the coordinates would take registers from the loop above)
+        // ---- this tile's share of the output: slice 0 goes to the output rows, later slices to the part buffers
+        if (*D.failed) return false;
+        const int orow = (sg.pair * RT + rt) * 128 + rec16 * 16 + rr, m0 = sg.tb * tq;
+        const size_t ld = sg.slice == 0 ? (size_t)X.ldo : (size_t)X.rows;
+        float* dst = (sg.slice == 0 ? X.out : X.part + (size_t)(sg.slice - 1) * P.M * X.rows) + (size_t)m0 * ld + orow;
+        if (orow < X.rows) {
+#pragma unroll
+            for (int i = 0; i < 8 * NT; i++) {
+                const float2 y = unpack2(acc[i]);
+                if (m0 + 2 * i < P.M) dst[(size_t)(2 * i) * ld] = y.x * __ldg(P.osc + m0 + 2 * i);
+                if (m0 + 2 * i + 1 < P.M) dst[(size_t)(2 * i + 1) * ld] = y.y * __ldg(P.osc + m0 + 2 * i + 1);
+            }
+        }
+    }
+    return true;
 }
 
 }  // namespace
 
-template <int W>
+template <int W, int RT>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_constant__ TcParams P) {
-    constexpr uint32_t GS = 32 * W, A_BYTES = 128 * GS, RAW_BYTES = 8 * 64 * W * 4, UW = 64 * W + 20;  // UW: words per unit record
-    constexpr int ITEMS = 512 / TC_LOADERS;      // (record, half, lane) items of a group's A tile per loader thread
+    constexpr int GS = 32 * W, GPS = TC_KSTEP / GS;          // inputs per group, groups per K step
+    constexpr uint32_t UB = 256u * W + 80u;                  // bytes of a unit record
+    constexpr uint32_t RUN = tc_run_bytes(W);                // room of a record run (16 rows x one K step)
+    constexpr uint32_t RAW_BYTES = 8 * RUN;                  // raw weights of one 128-row tile and K step
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t ab_full[TC_RING], mma_done[TC_RING], acc_free[2], raw_full[TC_RAW], side_full[TC_SIDE];
+    __shared__ __align__(8) uint64_t raw_full[TC_MAX_RAW], raw_empty[TC_MAX_RAW], a_full[RT], a_empty[RT], b_full[TC_B_SLOTS], b_empty[TC_B_SLOTS], mma_done[TC_D_SLOTS], acc_free[TC_D_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int failed;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t N = P.n;
-    const int tile = blockIdx.x;                 // 128 output rows
+    const uint32_t b_bytes = 512u * (uint32_t)P.tq;           // a digit block
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t b_bytes = N * GS, sv_bytes = (uint32_t)P.mpad * 4u;
-    const uint32_t b_stage = (b_bytes + 1023) & ~1023u;
-    const uint32_t side_bytes = TC_META + sv_bytes;
-    uint8_t* stage_a = smem;                                 // [TC_STAGES][A_BYTES]
-    uint8_t* stage_b = smem + TC_STAGES * A_BYTES;           // [TC_STAGES][b_stage]
-    uint8_t* raw = stage_b + TC_STAGES * b_stage;            // [TC_RAW][8 records][64 W words]
-    uint8_t* side = raw + TC_RAW * RAW_BYTES;                // [TC_SIDE][8 records x 20 words | mpad floats]
+    uint8_t* stage_b = smem;                                  // [TC_B_SLOTS][2 halves][2 tq rows][128 bytes]
+    uint8_t* raw = stage_b + TC_B_SLOTS * b_bytes;            // [nraw][8 runs]
 
     if (tid == 0) {
-        for (int i = 0; i < TC_RING; i++) { mbar_init(&ab_full[i], TC_LOADERS + 1); mbar_init(&mma_done[i], 1); }
-        for (int i = 0; i < 2; i++) mbar_init(&acc_free[i], TC_DRAINERS);
-        for (int i = 0; i < TC_RAW; i++) mbar_init(&raw_full[i], TC_LOADERS);
-        for (int i = 0; i < TC_SIDE; i++) mbar_init(&side_full[i], TC_DRAINERS);
+        for (int i = 0; i < TC_MAX_RAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
+        for (int i = 0; i < RT; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < TC_B_SLOTS; i++) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < TC_D_SLOTS; i++) { mbar_init(&mma_done[i], 1); mbar_init(&acc_free[i], 4); }
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == TC_MMA_WARP) {  // 512 columns of tensor memory: two accumulators of up to 256 columns
+    if (warp == TC_MMA_WARP) {  // all 512 columns of tensor memory
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base_s)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -169,296 +320,253 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the kernel behind this one may set itself up
 
-    // split K: blockIdx.y takes groups [gb, gb + G) of the matrix's Gfull
-    const int Gfull = P.G;
-    const int gper = (Gfull + (int)gridDim.y - 1) / (int)gridDim.y;
-    const int gb = (int)blockIdx.y * gper;
-    const int G = min(gper, Gfull - gb);  // groups of this CTA (at least one: the host never launches empty slices)
-    const size_t img_group = (size_t)b_bytes + sv_bytes;  // a group's block of the digit image: digits, then digit sums
-
+    static_assert(RT == 2, "a tile is two weight tiles: one per group of loader and drain warps");
+    // tensor-memory lane 32 q + l of a tile is row 16 (l & 7) + 4 q + (l >> 3) of its 128 rows
+    const int quad = warp & 3, rec16 = lane & 7, rr = 4 * quad + (lane >> 3);
+    Walk walk(P);
+    Seg sg;
     if (warp < TC_LOAD_WARPS) {
+        regs_down<80>();
         // ================= loaders ==================================================================================
-        // item (record sub, half h, lane (r, t)) = W words of row 8h + r, inputs 8 (t W + j) ..; thread tid owns the items
-        // tid + 128 it: its own 16-byte piece of records sub0 + 2 it (GS = 128; smaller groups have fewer pieces, and a
-        // thread then unpacks words that another thread asked for: the barrier of the raw slot covers all of them)
-        constexpr int NW16 = 8 * 16 * W;                          // 16-byte pieces of a group's weight words
-        // A request overwrites the raw slot of an earlier group.  With GS = 128 a thread reads only pieces it asked for itself, so
-        // the slot of the group it unpacked last is free; otherwise the slot must be one that every loader warp has left: the
-        // warps are at most two groups apart (a warp passes group g only after all have delivered group g - 3).
-        constexpr int AHEAD = W == 4 ? TC_RAW - 1 : TC_RAW - 3;
-        const uint32_t* rq_w[ITEMS];
-        bool has_w[ITEMS];
-#pragma unroll
-        for (int it = 0; it < ITEMS; it++) {
-            const int piece = tid + it * TC_LOADERS;
-            has_w[it] = W == 4 || piece < NW16;
-            rq_w[it] = P.rec + ((size_t)min(tile * 8 + piece / (16 * W), P.tiles16 - 1) * Gfull + gb) * UW + (size_t)(piece % (16 * W)) * 4;  // rows beyond the matrix read the last record (results dropped)
-        }
-        const uint32_t raw_s = smem_addr(raw) + (uint32_t)tid * 16u, rawfull_s = smem_addr(&raw_full[0]);
-        int rq_g = 0;
-        uint32_t rq_raw = 0;
-        auto request = [&]() {
-            if (rq_g < G) {
-#pragma unroll
-                for (int it = 0; it < ITEMS; it++) {
-                    if (has_w[it]) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(raw_s + rq_raw * RAW_BYTES + (uint32_t)(it * TC_LOADERS * 16)), "l"(rq_w[it]) : "memory");
-                    rq_w[it] += UW;
-                }
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(rawfull_s + rq_raw * 8u) : "memory");
-            }
-            rq_g++;
-            rq_raw = (rq_raw + 1) & (TC_RAW - 1);
-        };
-        const uint8_t* up_src[ITEMS];
-        uint8_t *up_dst0[ITEMS], *up_dst1[ITEMS];
-#pragma unroll
-        for (int it = 0; it < ITEMS; it++) {
-            const int idx = tid + it * TC_LOADERS, sub = idx >> 6, hl = idx & 63, uh = hl >> 5, ur = (hl & 31) >> 2, ut = hl & 3;
-            const uint32_t arow = sub * 16 + uh * 8 + ur;
-            up_src[it] = raw + ((size_t)sub * 64 + hl) * W * 4;
-            up_dst0[it] = stage_a + (W == 4 ? arow * 128u + ((((uint32_t)ut * 2u) ^ (uint32_t)ur) << 4) : swz(arow, (uint32_t)ut * W * 8, GS));
-            up_dst1[it] = stage_a + (W == 4 ? arow * 128u + ((((uint32_t)ut * 2u + 1u) ^ (uint32_t)ur) << 4) : swz(arow, ((uint32_t)ut * W + 1) * 8, GS));
-        }
-#pragma unroll 1
-        for (int j = 0; j < AHEAD; j++) request();
+        // warps 0-3 take the first weight tile of every K step, warps 4-7 the second; a thread has a whole row of it
+        const int rt = warp >> 2;
+        const uint8_t* rec = raw + rec16 * RUN + rr * (16 * W);      // a row's words of a group follow one another
+        const uint32_t z_shift = 4 * (rr & 7);
+        const uint8_t* zeros = raw + rec16 * RUN + 256 * W + 64 + 4 * (rr >> 3);
+        const uint32_t tcol = tmem_base + ((uint32_t)(32 * quad) << 16) + TC_A_COL0 + rt * TC_A_COLS;
+        uint32_t rs = rt, rph = 0, aph = 1;  // slot and parity of the raw ring, parity of the A slot (a fresh "empty" barrier passes parity 1)
         bool ok = true;
-        uint32_t up_raw = 0, up_rawph = 0, up_a = 0;
+        while (ok && walk.next(P, sg)) {
 #pragma unroll 1
-        for (int g = 0; g < G; g++) {
-            request();  // group g + AHEAD
-            if (!mbar_wait_fast(&raw_full[up_raw], up_rawph, &failed)) { ok = false; break; }
-            // the A stage was read by the MMAs of group g - 3
-            if (g >= TC_STAGES && !mbar_wait_fast(&mma_done[(g - TC_STAGES) & (TC_RING - 1)], ((uint32_t)(g - TC_STAGES) >> 2) & 1u, &failed)) { ok = false; break; }
-            // 8 weights -> 8 bytes in the block order (0,2,4,6,1,3,5,7), the order of the digit image
-            if (W == 4) {  // two words share a 16-byte piece of the swizzled row: an item is two 16-byte stores
-                uint4 v[ITEMS];
+            for (int n = sg.k1 - sg.k0; n > 0; n--) {
+                if (!mbar_wait_warp(&raw_full[rs], rph, &failed)) { ok = false; break; }
+                const uint32_t so = rs * RAW_BYTES;
+                constexpr int PER = 4 / GPS;                     // 32-weight pieces of a group
+                uint4 v[4];
+                uint32_t z[GPS];
 #pragma unroll
-                for (int it = 0; it < ITEMS; it++) v[it] = *reinterpret_cast<const uint4*>(up_src[it] + up_raw * RAW_BYTES);
+                for (int i = 0; i < 4; i++) v[i] = *reinterpret_cast<const uint4*>(rec + so + (i / PER) * UB + (i % PER) * 16);
 #pragma unroll
-                for (int it = 0; it < ITEMS; it++) {
-                    *reinterpret_cast<uint4*>(up_dst0[it] + up_a * A_BYTES) = make_uint4(v[it].x & 0x0F0F0F0Fu, (v[it].x >> 4) & 0x0F0F0F0Fu, v[it].y & 0x0F0F0F0Fu, (v[it].y >> 4) & 0x0F0F0F0Fu);
-                    *reinterpret_cast<uint4*>(up_dst1[it] + up_a * A_BYTES) = make_uint4(v[it].z & 0x0F0F0F0Fu, (v[it].z >> 4) & 0x0F0F0F0Fu, v[it].w & 0x0F0F0F0Fu, (v[it].w >> 4) & 0x0F0F0F0Fu);
-                }
-            } else if (W == 2) {
-#pragma unroll
-                for (int it = 0; it < ITEMS; it++) {
-                    const uint2 v = *reinterpret_cast<const uint2*>(up_src[it] + up_raw * RAW_BYTES);
-                    *reinterpret_cast<uint2*>(up_dst0[it] + up_a * A_BYTES) = make_uint2(v.x & 0x0F0F0F0Fu, (v.x >> 4) & 0x0F0F0F0Fu);
-                    *reinterpret_cast<uint2*>(up_dst1[it] + up_a * A_BYTES) = make_uint2(v.y & 0x0F0F0F0Fu, (v.y >> 4) & 0x0F0F0F0Fu);
-                }
-            } else {
-#pragma unroll
-                for (int it = 0; it < ITEMS; it++) {
-                    const uint32_t v = *reinterpret_cast<const uint32_t*>(up_src[it] + up_raw * RAW_BYTES);
-                    *reinterpret_cast<uint2*>(up_dst0[it] + up_a * A_BYTES) = make_uint2(v & 0x0F0F0F0Fu, (v >> 4) & 0x0F0F0F0Fu);
-                }
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> visible to the MMA unit
-            mbar_arrive(&ab_full[g & (TC_RING - 1)]);
-            up_raw = (up_raw + 1) & (TC_RAW - 1);
-            up_rawph ^= up_raw == 0 ? 1u : 0u;
-            up_a = up_a == TC_STAGES - 1 ? 0 : up_a + 1;
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2003); }
-    } else if (warp < TC_MMA_WARP) {
-        // ================= drain warps ==================================================================================
-        // a warp may read the 32 tensor-memory lanes (= rows) of the quadrant given by its index in the CTA modulo 4;
-        // the first four drain warps take the first half of the token columns, the other four the second half
-        const int dt = tid - TC_LOADERS;                         // 0 .. 255
-        const int quad = warp & 3, half = (warp - TC_LOAD_WARPS) >> 2;
-        const int row = 32 * quad + lane;                        // row inside the 128-row tile
-        const int orow = tile * 128 + row;                       // output row
-        const bool row_ok = (orow >> 4) < P.tiles16;
-        const int tq = P.mpad / 2;                               // tokens per column half, a multiple of 8 (mpad % 16 == 0)
-        const uint32_t moff_s = (uint32_t)(row >> 4) * 20u + (uint32_t)(orow & 15), moff_z = (uint32_t)(row >> 4) * 20u + 16u + (uint32_t)((orow & 15) >> 3);
-        const uint32_t zsh = 4 * (orow & 7);
-        const uint32_t tcol = tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(half * tq);  // column of digit p, token t: p * mpad + t
-        // ---- side ring: 16-byte pieces of the 8 records' scales and zero points (40) and of the tokens' digit sums (mpad / 4)
-        // the tokens' digit sums are written by the quantiser that runs in front of this kernel; with a programmatic launch
-        // this kernel may have started before that one finished (the loaders need nothing of it): wait for it here
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        const bool has_m = dt < 40, has_s = dt >= 64 && dt < 64 + (int)(sv_bytes / 16);
-        const uint32_t* rq_m = P.rec + ((size_t)min(tile * 8 + dt / 5, P.tiles16 - 1) * Gfull + gb) * UW + 64 * W + (size_t)(dt % 5) * 4;
-        const uint8_t* rq_s = P.bimg + (size_t)gb * img_group + b_bytes + (size_t)(dt - 64) * 16;
-        const uint32_t side_dst = smem_addr(side) + (has_m ? (uint32_t)dt * 16u : TC_META + (uint32_t)(dt - 64) * 16u), sidefull_s = smem_addr(&side_full[0]);
-        int rq_g = 0;
-        uint32_t rq_side = 0;
-        auto request = [&]() {
-            if (rq_g < G) {
-                if (has_m) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(side_dst + rq_side * side_bytes), "l"(rq_m) : "memory");
-                if (has_s) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(side_dst + rq_side * side_bytes), "l"(rq_s) : "memory");
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sidefull_s + rq_side * 8u) : "memory");
-                rq_m += UW; rq_s += img_group;
-            }
-            rq_g++;
-            rq_side = rq_side == TC_SIDE - 1 ? 0 : rq_side + 1;
-        };
-        float acc[TC_HALF];
-#pragma unroll
-        for (int i = 0; i < TC_HALF; i++) acc[i] = 0.f;
-#pragma unroll 1
-        for (int j = 0; j < TC_AHEAD; j++) request();
-        bool ok = true;
-        uint32_t dr_side = 0, dr_sideph = 0;
-#pragma unroll 1
-        for (int g = 0; g < G; g++) {
-            request();  // group g + 7
-            const uint32_t b = (uint32_t)g & 1u;
-            if (!mbar_wait_fast(&side_full[dr_side], dr_sideph, &failed)) { ok = false; break; }
-            const uint32_t* meta = reinterpret_cast<const uint32_t*>(side + dr_side * side_bytes);
-            const float* sv = reinterpret_cast<const float*>(meta + TC_META / 4) + half * tq;
-            const float zf = (float)((int)((meta[moff_z] >> zsh) & 15u) + 1);  // src/gptq.rs:148
-            const float scf = row_ok ? __uint_as_float(meta[moff_s]) : 0.f;
-            const float nzs = -zf * scf;
-            if (!mbar_wait_fast(&mma_done[g & (TC_RING - 1)], ((uint32_t)g >> 2) & 1u, &failed)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tbase = tcol + b * 256u;
-#pragma unroll
-            for (int t0 = 0; t0 < TC_HALF; t0 += 16) {  // 16 tokens per step: one 16-column load per digit
-                if (t0 >= tq) break;  // warp-uniform: tq is a multiple of 8
-                uint32_t v[3][16];
-#pragma unroll
-                for (int p = 0; p < 3; p++)
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[p][0]), "=r"(v[p][1]), "=r"(v[p][2]), "=r"(v[p][3]), "=r"(v[p][4]), "=r"(v[p][5]), "=r"(v[p][6]), "=r"(v[p][7]),
-                                   "=r"(v[p][8]), "=r"(v[p][9]), "=r"(v[p][10]), "=r"(v[p][11]), "=r"(v[p][12]), "=r"(v[p][13]), "=r"(v[p][14]), "=r"(v[p][15])
-                                 : "r"(tbase + (uint32_t)(p * P.mpad + t0)) : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (t0 + 16 >= tq) {  // the last columns of this accumulator have been read: the MMAs of group g + 2 may overwrite it
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    mbar_arrive(&acc_free[b]);
-                }
-#pragma unroll
-                for (int q8 = 0; q8 < 16; q8 += 8) {
-                    if (t0 + q8 < tq) {  // warp-uniform
-#pragma unroll
-                        for (int q = q8; q < q8 + 8; q++) {
-                            // c0 2^16 + c1 2^8 + c2 (|c| < 2^18): the upper two as an integer through the conversion unit (quarter
-                            // rate, but one issue slot; rounded once to f32), the lowest through floats: an integer below 2^22 becomes
-                            // a float exactly with one integer add and one float add.  The zero point enters through the token's sum
-                            // of integers over the group (a float).
-                            const int tk = t0 + q;  // token inside this half
-                            const float fh = (float)((int)v[0][q] * 256 + (int)v[1][q]);
-                            acc[tk] = fmaf(nzs, sv[tk], fmaf(scf, fmaf(fh, 256.0f, magic_float((int)v[2][q])), acc[tk]));
-                        }
-                    }
-                }
-            }
-            dr_side = dr_side == TC_SIDE - 1 ? 0 : dr_side + 1;
-            dr_sideph ^= dr_side == 0 ? 1u : 0u;
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2002); }
-        // ---- output: out[m][orow] (+= for the residual epilogue), scaled per token; a slice of a split tile stores its part
-        //      instead ([slice][m][rows]), and ksum_kernel adds the parts in slice order
-        if (ok && !failed && row_ok && orow < P.rows) {
-            const bool split = gridDim.y > 1;
-#pragma unroll
-            for (int tk = 0; tk < TC_HALF; tk++) {
-                const int m = half * tq + tk;
-                if (tk < tq && m < P.m) {
-                    const float y = acc[tk] * __ldg(P.oscale + m);
-                    if (split) P.part[(size_t)blockIdx.y * P.kstride + (size_t)m * P.rows + orow] = y;
-                    else {
-                        float* dst = P.out + (size_t)m * P.ldo + orow;
-                        *dst = P.epi == EPI_RESID ? *dst + y : y;
-                    }
-                }
-            }
-        }
-    } else if (warp == TC_MMA_WARP) {
-        // ================= MMA issue: one thread ===================================================================
-        if (lane == 0) {
-            // instruction descriptor: D s32, A u8, B s8, both K-major, N, M = 128
-            const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-            const uint64_t desc_a0 = umma_desc(smem_addr(stage_a), GS), desc_b0 = umma_desc(smem_addr(stage_b), GS);  // stage 0, K step 0
-            uint32_t s = 0;
-#pragma unroll 1
-            for (int g = 0; g < G; g++) {
-                const uint32_t b = (uint32_t)g & 1u, ring = (uint32_t)g & (TC_RING - 1);
-                bool ok = mbar_wait(&ab_full[ring], ((uint32_t)g >> 2) & 1u, &failed);
-                if (ok && g >= 2) ok = mbar_wait(&acc_free[b], (((uint32_t)g >> 1) - 1u) & 1u, &failed);
-                if (!ok) { failed = 1; if (P.status) atomicExch(P.status, 2001); break; }
+                for (int gg = 0; gg < GPS; gg++) z[gg] = *reinterpret_cast<const uint32_t*>(zeros + so + gg * UB);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[rs]);
+                // the first half is turned into f16 before the A slot is free, the second while the first is stored
+                uint32_t a[4][16];
+                auto unpack32 = [&](int i) {
+                    const uint32_t zz = ((z[i / PER] >> z_shift) & 15u) + 1u;                                  // src/gptq.rs:148
+                    const uint32_t c1 = 0xE400E400u + zz * 0x00010001u, c2 = 0xD400D400u + zz * 0x00100010u;  // -(1024 + z), -(64 + z), twice each
+                    unpack8(v[i].x, c1, c2, a[i]); unpack8(v[i].y, c1, c2, a[i] + 4); unpack8(v[i].z, c1, c2, a[i] + 8); unpack8(v[i].w, c1, c2, a[i] + 12);
+                };
+                unpack32(0);
+                unpack32(1);
+                if (!mbar_wait_warp(&a_empty[rt], aph, &failed)) { ok = false; break; }
+                aph ^= 1u;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem_base + b * 256u;
-                const uint64_t da0 = desc_a0 + (uint64_t)(s * (A_BYTES >> 4)), db0 = desc_b0 + (uint64_t)(s * (b_stage >> 4));
-#pragma unroll
-                for (uint32_t k = 0; k < (uint32_t)W; k++) {
-                    const uint64_t da = da0 + 2 * k, db = db0 + 2 * k;  // 32 bytes further along K: the address field counts 16-byte units
-                    const uint32_t accumulate = k ? 1u : 0u;
-                    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
-                                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-                }
-                commit_to(&mma_done[ring]);  // the accumulator of group g is complete, its A and B stages may be refilled
-                s = s == TC_STAGES - 1 ? 0 : s + 1;
+                tmem_st16(tcol, a[0]);
+                tmem_st16(tcol + 16, a[1]);
+                unpack32(2);
+                tmem_st16(tcol + 32, a[2]);
+                unpack32(3);
+                tmem_st16(tcol + 48, a[3]);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_full[rt]);
+                rs += RT; if (rs >= (uint32_t)P.nraw) { rs -= P.nraw; rph ^= 1u; }
             }
         }
+        if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2003); }
+    } else if (warp < TC_RAW_WARP) {
+        regs_up<136>();
+        // ================= drain warps ==================================================================================
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // the tokens' factors (and the output buffers) belong to the kernels in front of this one
+        bool ok;
+        const Drain D{mma_done, acc_free, &failed, tmem_base, warp, lane};
+        switch (P.tq / 16) {  // one body per number of 16-token steps: with a run-time count the columns in flight change registers at every branch
+            case 1: ok = drain_tiles<W, 1>(P, D, walk); break;
+            case 2: ok = drain_tiles<W, 2>(P, D, walk); break;
+            case 3: ok = drain_tiles<W, 3>(P, D, walk); break;
+            default: ok = drain_tiles<W, 4>(P, D, walk); break;
+        }
+        if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2002); }
     } else {
-        // ================= B stages: one thread ========================================================================
+        regs_down<40>();  // one instruction for the four warps: it is a warpgroup operation
+        if (warp == TC_RAW_WARP) {
+        // ================= raw weights: lanes 0-7 copy one record run each ================================================
+        uint32_t rs = 0, rph = 1;
+        bool ok = true;
+        while (ok && walk.next(P, sg)) {
+            const TcMat& X = P.mat[sg.mat];
+            const uint8_t* base[RT];
+#pragma unroll
+            for (int rt = 0; rt < RT; rt++) {  // rows beyond the matrix read the last records (results dropped)
+                const int t16 = min((sg.pair * RT + rt) * 8 + (lane & 7), X.tiles16 - 1);
+                base[rt] = reinterpret_cast<const uint8_t*>(X.rec) + ((size_t)t16 * P.G + (size_t)sg.k0 * GPS) * UB;
+            }
+#pragma unroll 1
+            for (int k = sg.k0; k < sg.k1 && ok; k++) {
+                const uint32_t bytes = (uint32_t)min(GPS, P.G - k * GPS) * UB;
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++) {
+                    if (!mbar_wait_warp(&raw_empty[rs], rph, &failed)) { ok = false; break; }
+                    if (lane == 0) mbar_expect_tx(&raw_full[rs], 8 * bytes);
+                    __syncwarp();
+                    if (lane < 8) bulk_g2s(smem_addr(raw) + rs * RAW_BYTES + lane * RUN, base[rt], bytes, &raw_full[rs]);
+                    base[rt] += GPS * UB;
+                    if (++rs == (uint32_t)P.nraw) { rs = 0; rph ^= 1u; }
+                }
+            }
+        }
+        if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2005); }
+        } else if (warp == TC_B_WARP) {
+        // ================= digit blocks: one thread ========================================================================
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the digit image is the output of the kernel in front of this one
-            uint32_t s = 0;
-            const uint8_t* src = P.bimg + (size_t)gb * img_group;
+            uint32_t bs = 0, bph = 1;
+            bool ok = true;
+            while (ok && walk.next(P, sg)) {
+                const uint8_t* src = P.mat[sg.mat].img + ((size_t)sg.tb * P.KS + sg.k0) * b_bytes;
 #pragma unroll 1
-            for (int g = 0; g < G; g++) {
-                bool ok = true;
-                if (g >= TC_STAGES) ok = mbar_wait(&mma_done[(g - TC_STAGES) & (TC_RING - 1)], ((uint32_t)(g - TC_STAGES) >> 2) & 1u, &failed);  // the MMAs of group g - 3 have read the stage
-                if (!ok) { failed = 1; if (P.status) atomicExch(P.status, 2004); break; }
-                uint64_t* full = &ab_full[g & (TC_RING - 1)];
-                mbar_expect_tx(full, b_bytes);
-                bulk_g2s(stage_b + (size_t)s * b_stage, src, b_bytes, full);
-                src += img_group;
-                s = s == TC_STAGES - 1 ? 0 : s + 1;
+                for (int k = sg.k0; k < sg.k1; k++) {
+                    if (!mbar_wait(&b_empty[bs], bph, &failed)) { ok = false; break; }
+                    mbar_expect_tx(&b_full[bs], b_bytes);
+                    bulk_g2s(smem_addr(stage_b) + bs * b_bytes, src, b_bytes, &b_full[bs]);
+                    src += b_bytes;
+                    if (++bs == TC_B_SLOTS) { bs = 0; bph ^= 1u; }
+                }
             }
+            if (!ok) { failed = 1; if (P.status) atomicExch(P.status, 2004); }
+        }
+        } else if (warp == TC_MMA_WARP) {
+            // ================= MMA issue ===============================================================================
+            // The whole warp walks the loop and one elected lane issues: the operands of tcgen05.mma are uniform registers, and values
+            // that the compiler knows to be the same in all lanes need no move into them (inside an `if (lane == 0)` every MMA took
+            // about 90 clocks to issue, more than it takes to execute).  The tensor memory allocated is all there is: it starts at 0.
+            // Operand addresses are kept as the low words of the descriptors and advanced by constants: this warp shares its scheduler
+            // with four busy ones and every instruction between two MMAs costs it about ten clocks.
+            const bool leader = elect_one();
+            const uint32_t N = 2u * (uint32_t)P.tq;
+            // instruction descriptor: D f32, A and B f16, both K-major, N, M = 128
+            const uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+            const uint32_t b_lo0 = umma_desc_lo(smem_addr(stage_b)), slot_units = b_bytes >> 4, half_units = N * 128 / 16;
+            uint32_t aph = 0, bs = 0, bph = 0, d = 0, dph = 1;
+            bool ok = true;
+            while (ok && walk.next(P, sg)) {
+#pragma unroll 1
+                for (int k = sg.k0; k < sg.k1 && ok; k++) {
+                    const int ng = min(GPS, P.G - k * GPS);
+                    const uint32_t b_half[2] = {b_lo0 + bs * slot_units, b_lo0 + bs * slot_units + half_units};
+                    if (!mbar_wait_warp(&b_full[bs], bph, &failed)) { ok = false; break; }
+#pragma unroll
+                    for (int gg = 0; gg < GPS; gg++) {
+                        if (gg >= ng) break;
+#pragma unroll
+                        for (int rt = 0; rt < RT; rt++) {
+                            if (gg == 0 && ok) ok = mbar_wait_warp(&a_full[rt], aph, &failed);
+                            if (ok) ok = mbar_wait_warp(&acc_free[d], dph, &failed);
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            const uint32_t td = d * TC_D_COLS;
+                            if (leader) {
+#pragma unroll
+                                for (int j = 0; j < GS / 16; j++) {  // 16 inputs: 8 columns of A, 32 bytes of B
+                                    const int k0 = gg * GS + 16 * j;
+                                    if (j == 0) mma_f16<false>(td, TC_A_COL0 + rt * TC_A_COLS + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
+                                    else mma_f16<true>(td, TC_A_COL0 + rt * TC_A_COLS + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
+                                }
+                                commit_to(&mma_done[d]);
+                                if (gg == ng - 1) {
+                                    commit_to(&a_empty[rt]);
+                                    if (rt == RT - 1) commit_to(&b_empty[bs]);
+                                }
+                            }
+                            __syncwarp();
+                            if (++d == TC_D_SLOTS) { d = 0; dph ^= 1u; }
+                        }
+                        if (!ok) break;
+                    }
+                    aph ^= 1u;
+                    if (++bs == TC_B_SLOTS) { bs = 0; bph ^= 1u; }
+                }
+            }
+            if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2001); }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (failed && tid < TC_MAX_RAW + TC_B_SLOTS) {  // copies may still be on their way into this CTA's shared memory: a bounded time to land
+        uint64_t* bar = tid < TC_MAX_RAW ? &raw_full[tid] : &b_full[tid - TC_MAX_RAW];
+        for (int i = 0; i < 64; i++) { mbar_try_wait(bar, 0); mbar_try_wait(bar, 1); }
+    }
     if (warp == TC_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
 }
 
-// at least 120 KB so that only one CTA (one owner of the tensor memory) is resident per SM
-size_t gemm_tc_smem_bytes(int gs, int n) {
-    const size_t need = (size_t)TC_STAGES * ((size_t)128 * gs + (((size_t)n * gs + 1023) & ~(size_t)1023)) + (size_t)TC_RAW * 8 * 64 * (gs / 32) * 4 +
-                        (size_t)TC_SIDE * (TC_META + (size_t)n / 3 * 4) + 1024;  // digit sums: 4 bytes per token, n = 3 tokens
-    return need < 120 * 1024 ? 120 * 1024 : need;
+namespace {
+int tc_max_smem = 200 * 1024;
+size_t tc_fixed_bytes(int tq) { return 1024 + (size_t)TC_B_SLOTS * 512 * tq; }
+size_t tc_raw_bytes(int gs) { return 8 * (size_t)tc_run_bytes(gs / 32); }
+int tc_raw_slots(int gs, int tq) { return (int)std::min<size_t>(TC_MAX_RAW, (tc_max_smem - tc_fixed_bytes(tq)) / tc_raw_bytes(gs)); }
+}  // namespace
+
+void gemm_tc_tokens(int M, int* tq, int* ntb) {  // blocks of at most 64 tokens, as even as multiples of 16 allow
+    *ntb = (M + TC_MAX_TOKENS - 1) / TC_MAX_TOKENS;
+    *tq = ((M + *ntb - 1) / *ntb + 15) & ~15;
 }
 
-int gemm_tc_mpad(int tokens) { return (tokens + 15) & ~15; }
-
 size_t gemm_tc_image_bytes(int in, int gs, int tokens) {
-    const size_t mpad = (size_t)gemm_tc_mpad(tokens);
-    return (size_t)(in / gs) * (3 * mpad * gs + mpad * 4);
+    (void)gs;
+    return (size_t)((in + TC_KSTEP - 1) / TC_KSTEP) * 512 * ((tokens + TC_MAX_TOKENS - 1) / TC_MAX_TOKENS * TC_MAX_TOKENS);
+}
+
+// slices the most divided tile of a launch can have
+int gemm_tc_slices(const TcParams& p) { return p.total <= p.q ? 1 : p.q >= p.KS ? (p.q % p.KS ? 2 : 1) : (p.KS - 2) / p.q + 2; }
+
+// Fills in the geometry of a launch: p.mat[0 .. nmat) hold the matrices, p.G / p.M the groups and tokens.
+void gemm_tc_plan(TcParams& p, int gs, int sms) {
+    gemm_tc_tokens(p.M, &p.tq, &p.ntb);
+    p.gs = gs;
+    p.KS = (p.G * gs + TC_KSTEP - 1) / TC_KSTEP;
+    p.rt = 2;
+    int tiles = 0;
+    for (int i = 0; i < p.nmat; i++) {
+        tiles += (p.mat[i].tiles16 + 8 * p.rt - 1) / (8 * p.rt) * p.ntb;
+        p.mat[i].tile_end = tiles;
+    }
+    p.total = tiles * p.KS;
+    // equal pieces for the SMs, but no tile in more than TC_MAX_SLICES pieces
+    p.q = std::max((p.total + sms - 1) / sms, (p.KS + TC_MAX_SLICES - 2) / (TC_MAX_SLICES - 1));
+    p.grid = (p.total + p.q - 1) / p.q;
+    p.nraw = tc_raw_slots(gs, p.tq);
 }
 
 cudaError_t gemm_tc_init(int max_smem) {
+    tc_max_smem = max_smem;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(gemm_q4_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(gemm_q4_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(gemm_q4_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+#define L2_TC_ATTR(W, RT) if ((e = cudaFuncSetAttribute(gemm_q4_tc_kernel<W, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_max_smem)) != cudaSuccess) return e;
+    L2_TC_ATTR(4, 2) L2_TC_ATTR(2, 2) L2_TC_ATTR(1, 2)
+#undef L2_TC_ATTR
+    return cudaSuccess;
 }
 
-// Launched programmatically after the activation quantiser: set-up, tensor-memory allocation and the first weight requests
-// of this kernel overlap the quantiser's run (about a third of a short GEMM is the time to fill its pipeline); the two
-// roles that read the quantiser's output wait for it inside the kernel.
+// Launched programmatically behind the quantiser; the roles that read the quantiser's output wait for it inside the kernel.
 cudaError_t launch_gemm_tc(const TcParams& p, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
-    cfg.gridDim = dim3((p.tiles16 + 7) / 8, p.ksplit > 1 ? p.ksplit : 1);
+    cfg.gridDim = dim3(p.grid);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = gemm_tc_smem_bytes(p.gs, p.n);
+    // (always more than half of an SM: one CTA, one owner of the tensor memory, per SM)
+    cfg.dynamicSmemBytes = std::max<size_t>(120 * 1024, tc_fixed_bytes(p.tq) + (size_t)p.nraw * tc_raw_bytes(p.gs));
     cfg.stream = st;
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     g_launches++;
-    if (p.gs == 128) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<4>, p);
-    if (p.gs == 64) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<2>, p);
-    return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<1>, p);
+    if (p.gs == 128) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<4, 2>, p);
+    if (p.gs == 64) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<2, 2>, p);
+    return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<1, 2>, p);
 }
 
 }  // namespace l2

@@ -73,38 +73,69 @@ struct alignas(16) SkParams {
     int ptiles;                 // tiles the per-CTA sum buffer holds
 };
 
-// Batched QLinear on tcgen05 (gemm_tc.cu): out[m][o] for m < M tokens, 128 output rows per CTA.
-struct TcParams {
+// Batched QLinear on tcgen05 (gemm_tc.cu): out[m][o] for m < M tokens.  One launch covers up to three matrices with the same
+// input length; the output of a tile that several CTAs share is a sum of slices (see TcOut).
+constexpr int TC_MAX_TOKENS = 64;  // tokens of one token block (an accumulator holds 2 digits x 64 tokens = 128 columns)
+struct TcMat {
     const uint32_t* rec;   // unit records of the matrix (see repack.cpp)
-    const uint8_t* bimg;   // [G] blocks of [n][gs] signed digit bytes of the activations, swizzled, followed by [mpad] digit sums
-                           // per token (f32): one contiguous block per group (act_quant_kernel)
-    const float* oscale;   // [mpad] factor of the integer result per token
-    float* out;            // [M][ldo]
-    int* status;
-    int tiles16, G, gs, rows;
-    int m, mpad, n;        // tokens, tokens padded to a multiple of 16, n = 3 * mpad (three digits per token)
-    int ldo, epi;
-    int ksplit;            // > 1: the groups are split over gridDim.y CTAs; slice k stores part + k * kstride [m][rows]
-    size_t kstride;
-    float* part;
+    const uint8_t* img;    // digit image of the activations in this matrix's K order (row_quant_kernel)
+    float* out;            // [M][ldo]: slice 0
+    float* part;           // [slices - 1][M][rows]: the others
+    int tiles16, rows, ldo, tile_end;  // tile_end: tiles of the launch up to and including this matrix
 };
+struct TcParams {
+    TcMat mat[3];
+    const float* osc;      // [M] factor of the integer result per token
+    int* status;
+    int nmat, M, tq, ntb;  // tokens, tokens per block (a multiple of 16), token blocks
+    int G, gs, KS;         // groups of a row, their size, K steps of 128 inputs
+    int rt, total, q, grid;  // 128-row tiles per tile, (tile, K step) pairs of the launch, pairs per CTA, CTAs
+    int nraw;              // slots of the raw weight ring
+};
+// How the readers of a launch's output find its slices: out plus the parts of slices 1 .. n - 1, in that order.
+struct TcOut {
+    const float* out; const float* part;
+    int ldo, rows, tile0;  // tile0: tiles of the launch in front of this matrix
+    int ntb, tq, KS, q, tile_rows, M;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ int tc_slices(const TcOut& t, int m, int o) {
+    const int T = t.tile0 + (o / t.tile_rows) * t.ntb + m / t.tq;
+    return (T * t.KS + t.KS - 1) / t.q - (T * t.KS) / t.q + 1;
+}
+__device__ __forceinline__ float4 tc_load4(const TcOut& t, int m, int o) {  // o a multiple of 4
+    float4 v = *reinterpret_cast<const float4*>(t.out + (size_t)m * t.ldo + o);
+    const int n = tc_slices(t, m, o);
+    const float* p = t.part + (size_t)m * t.rows + o;
+    for (int j = 1; j < n; j++, p += (size_t)t.M * t.rows) {
+        const float4 a = *reinterpret_cast<const float4*>(p);
+        v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+    }
+    return v;
+}
+#endif
 
-struct QuantParams {
-    const float* x;        // [M][ldx] activations, natural order
-    const int* perm;       // consumer's K order (g_index) or null
-    const float* nw;       // rmsnorm weight in the consumer's K order, or null (no norm)
-    uint8_t* bimg;         // [G] blocks of [n][gs] digit bytes + [mpad] digit sums (f32)
-    float* oscale;         // [mpad]
-    int in, gs, ldx, mpad, n;
+// What row_quant_kernel makes a token's row from.
+enum : int { ROW_PLAIN = 0, ROW_RESID = 1, ROW_SWIGLU = 2 };
+struct RowParams {
+    int mode;
+    float* x;              // PLAIN: the rows; RESID: the residual stream, updated in place; [M][ldx]
+    TcOut a, b;            // RESID: a is added to x; SWIGLU: silu(a) * b
+    const float* nw;       // rmsnorm weight, natural order, or null (no norm)
     float eps;
+    int in, gs, ldx, M, tq, ntb, KS, nmat;
+    const uint16_t* perm[3];  // consumers' K orders (16-bit g_index), or null: the row is in K order
+    uint8_t* img[3];       // [token block][K step][half][2 tq][64] f16 digits, swizzled
+    float* osc;            // [M] factors
 };
 
 struct RopeParams {
-    float* q; const float* k; const float* v;   // [M][ldq], [M][ldkv]
+    TcOut q, k, v;                               // projections of the batch
+    float* qout; int ldq;                        // rotated queries
     float* kc; float* vc;                        // this layer's caches
     const float* rope_cos; const float* rope_sin;
     const int* pos;                              // [M]
-    int n_kv_heads, ldq, ldkv;
+    int n_heads, n_kv_heads;
     int kv_stride;                               // floats between cache rows of consecutive positions (all kv heads of the model); 0 = n_kv_heads * 128
 };
 
@@ -232,19 +263,20 @@ size_t sk_smem_fixed(int in, int G, int nseg, int ptiles);  // digits, group sum
 size_t sk_slot_bytes(int group_size, int chunk);           // one ring slot of one warp
 cudaError_t sk_init(int max_smem);
 void launch_embed_batch(const float* table, const int* tokens, float* x, int dim, int M, cudaStream_t st);
-void launch_act_quant(const QuantParams& p, int M, cudaStream_t st);
-void launch_rope_append(const RopeParams& p, int n_heads, int M, cudaStream_t st);
+cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st);
+cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st);
 void launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, cudaStream_t st);
 void launch_tp_gather(const TpGatherParams& p, cudaStream_t st);
-void launch_swiglu(const float* h1, const float* h3, float* hb, int n, int ld, int M, cudaStream_t st);
-// out[m][o] (+)= sum over the K slices, in slice order: finishes a GEMM whose groups were split over several CTAs
+// dst[m][ld] (+)= the output of a GEMM, slices added in order; with b: dst = silu(a) * b
+void launch_finish(const TcOut& a, const TcOut* b, float* dst, int ld, bool add, cudaStream_t st);
 cudaError_t launch_gemm_tc(const TcParams& p, cudaStream_t st);
 cudaError_t gemm_tc_init(int max_smem);
 cudaError_t attn_batch_init();
-void launch_ksum(const float* part, size_t kstride, int ksplit, float* out, int ldo, int rows, int M, int epi, cudaStream_t st);
-size_t gemm_tc_smem_bytes(int gs, int n);
-int gemm_tc_mpad(int tokens);  // tokens of a pass, padded to the granularity of the kernel's drain (16)
-size_t gemm_tc_image_bytes(int in, int gs, int tokens);  // digit image of `tokens` activations rows for a matrix with IN = in
+cudaError_t row_quant_init(int max_smem);
+void gemm_tc_plan(TcParams& p, int gs, int sms);         // geometry of a launch whose matrices, G and M are set
+int gemm_tc_slices(const TcParams& p);                   // slices the most divided tile can have
+void gemm_tc_tokens(int M, int* tq, int* ntb);           // token blocks of a batch
+size_t gemm_tc_image_bytes(int in, int gs, int tokens);  // digit image of up to `tokens` activation rows for a matrix with IN = in
 extern unsigned long long* g_sk_trace;  // device buffer for SkParams::trace when tracing is on
 void launch_attn(const AttnParams& p, cudaStream_t st, bool pdl);
 void launch_cls(const ClsParams& p, int grid, cudaStream_t st, bool pdl);

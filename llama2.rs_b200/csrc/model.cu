@@ -460,9 +460,9 @@ static TaggedLayout tagged_layout(const l2_model* m) {
     TaggedLayout t{};
     size_t at = 0;
     for (int i = 0; i < 12; i++) { t.off[i] = at; t.n[i] = n[i]; at += (n[i] * 8 + 255) & ~(size_t)255; }
-    if (m->tp_world > 1) {  // batched forward: the vectors every rank needs in full (plain f32 rows of MAX_BATCH tokens) and the exchange counters
+    if (m->tp_world > 1) {  // batched forward: the vectors every rank needs in full (plain f32 rows of one token block) and the exchange counters
         const size_t bn[3] = {D, D, H};  // x, att, hb
-        for (int i = 0; i < 3; i++) { t.batch_off[i] = at; at += (MAX_BATCH * bn[i] * 4 + 255) & ~(size_t)255; }
+        for (int i = 0; i < 3; i++) { t.batch_off[i] = at; at += (TC_MAX_TOKENS * bn[i] * 4 + 255) & ~(size_t)255; }
         t.flag_off = at; at += 256;
     }
     t.total = at;
@@ -908,6 +908,7 @@ extern "C" void l2_model_close(l2_model* m) {
         if (m->tp_peers[r] && r != m->tp_rank && !m->tp_peer_borrowed[r]) cudaIpcCloseMemHandle(m->tp_peers[r]);
     if (m->tp_pool) cudaFree(m->tp_pool);
     tp_disconnect(m);
+    free_batch(m);
     free_allocs(m->allocs);
     if (m->own_stream) cudaStreamDestroy(m->own_stream);
     delete m;
@@ -1076,18 +1077,6 @@ extern "C" void l2_state_free(l2_state* s) {
     for (auto& g : s->graphs) if (g) cudaGraphExecDestroy(g);
     free_allocs(s->allocs);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
-    if (s->batch) {
-        if (s->batch->h_stage) cudaFreeHost(s->batch->h_stage);
-        for (int i = 0; i < 2; i++) {
-            if (s->batch->aux[i]) cudaStreamDestroy(s->batch->aux[i]);
-            if (s->batch->join[i]) cudaEventDestroy(s->batch->join[i]);
-        }
-        if (s->batch->fork) cudaEventDestroy(s->batch->fork);
-        for (auto& row : s->batch->graph)
-            for (cudaGraphExec_t g : row)
-                if (g) cudaGraphExecDestroy(g);
-        delete s->batch;
-    }
     if (s->m->gen_state == s) s->m->gen_state = nullptr;
     if (s->m->tp_pool_owner == s) s->m->tp_pool_owner = nullptr;
     delete s;
@@ -1121,7 +1110,7 @@ extern "C" int l2_forward(l2_model* m, l2_state* s, const int32_t* tokens, const
     clear_error();
     if (int rc = check_state(m, s, "l2_forward")) return rc;
     const l2_config& c = m->shape.c;
-    const int maxb = m->opt.max_batch > 0 ? std::min(m->opt.max_batch, (int)MAX_BATCH) : (int)MAX_BATCH;
+    const int maxb = m->opt.max_batch > 0 ? std::min(m->opt.max_batch, (int)CALL_BATCH) : (int)CALL_BATCH;
     if (!tokens || !pos || B < 1 || B > maxb) return fail(L2_EINVAL, "l2_forward: bad batch (B=%d, max %d)", B, maxb);
     for (int b = 0; b < B; b++) {
         if (pos[b] < 0 || pos[b] >= c.seq_len) return fail(L2_ERANGE, "l2_forward: position %d outside 0..%d", pos[b], c.seq_len - 1);
@@ -1152,8 +1141,8 @@ static int prefill_async(l2_model* m, l2_state* s, const int32_t* prompt, int n_
     if (int rc = upload_prompt(s, prompt, n_prompt)) return rc;
     // Positions the reference's ladder 64/32/16/8/4/2 covers (src/inference.rs:24, 78-127): the B=1 loop
     // must start where it starts there.  How those positions are cut into batches does not change the
-    // cache ("should lead to identical results", src/inference.rs:12-15), so they go in batches of up to
-    // MAX_BATCH rows.
+    // cache ("should lead to identical results", src/inference.rs:12-15), so they go in even batches of up to
+    // MAX_BATCH rows (every batch is a pass over the weights).
     static const int ladder[6] = {64, 32, 16, 8, 4, 2};
     int target = 0;
     if (chunk > 0) { while (target + chunk < n_prompt) target += chunk; }
@@ -1165,7 +1154,8 @@ static int prefill_async(l2_model* m, l2_state* s, const int32_t* prompt, int n_
         // stores into the peers' pools) and this state is the one that works in the pool; otherwise one position at a time
         if (m->tp_direct && !m->tp_pool_owner) m->tp_pool_owner = s;
         const bool batched = m->tp_world == 1 || (m->tp_direct && token_path(s));
-        const int A = batched ? std::min<int>(MAX_BATCH, target - pos) : 1;
+        const int left = target - pos, passes = (left + batch_limit(m) - 1) / batch_limit(m);
+        const int A = batched ? (left + passes - 1) / passes : 1;
         for (int i = 0; i < A; i++) {
             tokens[i] = pos == 0 ? L2_START : prompt[pos - 1];  // src/inference.rs:29-35
             positions[i] = pos++;
@@ -1483,14 +1473,21 @@ static int qlinear_reserve(l2_qlinear* h, int B) {
     if (B <= h->cap_b) return L2_OK;
     int rc;
     if ((rc = dev_alloc(reinterpret_cast<void**>(&h->x_dev), sizeof(float) * h->q.in * B, h->allocs))) return rc;
-    if ((rc = dev_alloc(reinterpret_cast<void**>(&h->xp_dev), sizeof(float) * h->q.in * B, h->allocs))) return rc;
+    if ((rc = dev_alloc(reinterpret_cast<void**>(&h->xp_dev), sizeof(float) * h->q.in, h->allocs))) return rc;
     if ((rc = dev_alloc(reinterpret_cast<void**>(&h->y_dev), sizeof(float) * h->q.out * B, h->allocs))) return rc;
-    if (!h->img) {  // buffers of the batched (tcgen05) path, one chunk of MAX_BATCH tokens
-        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->img), gemm_tc_image_bytes(h->q.in, h->q.gs, MAX_BATCH), h->allocs))) return rc;
-        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->osc), sizeof(float) * MAX_BATCH, h->allocs))) return rc;
-        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->kpart), sizeof(float) * 4 * MAX_BATCH * h->q.out, h->allocs))) return rc;
-        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->status), sizeof(int), h->allocs))) return rc;
-        L2_CUDA(cudaMemset(h->status, 0, sizeof(int)));
+    if (B >= 2) {  // buffers of the batched (tcgen05) path
+        const int cap = B <= TC_MAX_TOKENS ? TC_MAX_TOKENS : (int)MAX_BATCH;
+        if (cap > h->cap_tc) {
+            const int rows[1] = {h->q.out};
+            if ((rc = dev_alloc(reinterpret_cast<void**>(&h->img), gemm_tc_image_bytes(h->q.in, h->q.gs, cap), h->allocs))) return rc;
+            if ((rc = dev_alloc(reinterpret_cast<void**>(&h->osc), sizeof(float) * cap, h->allocs))) return rc;
+            if ((rc = dev_alloc(reinterpret_cast<void**>(&h->kpart), sizeof(float) * part_floats(rows, 1, h->q.in, h->q.gs, cap, h->sms), h->allocs))) return rc;
+            h->cap_tc = cap;
+        }
+        if (!h->status) {
+            if ((rc = dev_alloc(reinterpret_cast<void**>(&h->status), sizeof(int), h->allocs))) return rc;
+            L2_CUDA(cudaMemset(h->status, 0, sizeof(int)));
+        }
     }
     h->cap_b = B;
     return L2_OK;
@@ -1505,16 +1502,12 @@ extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* x
     if (B >= 2) {  // batched: tensor-core GEMM, MAX_BATCH tokens at a time
         for (int b0 = 0; b0 < B; b0 += MAX_BATCH) {
             const int M = std::min<int>(MAX_BATCH, B - b0);
-            if (int rc = gemm_batched(h->q, x_dev + (size_t)b0 * h->q.in, h->q.in, true, nullptr, 0.f, M, h->img, h->osc,
-                                      xout_dev + (size_t)b0 * h->q.out, h->q.out, EPI_STORE, h->status, st, h->kpart, h->sms)) return rc;
+            if (int rc = gemm_batched(h->q, x_dev + (size_t)b0 * h->q.in, M, h->img, h->osc, xout_dev + (size_t)b0 * h->q.out, h->kpart, h->status, h->sms, st)) return rc;
         }
         return L2_OK;
     }
-    for (int b = 0; b < B; b++) {
-        launch_permute(x_dev + (size_t)b * h->q.in, h->q.perm, h->xp_dev + (size_t)b * h->q.in, h->q.in, st);
-        if (int rc = run_gemv_single(h->q, h->xp_dev + (size_t)b * h->q.in, xout_dev + (size_t)b * h->q.out, h->sms, h->d_plan, st)) return rc;
-    }
-    return L2_OK;
+    launch_permute(x_dev, h->q.perm, h->xp_dev, h->q.in, st);
+    return run_gemv_single(h->q, h->xp_dev, xout_dev, h->sms, h->d_plan, st);
 }
 
 extern "C" int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B) {

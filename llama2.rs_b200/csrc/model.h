@@ -46,24 +46,24 @@ struct DevLayer {
 
 constexpr int CTL_RING = 128;
 constexpr int L2_MAX_TP = 8;   // ranks of a tensor-parallel group (the GPUs of one box)
-constexpr int MAX_BATCH = 64;  // tokens of one batched forward (one tcgen05 accumulator holds 3 digits x 64 tokens = 192 columns)
+constexpr int CALL_BATCH = 64;  // largest B of l2_forward
+constexpr int MAX_BATCH = 512;  // tokens of one batched forward of a long prompt: one pass over the weights each
+constexpr int BATCH_RING = 16;
 
 // Device buffers of the batched forward pass (transformer<B>, B >= 2).
 struct BatchBuffers {
-    float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *h1 = nullptr, *h3 = nullptr, *hb = nullptr;
-    float* kpart[3] = {nullptr, nullptr, nullptr};  // [4][tokens][rows] partial results of GEMMs whose groups are split over CTAs, one per stream
-    uint8_t* img[3] = {nullptr, nullptr, nullptr};  // digit images (with the digit sums) of up to three consumers
-    float* osc[3] = {nullptr, nullptr, nullptr};
-    int *tok = nullptr, *pos = nullptr;             // device token ids / positions of the batch
-    int* h_stage = nullptr;                         // pinned ring for their upload
+    int cap = 0;                                            // tokens they hold
+    float *x = nullptr, *att = nullptr, *hb = nullptr;      // residual stream, attention output; SwiGLU output (tensor parallel only)
+    float* q = nullptr;                                     // rotated queries
+    float *y = nullptr, *part = nullptr;                    // output of a GEMM: slice 0 and the other slices
+    uint8_t* img[3] = {nullptr, nullptr, nullptr};          // digit images of up to three consumers
+    float* osc = nullptr;
+    int* tok = nullptr;                                     // token ids of the batch, then its positions
+    int* h_stage = nullptr;                                 // pinned ring for their upload
     int stage_slot = 0;
-    // independent projections of a layer (wq/wk/wv, w1/w3) run side by side on two more streams
-    cudaStream_t aux[2] = {nullptr, nullptr};
-    cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
-    bool tp = false;          // tensor parallel over peer memory: x, att and hb live in the model's pool, the other buffers hold this rank's columns
+    bool tp = false;          // tensor parallel over peer memory: x, att and hb live in the model's pool, y and q hold this rank's columns
     unsigned* tp_done = nullptr;  // completion counter of the gather kernel
-    cudaGraphExec_t graph[2][MAX_BATCH + 1] = {};  // the pass as a CUDA graph, per (short / long context, batch size)
-    int graph_nodes[2][MAX_BATCH + 1] = {};
+    std::vector<void*> allocs;
 };
 
 enum GraphKind : int { G_DECODE = 0, G_FEED, G_FWD_CLS, G_FWD, G_COUNT };
@@ -87,6 +87,7 @@ struct l2_model {
     uint64_t decode_bytes = 0;
     size_t device_bytes = 0;
     l2_state* gen_state = nullptr;  // reused by l2_generate_ids
+    l2::BatchBuffers* batch = nullptr;  // activations of the batched forward, allocated on first use
     bool use_graph = true, use_pdl = true;
     bool use_token_kernel = true;    // B=1 forward as one persistent kernel (single GPU only)
     int tp_rank = 0, tp_world = 1;   // tensor parallelism: this process owns 1/tp_world of every matrix's rows
@@ -120,7 +121,6 @@ struct l2_state {
     int failed_status = 0;              // device status of a launch that gave up; cleared by l2_state_reset
     std::vector<l2::SkLaunch> plans;     // [layer][4] GEMV launches, planned once
     l2::SkParams* d_plans = nullptr;     // their parameter records on the device
-    l2::BatchBuffers* batch = nullptr;   // activations of the batched forward, allocated on first use
     l2::PhaseRec* d_phases[l2::G_COUNT] = {nullptr, nullptr, nullptr, nullptr};  // phase tables of the token kernel
     int n_phases[l2::G_COUNT] = {0, 0, 0, 0};
     l2::TokenParams tk{};                // ring geometry and barrier of the token kernel
@@ -147,9 +147,9 @@ struct l2_qlinear {
     l2::SkParams* d_plan = nullptr;
     uint8_t* img = nullptr;   // batched path: digit image with the digit sums, and the factors
     float* osc = nullptr;
-    float* kpart = nullptr;   // [4][MAX_BATCH][out] partial results when the groups of a tile are split over CTAs
+    float* kpart = nullptr;   // slices of the output beyond the first
     int* status = nullptr;
-    int cap_b = 0;
+    int cap_b = 0, cap_tc = 0;  // batch sizes the buffers hold
     cudaStream_t stream = nullptr;
     std::vector<void*> allocs;
 };
@@ -169,8 +169,10 @@ struct NcclId { char bytes[128]; };  // ncclUniqueId
 int tp_all_gather(l2_model* m, float* buf, size_t count, cudaStream_t st);
 void tp_disconnect(l2_model* m);
 void tp_rows(int total_rows, int rank, int world, int* row0, int* nrows);
-int gemm_batched(const DevQ& q, const float* x, int ldx, bool gather, const float* nw, float eps, int M, uint8_t* img, float* osc,
-                 float* out, int ldo, int epi, int* status, cudaStream_t st, float* kpart = nullptr, int sms = 148, int side_tiles = 0);
+int gemm_batched(const DevQ& q, const float* x, int M, uint8_t* img, float* osc, float* out, float* part, int* status, int sms, cudaStream_t st);
+size_t part_floats(const int* rows, int n, int in, int gs, int cap, int sms);
+void free_batch(l2_model* m);
+inline int batch_limit(const l2_model* m) { return m->tp_world > 1 ? TC_MAX_TOKENS : MAX_BATCH; }  // tokens of one batched forward (the ranks' pools hold one token block)
 int dev_alloc_bytes(void** p, size_t bytes, std::vector<void*>& allocs);
 void sk_set_matrix(SkJob& j, int seg, const DevQ& q, const float* x, const float* nw);
 }  // namespace l2

@@ -1,5 +1,5 @@
 // Host side of the batched forward pass transformer<B>, B >= 2 (src/models.rs:178-298): the
-// sequence of launches for a chunk of M <= 64 tokens.  Every QLinear is a tcgen05 GEMM on exact
+// sequence of launches for a batch of tokens.  Every QLinear is a tcgen05 GEMM on exact
 // integer digits of the activations (gemm_tc.cu); no logits are produced, as in the reference.
 #include <cstring>
 
@@ -13,102 +13,123 @@ int dev_alloc_bytes(void** p, size_t bytes, std::vector<void*>& allocs) {
     return L2_OK;
 }
 
-// out[m][:] = QLinear(x[m][:]) for m < M.  gather: x is in natural order and is brought into the
-// matrix's K order through its g_index; nw (K order) folds an rmsnorm in.
-int gemm_batched(const DevQ& q, const float* x, int ldx, bool gather, const float* nw, float eps, int M, uint8_t* img,
-                 float* osc, float* out, int ldo, int epi, int* status, cudaStream_t st, float* kpart, int sms, int side_tiles) {
-    const int mpad = gemm_tc_mpad(M);
-    QuantParams a{};
-    a.x = x; a.perm = gather ? q.perm : nullptr; a.nw = nw;
-    a.bimg = img; a.oscale = osc;
-    a.in = q.in; a.gs = q.gs; a.ldx = ldx; a.mpad = mpad; a.n = 3 * mpad; a.eps = eps;
-    launch_act_quant(a, M, st);
+void tc_set_matrix(TcParams& t, int i, const DevQ& q, const uint8_t* img, float* out, int ldo, float* part) {
+    TcMat& m = t.mat[i];
+    m.rec = q.rec; m.img = img; m.out = out; m.part = part;
+    m.tiles16 = q.tiles; m.rows = q.out; m.ldo = ldo;
+    t.G = q.G;
+}
+
+TcOut tc_out(const TcParams& t, int i) {
+    TcOut o{};
+    o.out = t.mat[i].out; o.part = t.mat[i].part; o.ldo = t.mat[i].ldo; o.rows = t.mat[i].rows;
+    o.tile0 = i ? t.mat[i - 1].tile_end : 0;
+    o.ntb = t.ntb; o.tq = t.tq; o.KS = t.KS; o.q = t.q; o.tile_rows = 128 * t.rt; o.M = t.M;
+    return o;
+}
+
+static RowParams row_params(int mode, int in, int gs, const TcParams& t) {
+    RowParams r{};
+    r.mode = mode; r.in = in; r.gs = gs; r.M = t.M; r.tq = t.tq; r.ntb = t.ntb; r.KS = t.KS;
+    return r;
+}
+
+// out[m][:] = QLinear(x[m][:]) for m < M, x in natural order.  part: room for (slices - 1) * M * rows floats (qlinear_part_floats).
+int gemm_batched(const DevQ& q, const float* x, int M, uint8_t* img, float* osc, float* out, float* part, int* status, int sms, cudaStream_t st) {
     TcParams t{};
-    t.rec = q.rec; t.bimg = img; t.oscale = osc; t.out = out; t.status = status;
-    t.tiles16 = q.tiles; t.G = q.G; t.gs = q.gs; t.rows = q.out;
-    t.m = M; t.mpad = mpad; t.n = 3 * mpad; t.ldo = ldo; t.epi = epi;
-    // A matrix with few 128-row tiles would leave most SMs idle: its groups are split over several CTAs
-    // per tile, which store partial results that a small kernel adds up in slice order.
-    // (side_tiles: 128-row tiles of the GEMMs that run side by side with this one on other streams)
-    const int tiles128 = (q.tiles + 7) / 8;
-    int ks = 1;
-    if (kpart) {  // cost in group times: waves x (groups per CTA + about four to fill the CTA's pipeline) + about five for the sum kernel
-        long best = -1;
-        for (int k = 1; k <= 4 && k * 4 <= q.G; k++) {
-            const long waves = ((long)(tiles128 + side_tiles) * k + sms - 1) / sms;
-            const long cost = waves * ((q.G + k - 1) / k + 4) + (k > 1 ? 5 : 0);
-            if (best < 0 || cost < best) { best = cost; ks = k; }
-        }
-    }
-    if (ks > 1) {
-        t.ksplit = ks;
-        t.kstride = (size_t)M * q.out;
-        t.part = kpart;
-    }
+    t.nmat = 1; t.M = M; t.osc = osc; t.status = status;
+    tc_set_matrix(t, 0, q, img, out, q.out, part);
+    gemm_tc_plan(t, q.gs, sms);
+    RowParams r = row_params(ROW_PLAIN, q.in, q.gs, t);
+    r.x = const_cast<float*>(x); r.ldx = q.in; r.nmat = 1; r.perm[0] = q.perm16; r.img[0] = img; r.osc = osc;
+    L2_CUDA(launch_row_quant(r, sms, st));
     L2_CUDA(launch_gemm_tc(t, st));
-    if (ks > 1) launch_ksum(kpart, t.kstride, ks, out, ldo, q.out, M, epi, st);
+    if (gemm_tc_slices(t) > 1) launch_finish(tc_out(t, 0), nullptr, out, q.out, false, st);
     return L2_OK;
 }
 
-static int ensure_batch(l2_state* s) {
-    if (s->batch) return L2_OK;
-    l2_model* m = s->m;
+// Floats of part buffer that launches of up to `cap` tokens over matrices of rows[0 .. n) rows (inputs: in) need.
+size_t part_floats(const int* rows, int n, int in, int gs, int cap, int sms) {
+    size_t most = 0, total_rows = 0;
+    for (int i = 0; i < n; i++) total_rows += rows[i];
+    for (int M = 2; M <= cap; M++) {
+        TcParams t{};
+        t.nmat = n; t.M = M; t.G = in / gs;
+        for (int i = 0; i < n; i++) t.mat[i].tiles16 = (rows[i] + 15) / 16;
+        gemm_tc_plan(t, gs, sms);
+        most = std::max(most, (size_t)(gemm_tc_slices(t) - 1) * M * total_rows);
+    }
+    return most;
+}
+
+void free_batch(l2_model* m) {
+    BatchBuffers* b = m->batch;
+    if (!b) return;
+    for (void* p : b->allocs) cudaFree(p);
+    if (b->h_stage) cudaFreeHost(b->h_stage);
+    delete b;
+    m->batch = nullptr;
+}
+
+// The batched forward's buffers belong to the model: its calls run one after another on one stream and every call that uses
+// them ends synchronised, so all run states share them.  They grow once, from the size of a short batch to that of a long one.
+static int ensure_batch(l2_model* m, int M) {
+    const bool tp = m->tp_world > 1;
+    const int cap = M <= TC_MAX_TOKENS || tp ? TC_MAX_TOKENS : MAX_BATCH;
+    if (m->batch && m->batch->cap >= cap) return L2_OK;
+    if (m->batch) {
+        L2_CUDA(cudaStreamSynchronize(m->stream));
+        free_batch(m);
+    }
     const l2_config& c = m->shape.c;
-    const size_t B = MAX_BATCH, D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim;
-    const size_t kmax = std::max(D, H);
-    BatchBuffers* b = new BatchBuffers;
-    int rc = 0;
-    auto F = [&](float** p, size_t n) { return dev_alloc_bytes(reinterpret_cast<void**>(p), n * sizeof(float), s->allocs); };
-    // Tensor parallel over peer memory: the vectors that every rank needs in full (x, the attention output, the SwiGLU
-    // output) live in the model's pool, where the peers store their columns; q, k, v, h1, h3 hold this rank's columns only.
-    b->tp = m->tp_world > 1;
-    const size_t T = b->tp ? (size_t)m->tp_world : 1;
-    if (b->tp) {
-        if (!m->tp_direct || !m->tp_pool) { delete b; return fail(L2_EINVAL, "batched forward under tensor parallelism needs the peers' pools attached"); }
-        if (!m->tp_pool_owner) m->tp_pool_owner = s;
-        if (m->tp_pool_owner != s) { delete b; return fail(L2_EINVAL, "batched forward under tensor parallelism: another run state of this model works in the pool"); }
+    const int T = m->tp_world, D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim, Dl = D / T, KVl = KV / T, Hl = H / T, gs = c.group_size;
+    BatchBuffers* b = m->batch = new BatchBuffers;
+    b->cap = cap; b->tp = tp;
+    const int qkv[3] = {Dl, KVl, KVl}, w13[2] = {Hl, Hl}, one[1] = {Dl};
+    const size_t parts = std::max(std::max(part_floats(qkv, 3, D, gs, cap, m->sms), part_floats(w13, 2, D, gs, cap, m->sms)),
+                                  std::max(part_floats(one, 1, D, gs, cap, m->sms), part_floats(one, 1, H, gs, cap, m->sms)));
+    const size_t B = cap, outs = std::max<size_t>((size_t)Dl + 2 * KVl, 2 * (size_t)Hl);
+    // one allocation, cut into pieces of whole 256-byte lines
+    size_t total = 0;
+    auto room = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t x = tp ? 0 : room(B * D * 4), att = tp ? 0 : room(B * D * 4), q = room(B * Dl * 4), y = room(B * outs * 4), part = room(parts * 4), osc = room(B * 4);
+    const size_t img0 = room(gemm_tc_image_bytes(std::max(D, H), gs, cap)), img1 = room(gemm_tc_image_bytes(D, gs, cap)), img2 = room(gemm_tc_image_bytes(D, gs, cap));
+    const size_t tok = room(2 * B * sizeof(int)), done = room(256);
+    char* base = nullptr;
+    if (int rc = dev_alloc_bytes(reinterpret_cast<void**>(&base), total, b->allocs)) { free_batch(m); return rc; }
+    auto at = [&](size_t off) { return reinterpret_cast<float*>(base + off); };
+    b->x = at(x); b->att = at(att); b->q = at(q); b->y = at(y); b->part = at(part); b->osc = at(osc);
+    b->img[0] = reinterpret_cast<uint8_t*>(base + img0); b->img[1] = reinterpret_cast<uint8_t*>(base + img1); b->img[2] = reinterpret_cast<uint8_t*>(base + img2);
+    b->tok = reinterpret_cast<int*>(base + tok);
+    if (tp) {  // the vectors every rank needs in full live in the model's pool, where the peers store their columns
         b->x = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[0]);
         b->att = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[1]);
         b->hb = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[2]);
-        if ((rc = dev_alloc_bytes(reinterpret_cast<void**>(&b->tp_done), 256, s->allocs))) { delete b; return rc; }
-        L2_CUDA(cudaMemset(b->tp_done, 0, 256));
-    } else if ((rc = F(&b->x, B * D)) || (rc = F(&b->att, B * D)) || (rc = F(&b->hb, B * H))) { delete b; return rc; }
-    if ((rc = F(&b->q, B * D / T)) || (rc = F(&b->k, B * KV / T)) || (rc = F(&b->v, B * KV / T)) ||
-        (rc = F(&b->h1, B * H / T)) || (rc = F(&b->h3, B * H / T)) ||
-        (rc = F(&b->kpart[0], 4 * B * kmax)) || (rc = F(&b->kpart[1], 4 * B * kmax)) || (rc = F(&b->kpart[2], 4 * B * kmax))) { delete b; return rc; }
-    for (int i = 0; i < 3; i++) {
-        const size_t img_bytes = gemm_tc_image_bytes((int)kmax, c.group_size, (int)B);
-        if ((rc = dev_alloc_bytes(reinterpret_cast<void**>(&b->img[i]), img_bytes, s->allocs)) ||
-            (rc = F(&b->osc[i], B))) { delete b; return rc; }
-        L2_CUDA(cudaMemset(b->img[i], 0, img_bytes));
+        b->tp_done = reinterpret_cast<unsigned*>(base + done);
+        if (cudaMemset(b->tp_done, 0, 256) != cudaSuccess) { free_batch(m); return fail(L2_ECUDA, "cudaMemset failed"); }
     }
-    if ((rc = dev_alloc_bytes(reinterpret_cast<void**>(&b->tok), B * sizeof(int), s->allocs)) ||
-        (rc = dev_alloc_bytes(reinterpret_cast<void**>(&b->pos), B * sizeof(int), s->allocs))) { delete b; return rc; }
-    if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), sizeof(int) * 2 * B * CTL_RING) != cudaSuccess) { delete b; return fail(L2_ECUDA, "cudaMallocHost failed"); }
-    for (int i = 0; i < 2; i++) {
-        L2_CUDA(cudaStreamCreateWithFlags(&b->aux[i], cudaStreamNonBlocking));
-        L2_CUDA(cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming));
-    }
-    L2_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-    s->batch = b;
+    if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), sizeof(int) * 2 * B * BATCH_RING) != cudaSuccess) { free_batch(m); return fail(L2_ECUDA, "cudaMallocHost failed"); }
     return L2_OK;
 }
 
-// The kernels of one batched forward of M tokens (their ids and positions already in b->tok / b->pos), enqueued on `st`
-// and, for the projections that run side by side, on the two auxiliary streams forked from it and joined back.
+// The kernels of one batched forward of M tokens (their ids and positions already at b->tok), enqueued on `st`: per layer
+//   row_quant -> wq/wk/wv -> rope_append -> attention -> row_quant -> wo -> row_quant (+ residual) -> w1/w3 -> row_quant (SwiGLU) -> w2
+// each launched programmatically behind the one before it.  The GEMMs leave slices of their outputs and the kernels behind them
+// add those up while they read them.
 static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st) {
     l2_model* m = s->m;
     const l2_config& c = m->shape.c;
-    BatchBuffers* b = s->batch;
-    const int D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim;
+    BatchBuffers* b = m->batch;
+    const int D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim, gs = c.group_size;
     // this rank's share (everything on one GPU): rows of wq / wo (= heads), of wk / wv (= kv heads), of w1 / w3 / w2's inputs
     const int T = b->tp ? m->tp_world : 1, R = b->tp ? m->tp_rank : 0;
     const int Dl = D / T, KVl = KV / T, Hl = H / T, heads_l = c.n_heads / T, kvh_l = c.n_kv_heads / T;
     int* status = &s->ctl->status;
+    const int* tok = b->tok;
+    const int* pos = b->tok + M;
     // After a stage whose result every rank needs in full, this rank's columns go to the peers (stores over NVLink into their
     // pools) and the peers' columns are waited for: the same data flow as the tagged exchanges of the token kernel.  The
-    // exchanges are numbered by a counter on the device (every rank makes the same exchanges in the same order), so that
-    // the launch parameters do not change from call to call and the pass can be replayed as a CUDA graph.
+    // exchanges are numbered by a counter on the device (every rank makes the same exchanges in the same order).
     auto gather = [&](int which, int ld, int col0, int ncols) {
         if (!b->tp) return;
         TpGatherParams g{};
@@ -117,95 +138,110 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
         g.done = b->tp_done; g.status = status; g.rank = R; g.world = T; g.M = M; g.ld = ld; g.col0 = col0; g.ncols = ncols;
         launch_tp_gather(g, st);
     };
-    launch_embed_batch(m->tok_emb, b->tok, b->x, D, M, st);  // src/models.rs:189-191 (every rank holds the table: no exchange)
+    // the four launches of a layer differ from layer to layer in their matrices only
+    auto launch = [&](std::initializer_list<const DevQ*> mats, TcParams& t) {
+        t = TcParams{};
+        t.nmat = (int)mats.size(); t.M = M; t.osc = b->osc; t.status = status;
+        float *y = b->y, *part = b->part;
+        int i = 0;
+        for (const DevQ* q : mats) {
+            tc_set_matrix(t, i, *q, b->img[i], y, q->out, part);
+            y += (size_t)M * q->out;
+            i++;
+        }
+        gemm_tc_plan(t, gs, m->sms);
+        const size_t extra = (size_t)(gemm_tc_slices(t) - 1) * M;
+        for (i = 0; i < t.nmat; i++) { t.mat[i].part = part; part += extra * t.mat[i].rows; }
+    };
+    auto quant = [&](RowParams r, std::initializer_list<const DevQ*> mats, bool permuted) {
+        int i = 0;
+        for (const DevQ* q : mats) { r.perm[i] = permuted ? q->perm16 : nullptr; r.img[i] = b->img[i]; i++; }
+        r.nmat = i; r.osc = b->osc; r.eps = m->eps;
+        return launch_row_quant(r, m->sms, st);
+    };
+    launch_embed_batch(m->tok_emb, tok, b->x, D, M, st);  // src/models.rs:189-191 (every rank holds the table: no exchange)
     const size_t ls = (size_t)c.seq_len * KV;
+    TcParams t{};
+    TcOut resid{};          // output of the GEMM whose result has not been added to x yet
+    bool pending = false;
     for (int l = 0; l < c.n_layers; l++) {
         const DevLayer& y = m->layers[l];
-        int rc;
-        // rmsnorm + wq/wk/wv (:217-226): three independent GEMMs, side by side on three streams
-        L2_CUDA(cudaEventRecord(b->fork, st));
-        L2_CUDA(cudaStreamWaitEvent(b->aux[0], b->fork, 0));
-        L2_CUDA(cudaStreamWaitEvent(b->aux[1], b->fork, 0));
-        if ((rc = gemm_batched(y.wq, b->x, D, true, y.nw_q, m->eps, M, b->img[0], b->osc[0], b->q, Dl, EPI_STORE, status, st, b->kpart[0], m->sms, (y.wk.tiles + 7) / 8 + (y.wv.tiles + 7) / 8))) return rc;
-        if ((rc = gemm_batched(y.wk, b->x, D, true, y.nw_k, m->eps, M, b->img[1], b->osc[1], b->k, KVl, EPI_STORE, status, b->aux[0], b->kpart[1], m->sms, (y.wq.tiles + 7) / 8 + (y.wv.tiles + 7) / 8))) return rc;
-        if ((rc = gemm_batched(y.wv, b->x, D, true, y.nw_v, m->eps, M, b->img[2], b->osc[2], b->v, KVl, EPI_STORE, status, b->aux[1], b->kpart[2], m->sms, (y.wq.tiles + 7) / 8 + (y.wk.tiles + 7) / 8))) return rc;
-        for (int i = 0; i < 2; i++) {
-            L2_CUDA(cudaEventRecord(b->join[i], b->aux[i]));
-            L2_CUDA(cudaStreamWaitEvent(st, b->join[i], 0));
-        }
+        auto with_x = [&](const float* nw) {
+            RowParams r = row_params(pending ? ROW_RESID : ROW_PLAIN, D, gs, t);
+            r.x = b->x; r.ldx = D; r.a = resid; r.nw = nw;
+            pending = false;
+            return r;
+        };
+        // a residual projection: on one GPU the next row_quant adds it to x; under tensor parallelism it updates this rank's columns of x
+        auto add_to_x = [&](const DevQ& q) {
+            resid = tc_out(t, 0);
+            if (b->tp) { launch_finish(resid, nullptr, b->x + q.row0, D, true, st); gather(0, D, q.row0, q.out); }
+            else pending = true;
+        };
+        // rmsnorm + wq/wk/wv (:217-226)
+        launch({&y.wq, &y.wk, &y.wv}, t);
+        L2_CUDA(quant(with_x(y.rms_att), {&y.wq, &y.wk, &y.wv}, true));
+        L2_CUDA(launch_gemm_tc(t, st));
         // rope, all rows into the cache (this rank's kv heads of the full-width cache rows), then attention (:228-256)
         RopeParams r{};
-        r.q = b->q; r.k = b->k; r.v = b->v;
+        r.q = tc_out(t, 0); r.k = tc_out(t, 1); r.v = tc_out(t, 2);
+        r.qout = b->q; r.ldq = Dl;
         r.kc = s->kc + (size_t)l * ls + (size_t)R * KVl; r.vc = s->vc + (size_t)l * ls + (size_t)R * KVl;
-        r.rope_cos = m->rope_cos; r.rope_sin = m->rope_sin; r.pos = b->pos;
-        r.n_kv_heads = kvh_l; r.ldq = Dl; r.ldkv = KVl; r.kv_stride = KV;
-        launch_rope_append(r, heads_l, M, st);
+        r.rope_cos = m->rope_cos; r.rope_sin = m->rope_sin; r.pos = pos;
+        r.n_heads = heads_l; r.n_kv_heads = kvh_l; r.kv_stride = KV;
+        L2_CUDA(launch_rope_append(r, M, st));
         AttnBatchParams a{};
-        a.q = b->q; a.kc = r.kc; a.vc = r.vc; a.pos = b->pos; a.out = b->att + (size_t)R * Dl;
+        a.q = b->q; a.kc = r.kc; a.vc = r.vc; a.pos = pos; a.out = b->att + (size_t)R * Dl;
         a.n_kv_heads = kvh_l; a.ag = m->shape.attn_groups(); a.ldq = Dl; a.ldo = D; a.kv_stride = KV;
         launch_attn_batch(a, heads_l, M, long_context, st);
         gather(1, D, R * Dl, Dl);
-        // wo + residual (:260-264): this rank's rows of wo update its columns of x
-        if ((rc = gemm_batched(y.wo, b->att, D, true, nullptr, m->eps, M, b->img[0], b->osc[0], b->x + y.wo.row0, D, EPI_RESID, status, st, b->kpart[0], m->sms, 0))) return rc;
-        gather(0, D, y.wo.row0, y.wo.out);
+        // wo + residual (:260-264)
+        launch({&y.wo}, t);
+        RowParams ra = row_params(ROW_PLAIN, D, gs, t);
+        ra.x = b->att; ra.ldx = D;
+        L2_CUDA(quant(ra, {&y.wo}, true));
+        L2_CUDA(launch_gemm_tc(t, st));
+        add_to_x(y.wo);
         // rmsnorm + w1/w3 + SwiGLU (:266-276); their rows are stored in w2's K order
-        L2_CUDA(cudaEventRecord(b->fork, st));
-        L2_CUDA(cudaStreamWaitEvent(b->aux[0], b->fork, 0));
-        if ((rc = gemm_batched(y.w1, b->x, D, true, y.nw_1, m->eps, M, b->img[0], b->osc[0], b->h1, Hl, EPI_STORE, status, st, b->kpart[0], m->sms, (y.w3.tiles + 7) / 8))) return rc;
-        if ((rc = gemm_batched(y.w3, b->x, D, true, y.nw_3, m->eps, M, b->img[1], b->osc[1], b->h3, Hl, EPI_STORE, status, b->aux[0], b->kpart[1], m->sms, (y.w1.tiles + 7) / 8))) return rc;
-        L2_CUDA(cudaEventRecord(b->join[0], b->aux[0]));
-        L2_CUDA(cudaStreamWaitEvent(st, b->join[0], 0));
-        launch_swiglu(b->h1, b->h3, b->hb + y.w1.row0, Hl, H, M, st);
-        gather(2, H, y.w1.row0, y.w1.out);
+        launch({&y.w1, &y.w3}, t);
+        L2_CUDA(quant(with_x(y.rms_ffn), {&y.w1, &y.w3}, true));
+        L2_CUDA(launch_gemm_tc(t, st));
+        const TcOut h1 = tc_out(t, 0), h3 = tc_out(t, 1);
         // w2 + residual (:279-285)
-        if ((rc = gemm_batched(y.w2, b->hb, H, false, nullptr, m->eps, M, b->img[0], b->osc[0], b->x + y.w2.row0, D, EPI_RESID, status, st, b->kpart[0], m->sms, 0))) return rc;
-        gather(0, D, y.w2.row0, y.w2.out);
+        launch({&y.w2}, t);
+        RowParams rh = row_params(b->tp ? ROW_PLAIN : ROW_SWIGLU, H, gs, t);
+        rh.a = h1; rh.b = h3; rh.x = b->hb; rh.ldx = H;
+        if (b->tp) { launch_finish(h1, &h3, b->hb + y.w1.row0, H, false, st); gather(2, H, y.w1.row0, y.w1.out); }
+        L2_CUDA(quant(rh, {&y.w2}, false));
+        L2_CUDA(launch_gemm_tc(t, st));
+        add_to_x(y.w2);
+        (void)Hl;
     }
     L2_CUDA(cudaGetLastError());
     return L2_OK;
 }
 
-// One batched forward.  The ids and positions travel through a pinned ring; the kernels of the pass (about 25 per layer,
-// most of them a few microseconds long: launched one by one the host cannot keep up with the GPU) are captured once per
-// batch size into a CUDA graph and replayed.
+// One batched forward.  The ids and positions travel through a pinned ring.
 int forward_batch(l2_state* s, int M, const int32_t* tokens, const int32_t* pos) {
-    if (int rc = ensure_batch(s)) return rc;
     l2_model* m = s->m;
-    BatchBuffers* b = s->batch;
+    if (m->tp_world > 1) {
+        if (!m->tp_direct || !m->tp_pool) return fail(L2_EINVAL, "batched forward under tensor parallelism needs the peers' pools attached");
+        if (!m->tp_pool_owner) m->tp_pool_owner = s;
+        if (m->tp_pool_owner != s) return fail(L2_EINVAL, "batched forward under tensor parallelism: another run state of this model works in the pool");
+    }
+    if (M < 1 || M > batch_limit(m)) return fail(L2_EINVAL, "forward_batch: %d tokens", M);
+    if (int rc = ensure_batch(m, M)) return rc;
+    BatchBuffers* b = m->batch;
     cudaStream_t st = m->stream;
-    if (M < 1 || M > MAX_BATCH) return fail(L2_EINVAL, "forward_batch: %d tokens", M);
     // token ids and positions: own pinned slot per call until the copy has run
-    if (++b->stage_slot >= CTL_RING) { L2_CUDA(cudaStreamSynchronize(st)); b->stage_slot = 0; }
-    int* hs = b->h_stage + (size_t)b->stage_slot * 2 * MAX_BATCH;
+    if (++b->stage_slot >= BATCH_RING) { L2_CUDA(cudaStreamSynchronize(st)); b->stage_slot = 0; }
+    int* hs = b->h_stage + (size_t)b->stage_slot * 2 * b->cap;
     memcpy(hs, tokens, sizeof(int) * M);
-    memcpy(hs + MAX_BATCH, pos, sizeof(int) * M);
-    L2_CUDA(cudaMemcpyAsync(b->tok, hs, sizeof(int) * M, cudaMemcpyHostToDevice, st));
-    L2_CUDA(cudaMemcpyAsync(b->pos, hs + MAX_BATCH, sizeof(int) * M, cudaMemcpyHostToDevice, st));
-    // two graphs per batch size: the attention kernel differs between short and long contexts
+    memcpy(hs + M, pos, sizeof(int) * M);
+    L2_CUDA(cudaMemcpyAsync(b->tok, hs, sizeof(int) * 2 * M, cudaMemcpyHostToDevice, st));
     int last = 0;
     for (int i = 0; i < M; i++) last = std::max(last, (int)pos[i]);
-    const int lc = last >= 192 ? 1 : 0;
-    if (!m->use_graph) return enqueue_batch(s, M, lc != 0, st);
-    if (!b->graph[lc][M]) {
-        cudaStream_t cap;
-        L2_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-        const unsigned long long before = g_launches;
-        L2_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        const int rc = enqueue_batch(s, M, lc != 0, cap);
-        cudaGraph_t graph = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(cap, &graph);
-        b->graph_nodes[lc][M] = (int)(g_launches - before);
-        g_launches = before;  // captured launches have not run
-        cudaStreamDestroy(cap);
-        if (rc != L2_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
-        if (e != cudaSuccess) return fail(L2_ECUDA, "batched forward: graph capture failed: %s", cudaGetErrorString(e));
-        const cudaError_t e2 = cudaGraphInstantiate(&b->graph[lc][M], graph, 0);
-        cudaGraphDestroy(graph);
-        if (e2 != cudaSuccess) { b->graph[lc][M] = nullptr; return fail(L2_ECUDA, "batched forward: graph instantiate failed: %s", cudaGetErrorString(e2)); }
-    }
-    L2_CUDA(cudaGraphLaunch(b->graph[lc][M], st));
-    g_launches += b->graph_nodes[lc][M];
-    return L2_OK;
+    return enqueue_batch(s, M, last >= 192, st);
 }
 
 }  // namespace l2

@@ -1,6 +1,8 @@
 // Kernels of the batched forward pass transformer<B>, B >= 2 (src/models.rs:178-298), around the
-// tcgen05 GEMM of gemm_tc.cu: embedding rows, activation quantiser (rmsnorm folded in), RoPE +
-// cache append, causal attention over the cache, SwiGLU.  One CTA per token (and head).
+// tcgen05 GEMM of gemm_tc.cu: embedding rows, row quantiser (adds the slices of the GEMM in front of it, residual add or SwiGLU,
+// rmsnorm folded in), RoPE + cache append, causal attention over the cache.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -16,9 +18,14 @@ __device__ __forceinline__ float warp_sum_f(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t kbyte, uint32_t gs) {
-    const uint32_t off = row * gs + kbyte;
-    return off ^ (((off >> 7) & ((gs >> 4) - 1)) << 4);
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t peer_smem(const void* p, uint32_t rank) {  // the same shared-memory location of another CTA of the cluster
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 }  // namespace
@@ -26,179 +33,159 @@ __device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t kbyte, uint32_t g
 // ---- x[m] = token_embedding_table[tokens[m]] (src/models.rs:189-191) ---------------------------
 __global__ void embed_batch_kernel(const float* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int dim) {
     const int m = blockIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const float4* src = reinterpret_cast<const float4*>(table + (size_t)tokens[m] * dim);
     float4* dst = reinterpret_cast<float4*>(x + (size_t)m * dim);
     for (int i = threadIdx.x; i < dim / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// ---- activation quantiser ---------------------------------------------------------------------
-// Token m of x (natural order) is gathered into the consumer's K order, multiplied by the rmsnorm
-// weight (linearity: the 1/sqrt(mean(x^2)+eps) factor goes into oscale), scaled by a power of two
-// so that |X| <= 2^22 (23 of the 24 bits of an f32 mantissa for the token's largest element) and written
-// as three balanced base-256 digits (-128..127 each) into the K-major, swizzled byte image the GEMM
-// copies into shared memory: row digit * mpad + m (most significant digit first), inside a block of
-// 8 inputs the order (0,2,4,6,1,3,5,7) in which a weight word separates into nibbles.
-constexpr int AQ_THREADS = 256;
-constexpr int AQ_CACHE = 2;        // rounds of a CTA's own slice kept in registers between the two passes
+// ---- row quantiser ---------------------------------------------------------------------------------
+// One token's row per cluster of CTAs.  The row is made first: a plain buffer, or the residual stream plus the output of the
+// GEMM in front (its slices added in order, x updated in place), or silu(h1) * h3 of two GEMM outputs.  Every CTA makes its
+// share, multiplies by the rmsnorm weight (linearity: the 1/sqrt(mean(x^2)+eps) factor goes into osc) and puts it into the shared
+// memory of all CTAs of the cluster, with its part of the statistics; then every CTA cuts its share of each consumer's K order into
+// digits, gathering from shared memory.  So the row is read once and the statistics (the same for every K order) are taken
+// once, for up to three consumers.
+//
+// Digits: X = round(x * nw * 2^(22 - E)) with E the exponent of the row's largest |x * nw|, so |X| <= 2^23 (the 24 bits of an f32
+// mantissa for the largest element), X = 4096 hi + lo with hi in -2048..2048 and lo in -2048..2047, both exact in f16.  They go into the
+// K-major, 128-byte-swizzled blocks the GEMM copies into shared memory: per K step two halves of 64 inputs, row digit * tq + token,
+// inside a block of 8 inputs the order (0,4,1,5,2,6,3,7) in which a weight word separates into f16 pairs.
+constexpr int RQ_THREADS = 256;
+constexpr int RQ_MAX_CLUSTER = 8;
 
-__global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const __grid_constant__ QuantParams P) {
-    __shared__ float red[2 * (AQ_THREADS / 32) + 2];
-    // the GEMM behind this kernel is launched programmatically: it may start now (its loaders need nothing from here) and
-    // waits inside for this grid to finish before it reads the image
+__global__ void __launch_bounds__(RQ_THREADS) row_quant_kernel(const __grid_constant__ RowParams P) {
+    extern __shared__ __align__(16) float xs[];  // the row (times the norm weight), natural order
+    __shared__ float red[2][RQ_THREADS / 32];
+    __shared__ float stat[RQ_MAX_CLUSTER][2];    // (largest |x nw|, sum of x^2) of every CTA's share
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const float* x = P.x + (size_t)m * P.ldx;
-    const int nblk = P.in / 8;
-    const uint32_t gs = P.gs, lanes_per_group = gs / 8;
-    auto fetch = [&](int blk, float (&v)[8], float& sq) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int k = blk * 8 + j;
-            const float xv = x[P.perm ? P.perm[k] : k];
-            sq += xv * xv;
-            v[j] = P.nw ? xv * P.nw[k] : xv;
-        }
-    };
-    // The row is cut into gridDim.y slices of whole groups; every slice's CTA takes the statistics of the whole row (the
-    // row is 16 to 112 KB and sits in the L2) and writes the digits of its own slice.  It walks the row starting at its
-    // slice and keeps what it fetched there (AQ_CACHE rounds), so its slice is gathered once.
-    const int G = P.in / (int)gs, S = (int)gridDim.y, slice = (int)blockIdx.y;
-    const int b0 = (slice * G / S) * (int)lanes_per_group, nslice = ((slice + 1) * G / S) * (int)lanes_per_group - b0;
-    float cache[AQ_CACHE][8];
+    const int C = (int)gridDim.x, r = (int)cluster_rank(), m = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (C > 1) cluster_barrier();  // every CTA of the cluster has started: its shared memory may be written
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int n4 = P.in / 4, i0 = (int)((long long)n4 * r / C), i1 = (int)((long long)n4 * (r + 1) / C);
     float mx = 0.f, sq = 0.f;
-    const int rounds = (nblk + AQ_THREADS - 1) / AQ_THREADS;
-#pragma unroll
-    for (int k = 0; k < AQ_CACHE; k++) {
-        const int idx = tid + k * AQ_THREADS;
-        if (idx < nblk) {
-            fetch(b0 + idx < nblk ? b0 + idx : b0 + idx - nblk, cache[k], sq);
-#pragma unroll
-            for (int j = 0; j < 8; j++) mx = fmaxf(mx, fabsf(cache[k][j]));
+    for (int i = i0 + tid; i < i1; i += RQ_THREADS) {
+        float4 v;
+        if (P.mode == ROW_SWIGLU) {  // src/models.rs:92-98
+            const float4 a = tc_load4(P.a, m, i * 4), b = tc_load4(P.b, m, i * 4);
+            v.x = (a.x * (1.0f / (1.0f + expf(-a.x)))) * b.x; v.y = (a.y * (1.0f / (1.0f + expf(-a.y)))) * b.y;
+            v.z = (a.z * (1.0f / (1.0f + expf(-a.z)))) * b.z; v.w = (a.w * (1.0f / (1.0f + expf(-a.w)))) * b.w;
+        } else {
+            float4* xp = reinterpret_cast<float4*>(P.x + (size_t)m * P.ldx) + i;
+            v = *xp;
+            if (P.mode == ROW_RESID) {  // src/models.rs:47-51
+                const float4 a = tc_load4(P.a, m, i * 4);
+                v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+                *xp = v;
+            }
         }
-    }
-    for (int k = AQ_CACHE; k < rounds; k++) {
-        const int idx = tid + k * AQ_THREADS;
-        if (idx >= nblk) break;
-        float v[8];
-        fetch(b0 + idx < nblk ? b0 + idx : b0 + idx - nblk, v, sq);
-#pragma unroll
-        for (int j = 0; j < 8; j++) mx = fmaxf(mx, fabsf(v[j]));
+        sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        if (P.nw) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(P.nw) + i);
+            v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
+        }
+        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        reinterpret_cast<float4*>(xs)[i] = v;
+        for (int c = 0; c < C; c++)
+            if (c != r)
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(peer_smem(xs + 4 * i, c)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         sq += __shfl_xor_sync(0xffffffffu, sq, o);
     }
-    if (lane == 0) { red[warp] = mx; red[AQ_THREADS / 32 + warp] = sq; }
+    if (lane == 0) { red[0][warp] = mx; red[1][warp] = sq; }
     __syncthreads();
-    if (tid == 0) {
+    if (tid < C) {  // thread c delivers this CTA's statistics to CTA c
         float a = 0.f, b = 0.f;
-        for (int w = 0; w < AQ_THREADS / 32; w++) { a = fmaxf(a, red[w]); b += red[AQ_THREADS / 32 + w]; }
-        red[2 * (AQ_THREADS / 32)] = a;
-        red[2 * (AQ_THREADS / 32) + 1] = b;
+        for (int w = 0; w < RQ_THREADS / 32; w++) { a = fmaxf(a, red[0][w]); b += red[1][w]; }
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" ::"r"(peer_smem(&stat[r][0], tid)), "f"(a), "f"(b) : "memory");
     }
-    __syncthreads();
-    mx = red[2 * (AQ_THREADS / 32)];
-    const float total = red[2 * (AQ_THREADS / 32) + 1];
+    if (C > 1) cluster_barrier(); else __syncthreads();
+    float total = 0.f;
+    mx = 0.f;
+    for (int c = 0; c < C; c++) { mx = fmaxf(mx, stat[c][0]); total += stat[c][1]; }
     const float rs = P.nw ? 1.0f / sqrtf(total / (float)P.in + P.eps) : 1.0f;  // src/models.rs:58-60
     int e = 0;
-    // |x| * scale < 2^22: three balanced digits reach from -0x808080 to 0x7F7F7F, a little short of 2^23
-    if (mx > 0.f && mx < INFINITY) e = 21 - (int)((__float_as_uint(mx) >> 23) & 255u) + 127;
+    if (mx > 0.f && mx < INFINITY) e = 22 - (int)((__float_as_uint(mx) >> 23) & 255u) + 127;  // |x| * scale < 2^23
     e = max(-100, min(100, e));
     const float scale = __uint_as_float((uint32_t)(127 + e) << 23);
-    if (tid == 0 && slice == 0) P.oscale[m] = rs / scale;
+    if (tid == 0 && r == 0) P.osc[m] = rs / scale;
 
-    const size_t img_group = (size_t)P.n * gs + (size_t)P.mpad * 4;  // bytes of one group's block: the digit image, then the tokens' digit sums
-    const int erounds = (nslice + AQ_THREADS - 1) / AQ_THREADS;
+    const size_t blk_bytes = (size_t)512 * P.tq;
+    const int tb = m / P.tq, t = m - tb * P.tq;
+    const int b0 = (int)((long long)P.KS * r / C) * 16, b1 = min(P.in / 8, (int)((long long)P.KS * (r + 1) / C) * 16);  // blocks of 8 inputs, whole K steps
 #pragma unroll 1
-    for (int k = 0; k < erounds; k++) {
-        const int idx = tid + k * AQ_THREADS;
-        if ((idx & ~31) >= nslice) break;  // warp-uniform
-        const bool valid = idx < nslice;   // a group is 4 to 16 adjacent lanes and nslice a multiple of that: valid for all lanes of a group or none
-        const int blk = b0 + idx;
-        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (valid) {
-            static_assert(AQ_CACHE == 2, "the rounds kept in registers are picked by name");
-            if (k == 0) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = cache[0][j];
-            } else if (k == 1) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = cache[1][j];
-            } else {
-                float dummy = 0.f;
-                fetch(blk, v, dummy);
+    for (int j = 0; j < P.nmat; j++) {
+        uint8_t* img = P.img[j] + (size_t)tb * P.KS * blk_bytes;
+        const uint4* perm = reinterpret_cast<const uint4*>(P.perm[j]);
+#pragma unroll 1
+        for (int base = b0; base < b1; base += RQ_THREADS) {
+            const int blk = base + tid;
+            if (blk >= b1) break;
+            float v[8];
+            {
+                if (perm) {
+                    const uint4 ix = __ldg(perm + blk);
+                    v[0] = xs[ix.x & 0xFFFFu]; v[1] = xs[ix.x >> 16]; v[2] = xs[ix.y & 0xFFFFu]; v[3] = xs[ix.y >> 16];
+                    v[4] = xs[ix.z & 0xFFFFu]; v[5] = xs[ix.z >> 16]; v[6] = xs[ix.w & 0xFFFFu]; v[7] = xs[ix.w >> 16];
+                } else {
+                    const float4 a = reinterpret_cast<const float4*>(xs)[2 * blk], b = reinterpret_cast<const float4*>(xs)[2 * blk + 1];
+                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                }
             }
-        }
-        uint32_t E[8];  // per element: bytes d2, d1, d0 (least significant digit first), balanced: X = d0 2^16 + d1 2^8 + d2, d in -128..127
+            uint32_t hi[4], lo[4];
+            constexpr int order[8] = {0, 4, 1, 5, 2, 6, 3, 7};
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int X = __float2int_rn(v[j] * scale);
-            E[j] = ((uint32_t)X + 0x00808080u) ^ 0x00808080u;
-        }
-        // 4x4 byte transposes: words of one digit for inputs (0,2,4,6) and (1,3,5,7), the order in which the nibbles of a
-        // weight word separate into its low and high halves; index 0 = most significant digit
-        uint32_t lo[3], hi[3];
-        {
-            const uint32_t a = __byte_perm(E[0], E[2], 0x5140), b = __byte_perm(E[0], E[2], 0x7362);
-            const uint32_t c = __byte_perm(E[4], E[6], 0x5140), d = __byte_perm(E[4], E[6], 0x7362);
-            lo[2] = __byte_perm(a, c, 0x5410); lo[1] = __byte_perm(a, c, 0x7632);
-            lo[0] = __byte_perm(b, d, 0x5410);
-        }
-        {
-            const uint32_t a = __byte_perm(E[1], E[3], 0x5140), b = __byte_perm(E[1], E[3], 0x7362);
-            const uint32_t c = __byte_perm(E[5], E[7], 0x5140), d = __byte_perm(E[5], E[7], 0x7362);
-            hi[2] = __byte_perm(a, c, 0x5410); hi[1] = __byte_perm(a, c, 0x7632);
-            hi[0] = __byte_perm(b, d, 0x5410);
-        }
-        const int g = valid ? (int)((uint32_t)(blk * 8) / gs) : 0;
-        const uint32_t kb = (uint32_t)(blk * 8) % gs;
-        int sum[3];
-#pragma unroll
-        for (int p = 0; p < 3; p++) {
-            if (valid)
-                *reinterpret_cast<uint2*>(P.bimg + (size_t)g * img_group + swz((uint32_t)(p * P.mpad + m), kb, gs)) = make_uint2(lo[p], hi[p]);
-            sum[p] = __dp4a((int)lo[p], 0x01010101, __dp4a((int)hi[p], 0x01010101, 0));
-        }
-        int s01 = 256 * sum[0] + sum[1], s2 = sum[2];
-        for (uint32_t o = 1; o < lanes_per_group; o <<= 1) {
-            s01 += __shfl_xor_sync(0xffffffffu, s01, o);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-        }
-        if (valid && (tid & (lanes_per_group - 1)) == 0) {
-            // the sum of the token's integers over the group, as the f32 nearest to it (|s01| < 2^23 and |s2| < 2^15 are exact)
-            *reinterpret_cast<float*>(P.bimg + (size_t)g * img_group + (size_t)P.n * gs + (size_t)m * 4) = fmaf((float)s01, 256.0f, (float)s2);
+            for (int i = 0; i < 4; i++) {
+                const float x0 = rintf(v[order[2 * i]] * scale), x1 = rintf(v[order[2 * i + 1]] * scale);
+                const float h0 = rintf(x0 * (1.0f / 4096.0f)), h1 = rintf(x1 * (1.0f / 4096.0f));
+                const __half2 h = __floats2half2_rn(h0, h1), l = __floats2half2_rn(fmaf(h0, -4096.0f, x0), fmaf(h1, -4096.0f, x1));  // exact
+                hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+                lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+            }
+            // block `blk` of the K step: half (blk & 15) / 8, 16-byte chunk blk & 7 of the rows of both digits
+            uint8_t* dst = img + (size_t)(blk >> 4) * blk_bytes + (size_t)((blk >> 3) & 1) * P.tq * 256;
+            const uint32_t r0 = (uint32_t)t, r1 = (uint32_t)(P.tq + t), c = (uint32_t)blk & 7u;
+            *reinterpret_cast<uint4*>(dst + r0 * 128 + ((c ^ (r0 & 7u)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(dst + r1 * 128 + ((c ^ (r1 & 7u)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
     }
 }
 
 // ---- RoPE + cache append for M tokens (src/models.rs:100-129, 236-249) ----------------------------
-// grid (n_heads, M), 64 threads.  q is rotated in place; k (rotated) and v go to the cache rows.
-__global__ void __launch_bounds__(64) rope_append_kernel(const __grid_constant__ RopeParams P) {
-    const int h = blockIdx.x, m = blockIdx.y, i = threadIdx.x;
-    const int pos = P.pos[m];
-    const float c = P.rope_cos[(size_t)pos * (HS / 2) + i], s = P.rope_sin[(size_t)pos * (HS / 2) + i];
-    float* q = P.q + (size_t)m * P.ldq + (size_t)h * HS;
-    {
-        const float a = q[i], b = q[HS / 2 + i];
-        const float na = __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s));
-        const float nb = __fadd_rn(__fmul_rn(b, c), __fmul_rn(na, s));  // second half uses the rotated first half
-        q[i] = na;
-        q[HS / 2 + i] = nb;
-    }
-    if (h < P.n_kv_heads) {
-        const int KV = P.kv_stride ? P.kv_stride : P.n_kv_heads * HS;
-        const float* k = P.k + (size_t)m * P.ldkv + (size_t)h * HS;
-        const float* v = P.v + (size_t)m * P.ldkv + (size_t)h * HS;
-        const float a = k[i], b = k[HS / 2 + i];
-        const float na = __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s));
-        const float nb = __fadd_rn(__fmul_rn(b, c), __fmul_rn(na, s));
-        float* kc = P.kc + (size_t)pos * KV + (size_t)h * HS;
-        float* vc = P.vc + (size_t)pos * KV + (size_t)h * HS;
-        kc[i] = na;
-        kc[HS / 2 + i] = nb;
-        vc[i] = v[i];
-        vc[HS / 2 + i] = v[HS / 2 + i];
+// grid (M, slices of the row); a thread rotates four neighbouring pairs (i, i + 64) of one head.  Rotate-half as the reference does
+// it in place: the second half uses the already rotated first half.
+__device__ __forceinline__ void rotate4(const float4& a, const float4& b, const float4& c, const float4& s, float4& na, float4& nb) {
+    na.x = __fsub_rn(__fmul_rn(a.x, c.x), __fmul_rn(b.x, s.x)); nb.x = __fadd_rn(__fmul_rn(b.x, c.x), __fmul_rn(na.x, s.x));
+    na.y = __fsub_rn(__fmul_rn(a.y, c.y), __fmul_rn(b.y, s.y)); nb.y = __fadd_rn(__fmul_rn(b.y, c.y), __fmul_rn(na.y, s.y));
+    na.z = __fsub_rn(__fmul_rn(a.z, c.z), __fmul_rn(b.z, s.z)); nb.z = __fadd_rn(__fmul_rn(b.z, c.z), __fmul_rn(na.z, s.z));
+    na.w = __fsub_rn(__fmul_rn(a.w, c.w), __fmul_rn(b.w, s.w)); nb.w = __fadd_rn(__fmul_rn(b.w, c.w), __fmul_rn(na.w, s.w));
+}
+__global__ void __launch_bounds__(256) rope_append_kernel(const __grid_constant__ RopeParams P) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int m = blockIdx.x, pos = P.pos[m];
+    const int KV = P.kv_stride ? P.kv_stride : P.n_kv_heads * HS;
+    const int nq = P.n_heads * (HS / 8), nk = P.n_kv_heads * (HS / 8);  // units of four pairs
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < nq + 2 * nk; i += gridDim.y * blockDim.x) {
+        const int u = i < nq ? i : i < nq + nk ? i - nq : i - nq - nk, h = u / (HS / 8), e = (u % (HS / 8)) * 4, o = h * HS + e;
+        if (i < nq + nk) {
+            const float4 c = *reinterpret_cast<const float4*>(P.rope_cos + (size_t)pos * (HS / 2) + e), s = *reinterpret_cast<const float4*>(P.rope_sin + (size_t)pos * (HS / 2) + e);
+            const TcOut& T = i < nq ? P.q : P.k;
+            const float4 a = tc_load4(T, m, o), b = tc_load4(T, m, o + HS / 2);
+            float4 na, nb;
+            rotate4(a, b, c, s, na, nb);
+            float* dst = i < nq ? P.qout + (size_t)m * P.ldq + o : P.kc + (size_t)pos * KV + o;
+            *reinterpret_cast<float4*>(dst) = na;
+            *reinterpret_cast<float4*>(dst + HS / 2) = nb;
+        } else {
+            const float4 a = tc_load4(P.v, m, o), b = tc_load4(P.v, m, o + HS / 2);
+            float* dst = P.vc + (size_t)pos * KV + o;
+            *reinterpret_cast<float4*>(dst) = a;
+            *reinterpret_cast<float4*>(dst + HS / 2) = b;
+        }
     }
 }
 
@@ -208,6 +195,8 @@ __global__ void __launch_bounds__(64) rope_append_kernel(const __grid_constant__
 __global__ void __launch_bounds__(128) attn_batch_kernel(const __grid_constant__ AttnBatchParams P) {
     __shared__ __align__(16) float sm_acc[4][HS];
     __shared__ float sm_m[4], sm_l[4];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int h = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = h / P.ag, KV = P.kv_stride ? P.kv_stride : P.n_kv_heads * HS;
     const int T = P.pos[m] + 1;
@@ -243,30 +232,38 @@ __global__ void __launch_bounds__(128) attn_batch_kernel(const __grid_constant__
     P.out[(size_t)m * P.ldo + (size_t)h * HS + tid] = A / L;
 }
 
-// ---- hb = silu(h1) * h3 (src/models.rs:92-98) --------------------------------------------------------
-// h1, h3: [M][n] (this process's columns); hb: [M][ld] with those columns at the pointer given
-__global__ void swiglu_kernel(const float* __restrict__ h1, const float* __restrict__ h3, float* __restrict__ hb, int n, int ld, int M) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (size_t)M * n) {
-        const float a = h1[i];
-        hb[(i / n) * ld + i % n] = (a * (1.0f / (1.0f + expf(-a)))) * h3[i];
-    }
-}
-
 void launch_embed_batch(const float* table, const int* tokens, float* x, int dim, int M, cudaStream_t st) {
     g_launches++;
     embed_batch_kernel<<<M, 256, 0, st>>>(table, tokens, x, dim);
 }
-void launch_act_quant(const QuantParams& p, int M, cudaStream_t st) {
+// A launch that may start while the kernel in front of it still runs (it waits inside for that one's results).
+template <class K, class... A>
+static cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = cluster > 0 ? 2 : 1;
     g_launches++;
-    // slices of about one round of the CTA's threads (256 blocks of 8 inputs), whole groups each
-    const int G = p.in / p.gs;
-    const int S = std::max(1, std::min(std::min(4, G), p.in / 8 / AQ_THREADS));
-    act_quant_kernel<<<dim3(M, S), AQ_THREADS, 0, st>>>(p);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
-void launch_rope_append(const RopeParams& p, int n_heads, int M, cudaStream_t st) {
-    g_launches++;
-    rope_append_kernel<<<dim3(n_heads, M), 64, 0, st>>>(p);
+
+cudaError_t row_quant_init(int max_smem) { return cudaFuncSetAttribute(row_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem); }
+
+// As many CTAs per token as it takes to cover the SMs about twice with the batch (a row is 16 to 112 KB: one CTA walks it in 2 to
+// 10 us, and nothing else of a small batch would hide that), never more than the K steps of the row.
+cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st) {
+    int C = 1;
+    while (C < RQ_MAX_CLUSTER && 2 * C <= p.KS && (long long)p.M * C < sms) C *= 2;
+    return launch_pdl(row_quant_kernel, dim3(C, p.M), dim3(RQ_THREADS), (size_t)p.in * 4, C, st, p);
+}
+
+cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st) {
+    const int units = (p.n_heads + 2 * p.n_kv_heads) * (HS / 8);
+    return launch_pdl(rope_append_kernel, dim3(M, std::max(1, std::min((units + 255) / 256, 592 / M))), dim3(256), 0, 0, st, p);
 }
 
 // ---- the same attention with the cache rows shared by the queries that need them ---------------------------------------
@@ -280,6 +277,8 @@ constexpr int AT_WARPS = 8, AT_TILE = 32, AT_KPAD = HS + 4;  // K rows padded: a
 template <int AG, int NQW>  // query heads per kv head; queries per warp (NQW / AG tokens)
 __global__ void __launch_bounds__(32 * AT_WARPS) attn_batch_tiled_kernel(const __grid_constant__ AttnBatchParams P, int M) {
     extern __shared__ __align__(16) float at_smem[];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int TPW = NQW / AG;                       // tokens per warp
     constexpr int QB = AT_WARPS * TPW;                  // tokens per CTA
     float* Qs = at_smem;                                // [AT_WARPS * NQW][HS]
@@ -379,7 +378,7 @@ template <int AG, int NQW>
 static void launch_attn_tiled(const AttnBatchParams& p, int M, cudaStream_t st) {
     constexpr int QB = AT_WARPS * (NQW / AG);
     const size_t smem = (size_t)(AT_WARPS * NQW * HS + AT_TILE * AT_KPAD + AT_TILE * HS) * sizeof(float);
-    attn_batch_tiled_kernel<AG, NQW><<<dim3(p.n_kv_heads, (M + QB - 1) / QB), 32 * AT_WARPS, smem, st>>>(p, M);
+    launch_pdl(attn_batch_tiled_kernel<AG, NQW>, dim3(p.n_kv_heads, (M + QB - 1) / QB), dim3(32 * AT_WARPS), smem, 0, st, p, M);
 }
 
 // the tiled kernel's shared memory (65 KB at most) is above the default limit: once per device, at start-up
@@ -395,13 +394,12 @@ cudaError_t attn_batch_init() {
 // tiled: the kernel that shares cache tiles among queries (long contexts); otherwise one CTA per (head, token), which has
 // more CTAs and less set-up (short contexts: the cache is small and sits in the L2 anyway)
 void launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, cudaStream_t st) {
-    g_launches++;
     switch (tiled ? p.ag : 0) {
         case 1: launch_attn_tiled<1, 4>(p, M, st); break;
         case 2: launch_attn_tiled<2, 8>(p, M, st); break;
         case 4: launch_attn_tiled<4, 8>(p, M, st); break;
         case 8: launch_attn_tiled<8, 8>(p, M, st); break;
-        default: attn_batch_kernel<<<dim3(n_heads, M), 128, 0, st>>>(p); break;
+        default: launch_pdl(attn_batch_kernel, dim3(n_heads, M), dim3(128), 0, 0, st, p); break;
     }
 }
 // ---- all-gather of a column slice over peer memory (batched forward under tensor parallelism) ----------------------------
@@ -451,26 +449,27 @@ void launch_tp_gather(const TpGatherParams& p, cudaStream_t st) {
     tp_gather_kernel<<<std::min(p.M, 64), 256, 0, st>>>(p);
 }
 
-void launch_swiglu(const float* h1, const float* h3, float* hb, int n, int ld, int M, cudaStream_t st) {
-    g_launches++;
-    swiglu_kernel<<<(unsigned)(((size_t)M * n + 255) / 256), 256, 0, st>>>(h1, h3, hb, n, ld, M);
+// ---- the output of a GEMM as a plain buffer (callers that cannot add slices themselves) ----------------------------------------
+// dst (+)= the slices, or dst = silu(a) * b.  A destination that is slice 0 itself is only touched where there are more slices.
+__global__ void __launch_bounds__(256) finish_kernel(TcOut a, TcOut b, int pair, float* dst, int ld, int add) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 4, m = blockIdx.y;
+    if (o >= a.rows) return;
+    if (dst == a.out && tc_slices(a, m, o) == 1) return;
+    float4 v = tc_load4(a, m, o);
+    if (pair) {  // src/models.rs:92-98
+        const float4 w = tc_load4(b, m, o);
+        v.x = (v.x * (1.0f / (1.0f + expf(-v.x)))) * w.x; v.y = (v.y * (1.0f / (1.0f + expf(-v.y)))) * w.y;
+        v.z = (v.z * (1.0f / (1.0f + expf(-v.z)))) * w.z; v.w = (v.w * (1.0f / (1.0f + expf(-v.w)))) * w.w;
+    }
+    float4* d = reinterpret_cast<float4*>(dst + (size_t)m * ld + o);
+    if (add) { const float4 x = *d; v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
+    *d = v;
 }
 
-__global__ void __launch_bounds__(256) ksum_kernel(const float* __restrict__ part, size_t kstride, int ksplit, float* __restrict__ out,
-                                                   int ldo, int rows, int M, int epi) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M * rows) return;
-    const int m = (int)(i / rows), o = (int)(i % rows);
-    float v = 0.f;
-    for (int k = 0; k < ksplit; k++) v += part[(size_t)k * kstride + (size_t)m * rows + o];  // slice order: reproducible
-    float* dst = out + (size_t)m * ldo + o;
-    *dst = epi == EPI_RESID ? *dst + v : v;
-}
-
-void launch_ksum(const float* part, size_t kstride, int ksplit, float* out, int ldo, int rows, int M, int epi, cudaStream_t st) {
-    const size_t n = (size_t)M * rows;
-    g_launches++;
-    ksum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, kstride, ksplit, out, ldo, rows, M, epi);
+void launch_finish(const TcOut& a, const TcOut* b, float* dst, int ld, bool add, cudaStream_t st) {
+    launch_pdl(finish_kernel, dim3((a.rows / 4 + 255) / 256, a.M), dim3(256), 0, 0, st, a, b ? *b : a, b ? 1 : 0, dst, ld, add ? 1 : 0);
 }
 
 }  // namespace l2
