@@ -45,6 +45,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -56,9 +57,19 @@ constexpr int TC_LOAD_WARPS = 8, TC_DRAIN_WARPS = 8;
 constexpr int TC_RAW_WARP = TC_LOAD_WARPS + TC_DRAIN_WARPS, TC_B_WARP = TC_RAW_WARP + 1, TC_MMA_WARP = TC_RAW_WARP + 2;
 constexpr int TC_THREADS = 640;   // the last warp has no work: register counts are set per group of four warps
 constexpr int TC_KSTEP = 128;     // inputs per K step
-constexpr int TC_B_SLOTS = 3, TC_D_SLOTS = 3, TC_MAX_RAW = 12;
-constexpr uint32_t TC_D_COLS = 128, TC_A_COL0 = 384, TC_A_COLS = 64;  // tensor memory (512 columns): three accumulators, one A slot per weight tile
-constexpr int TC_MAX_SLICES = 8;
+constexpr int TC_B_SLOTS = 3, TC_MAX_RAW = 12;
+constexpr uint32_t TC_A_COLS = 64;
+// Tensor memory (512 columns) and registers by tokens per block (NT steps of 16).  Up to 32 tokens: four accumulators of 64 columns and two
+// A slots per weight tile, and few enough registers that the row kernels in front of and behind a GEMM fit beside it (its weight
+// requests start while they run).  More: three accumulators of 128 columns and one A slot per weight tile.
+template <int NT> struct TcShape {
+    static constexpr bool SMALL = NT <= 2;
+    static constexpr int D_SLOTS = SMALL ? 4 : 3, A_SLOTS = SMALL ? 2 : 1;
+    static constexpr uint32_t D_COLS = SMALL ? 64 : 128, A_COL0 = D_COLS * D_SLOTS;
+    // registers a thread: at launch (640 threads), then loaders (8 warps), drain (8 warps), the others (4 warps); the split never exceeds the launch
+    static constexpr int LAUNCH = SMALL ? 72 : 96, LOAD = SMALL ? 64 : 80, DRAIN = SMALL ? 96 : 136, REST = 40;
+    static_assert(8 * LOAD + 8 * DRAIN + 4 * REST <= 20 * LAUNCH && A_COL0 + 2 * A_SLOTS * TC_A_COLS == 512, "register split and tensor memory");
+};
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -167,8 +178,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t addr) {
                    "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Register split: the launch gives every thread 96; drain warps keep 64 tensor-memory words in flight beside 64 sums.
-// 8 warps x 80 + 8 warps x 136 + 4 warps x 40 = 60,416 of the launch's 61,440 registers.
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
@@ -222,6 +231,7 @@ __device__ __forceinline__ void add16(const uint32_t (&c)[2][16], unsigned long 
 template <int W, int NT>
 __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, Walk& walk) {
     constexpr int RT = 2, tq = 16 * NT, GPS = 4 / W;
+    using S = TcShape<NT>;
     constexpr uint32_t UB = 256u * W + 80u;
     const int quad = D.warp & 3, rec16 = D.lane & 7, rr = 4 * quad + (D.lane >> 3), rt = (D.warp - TC_LOAD_WARPS) >> 2;
     const uint32_t tquad = D.tmem_base + ((uint32_t)(32 * quad) << 16);
@@ -245,7 +255,7 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
         for (int i = 0; i < 8 * NT; i++) acc[i] = 0ull;
 #pragma unroll 1
         for (; n > 0; n--) {
-            const uint32_t tcol = tquad + d * TC_D_COLS;   // column of digit p, token t: p * tq + t
+            const uint32_t tcol = tquad + d * S::D_COLS;   // column of digit p, token t: p * tq + t
             if (!mbar_wait_warp(D.mma_done + d, dph, D.failed)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_fetch(ca, tcol, tq);
@@ -256,16 +266,17 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
             for (int st = 0; st < NT; st++) {
                 tmem_wait_ld();
                 if (st + 1 < NT) {
+                    if (S::SMALL) { add16(ca, acc + 8 * st, s2, k4096); tmem_fetch(ca, tcol + 16 * (st + 1), tq); continue; }  // (one set of registers)
                     if (st & 1) tmem_fetch(ca, tcol + 16 * (st + 1), tq); else tmem_fetch(cb, tcol + 16 * (st + 1), tq);
                 } else {  // everything has been read: the accumulator is free again
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (D.lane == 0) mbar_arrive(D.acc_free + d);
                 }
-                add16(st & 1 ? cb : ca, acc + 8 * st, s2, k4096);
+                add16(st & 1 && !S::SMALL ? cb : ca, acc + 8 * st, s2, k4096);
             }
             d += RT;
-            if (d >= TC_D_SLOTS) { d -= TC_D_SLOTS; dph ^= 1u; }
+            if (d >= S::D_SLOTS) { d -= S::D_SLOTS; dph ^= 1u; }
         }
         w0.next(P, sg);  // (worked out again: the coordinates would take registers from the loop above)
         // ---- this tile's share of the output: slice 0 goes to the output rows, later slices to the part buffers
@@ -287,28 +298,31 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
 
 }  // namespace
 
-template <int W, int RT>
-__global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_constant__ TcParams P) {
+template <int W, int NT>
+__global__ void __maxnreg__(TcShape<NT>::LAUNCH) gemm_q4_tc_kernel(const __grid_constant__ TcParams P) {
+    using S = TcShape<NT>;
+    constexpr int RT = 2, tq = 16 * NT;                      // weight tiles of a tile; tokens of a block
     constexpr int GS = 32 * W, GPS = TC_KSTEP / GS;          // inputs per group, groups per K step
     constexpr uint32_t UB = 256u * W + 80u;                  // bytes of a unit record
     constexpr uint32_t RUN = tc_run_bytes(W);                // room of a record run (16 rows x one K step)
     constexpr uint32_t RAW_BYTES = 8 * RUN;                  // raw weights of one 128-row tile and K step
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t raw_full[TC_MAX_RAW], raw_empty[TC_MAX_RAW], a_full[RT], a_empty[RT], b_full[TC_B_SLOTS], b_empty[TC_B_SLOTS], mma_done[TC_D_SLOTS], acc_free[TC_D_SLOTS];
+    __shared__ __align__(8) uint64_t raw_full[TC_MAX_RAW], raw_empty[TC_MAX_RAW], a_full[RT * S::A_SLOTS], a_empty[RT * S::A_SLOTS], b_full[TC_B_SLOTS], b_empty[TC_B_SLOTS],
+        mma_done[S::D_SLOTS], acc_free[S::D_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int failed;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t b_bytes = 512u * (uint32_t)P.tq;           // a digit block
+    constexpr uint32_t b_bytes = 512u * tq;                   // a digit block
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* stage_b = smem;                                  // [TC_B_SLOTS][2 halves][2 tq rows][128 bytes]
     uint8_t* raw = stage_b + TC_B_SLOTS * b_bytes;            // [nraw][8 runs]
 
     if (tid == 0) {
         for (int i = 0; i < TC_MAX_RAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
-        for (int i = 0; i < RT; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < RT * S::A_SLOTS; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
         for (int i = 0; i < TC_B_SLOTS; i++) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < TC_D_SLOTS; i++) { mbar_init(&mma_done[i], 1); mbar_init(&acc_free[i], 4); }
+        for (int i = 0; i < S::D_SLOTS; i++) { mbar_init(&mma_done[i], 1); mbar_init(&acc_free[i], 4); }
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -322,21 +336,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_
     const uint32_t tmem_base = tmem_base_s;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the kernel behind this one may set itself up
 
-    static_assert(RT == 2, "a tile is two weight tiles: one per group of loader and drain warps");
     // tensor-memory lane 32 q + l of a tile is row 16 (l & 7) + 4 q + (l >> 3) of its 128 rows
     const int quad = warp & 3, rec16 = lane & 7, rr = 4 * quad + (lane >> 3);
     Walk walk(P);
     Seg sg;
     if (warp < TC_LOAD_WARPS) {
-        regs_down<80>();
+        regs_down<S::LOAD>();
         // ================= loaders ==================================================================================
         // warps 0-3 take the first weight tile of every K step, warps 4-7 the second; a thread has a whole row of it
         const int rt = warp >> 2;
         const uint8_t* rec = raw + rec16 * RUN + rr * (16 * W);      // a row's words of a group follow one another
         const uint32_t z_shift = 4 * (rr & 7);
         const uint8_t* zeros = raw + rec16 * RUN + 256 * W + 64 + 4 * (rr >> 3);
-        const uint32_t tcol = tmem_base + ((uint32_t)(32 * quad) << 16) + TC_A_COL0 + rt * TC_A_COLS;
-        uint32_t rs = rt, rph = 0, aph = 1;  // slot and parity of the raw ring, parity of the A slot (a fresh "empty" barrier passes parity 1)
+        const uint32_t tquad = tmem_base + ((uint32_t)(32 * quad) << 16) + S::A_COL0;
+        uint32_t rs = rt, rph = 0, as = rt, aph = 1;  // slot and parity of the raw ring and of this weight tile's A slots (a fresh "empty" barrier passes parity 1)
         bool ok = true;
         while (ok && walk.next(P, sg)) {
 #pragma unroll 1
@@ -352,47 +365,45 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_
                 for (int gg = 0; gg < GPS; gg++) z[gg] = *reinterpret_cast<const uint32_t*>(zeros + so + gg * UB);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&raw_empty[rs]);
-                // the first half is turned into f16 before the A slot is free, the second while the first is stored
-                uint32_t a[4][16];
-                auto unpack32 = [&](int i) {
+                const uint32_t tcol = tquad + as * TC_A_COLS;
+                auto unpack32 = [&](int i, uint32_t* a) {
                     const uint32_t zz = ((z[i / PER] >> z_shift) & 15u) + 1u;                                  // src/gptq.rs:148
                     const uint32_t c1 = 0xE400E400u + zz * 0x00010001u, c2 = 0xD400D400u + zz * 0x00100010u;  // -(1024 + z), -(64 + z), twice each
-                    unpack8(v[i].x, c1, c2, a[i]); unpack8(v[i].y, c1, c2, a[i] + 4); unpack8(v[i].z, c1, c2, a[i] + 8); unpack8(v[i].w, c1, c2, a[i] + 12);
+                    unpack8(v[i].x, c1, c2, a); unpack8(v[i].y, c1, c2, a + 4); unpack8(v[i].z, c1, c2, a + 8); unpack8(v[i].w, c1, c2, a + 12);
                 };
-                unpack32(0);
-                unpack32(1);
-                if (!mbar_wait_warp(&a_empty[rt], aph, &failed)) { ok = false; break; }
-                aph ^= 1u;
+                // with one A slot per weight tile the first half is turned into f16 before the slot is free
+                constexpr int AHEAD = S::A_SLOTS == 1 ? 2 : 0;
+                uint32_t early[2][16];
+#pragma unroll
+                for (int i = 0; i < AHEAD; i++) unpack32(i, early[i]);
+                if (!mbar_wait_warp(&a_empty[as], aph, &failed)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                tmem_st16(tcol, a[0]);
-                tmem_st16(tcol + 16, a[1]);
-                unpack32(2);
-                tmem_st16(tcol + 32, a[2]);
-                unpack32(3);
-                tmem_st16(tcol + 48, a[3]);
+#pragma unroll
+                for (int i = 0; i < AHEAD; i++) tmem_st16(tcol + i * 16, early[i]);
+#pragma unroll
+                for (int i = AHEAD; i < 4; i++) {
+                    uint32_t a[16];
+                    unpack32(i, a);
+                    tmem_st16(tcol + i * 16, a);
+                }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[rt]);
+                if (lane == 0) mbar_arrive(&a_full[as]);
                 rs += RT; if (rs >= (uint32_t)P.nraw) { rs -= P.nraw; rph ^= 1u; }
+                as += RT; if (as >= RT * S::A_SLOTS) { as = rt; aph ^= 1u; }
             }
         }
         if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2003); }
     } else if (warp < TC_RAW_WARP) {
-        regs_up<136>();
+        regs_up<S::DRAIN>();
         // ================= drain warps ==================================================================================
         asm volatile("griddepcontrol.wait;" ::: "memory");     // the tokens' factors (and the output buffers) belong to the kernels in front of this one
-        bool ok;
         const Drain D{mma_done, acc_free, &failed, tmem_base, warp, lane};
-        switch (P.tq / 16) {  // one body per number of 16-token steps: with a run-time count the columns in flight change registers at every branch
-            case 1: ok = drain_tiles<W, 1>(P, D, walk); break;
-            case 2: ok = drain_tiles<W, 2>(P, D, walk); break;
-            case 3: ok = drain_tiles<W, 3>(P, D, walk); break;
-            default: ok = drain_tiles<W, 4>(P, D, walk); break;
-        }
+        const bool ok = drain_tiles<W, NT>(P, D, walk);
         if (!ok && lane == 0) { failed = 1; if (P.status) atomicExch(P.status, 2002); }
     } else {
-        regs_down<40>();  // one instruction for the four warps: it is a warpgroup operation
+        regs_down<S::REST>();  // one instruction for the four warps: it is a warpgroup operation
         if (warp == TC_RAW_WARP) {
         // ================= raw weights: lanes 0-7 copy one record run each ================================================
         uint32_t rs = 0, rph = 1;
@@ -447,11 +458,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_
             // Operand addresses are kept as the low words of the descriptors and advanced by constants: this warp shares its scheduler
             // with four busy ones and every instruction between two MMAs costs it about ten clocks.
             const bool leader = elect_one();
-            const uint32_t N = 2u * (uint32_t)P.tq;
+            constexpr uint32_t N = 2u * tq;
             // instruction descriptor: D f32, A and B f16, both K-major, N, M = 128
-            const uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t b_lo0 = umma_desc_lo(smem_addr(stage_b)), slot_units = b_bytes >> 4, half_units = N * 128 / 16;
-            uint32_t aph = 0, bs = 0, bph = 0, d = 0, dph = 1;
+            constexpr uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+            const uint32_t b_lo0 = umma_desc_lo(smem_addr(stage_b)), slot_units = b_bytes >> 4, half_units = N * 128 / 16;  // (N rows of 128 bytes per half)
+            uint32_t as = 0, aph = 0, bs = 0, bph = 0, d = 0, dph = 1;
             bool ok = true;
             while (ok && walk.next(P, sg)) {
 #pragma unroll 1
@@ -464,30 +475,30 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q4_tc_kernel(const __grid_
                         if (gg >= ng) break;
 #pragma unroll
                         for (int rt = 0; rt < RT; rt++) {
-                            if (gg == 0 && ok) ok = mbar_wait_warp(&a_full[rt], aph, &failed);
+                            if (gg == 0 && ok) ok = mbar_wait_warp(&a_full[as + rt], aph, &failed);
                             if (ok) ok = mbar_wait_warp(&acc_free[d], dph, &failed);
                             if (!ok) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t td = d * TC_D_COLS;
+                            const uint32_t td = d * S::D_COLS, ta = S::A_COL0 + (as + rt) * TC_A_COLS;
                             if (leader) {
 #pragma unroll
                                 for (int j = 0; j < GS / 16; j++) {  // 16 inputs: 8 columns of A, 32 bytes of B
                                     const int k0 = gg * GS + 16 * j;
-                                    if (j == 0) mma_f16<false>(td, TC_A_COL0 + rt * TC_A_COLS + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
-                                    else mma_f16<true>(td, TC_A_COL0 + rt * TC_A_COLS + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
+                                    if (j == 0) mma_f16<false>(td, ta + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
+                                    else mma_f16<true>(td, ta + k0 / 2, b_half[k0 / 64] + (k0 % 64) / 8, idesc);
                                 }
                                 commit_to(&mma_done[d]);
                                 if (gg == ng - 1) {
-                                    commit_to(&a_empty[rt]);
+                                    commit_to(&a_empty[as + rt]);
                                     if (rt == RT - 1) commit_to(&b_empty[bs]);
                                 }
                             }
                             __syncwarp();
-                            if (++d == TC_D_SLOTS) { d = 0; dph ^= 1u; }
+                            if (++d == S::D_SLOTS) { d = 0; dph ^= 1u; }
                         }
                         if (!ok) break;
                     }
-                    aph ^= 1u;
+                    as += RT; if (as == RT * S::A_SLOTS) { as = 0; aph ^= 1u; }
                     if (++bs == TC_B_SLOTS) { bs = 0; bph ^= 1u; }
                 }
             }
@@ -544,8 +555,10 @@ void gemm_tc_plan(TcParams& p, int gs, int sms) {
 cudaError_t gemm_tc_init(int max_smem) {
     tc_max_smem = max_smem;
     cudaError_t e;
-#define L2_TC_ATTR(W, RT) if ((e = cudaFuncSetAttribute(gemm_q4_tc_kernel<W, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_max_smem)) != cudaSuccess) return e;
-    L2_TC_ATTR(4, 2) L2_TC_ATTR(2, 2) L2_TC_ATTR(1, 2)
+#define L2_TC_ATTR(W, NT) if ((e = cudaFuncSetAttribute(gemm_q4_tc_kernel<W, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_max_smem)) != cudaSuccess) return e;
+#define L2_TC_ATTR_W(W) L2_TC_ATTR(W, 1) L2_TC_ATTR(W, 2) L2_TC_ATTR(W, 3) L2_TC_ATTR(W, 4)
+    L2_TC_ATTR_W(4) L2_TC_ATTR_W(2) L2_TC_ATTR_W(1)
+#undef L2_TC_ATTR_W
 #undef L2_TC_ATTR
     return cudaSuccess;
 }
@@ -564,9 +577,18 @@ cudaError_t launch_gemm_tc(const TcParams& p, cudaStream_t st) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     g_launches++;
-    if (p.gs == 128) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<4, 2>, p);
-    if (p.gs == 64) return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<2, 2>, p);
-    return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<1, 2>, p);
+    auto by_tokens = [&](auto w) {  // one instantiation per group size and 16-token steps
+        constexpr int W = decltype(w)::value;
+        switch (p.tq / 16) {
+            case 1: return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<W, 1>, p);
+            case 2: return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<W, 2>, p);
+            case 3: return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<W, 3>, p);
+            default: return cudaLaunchKernelEx(&cfg, gemm_q4_tc_kernel<W, 4>, p);
+        }
+    };
+    if (p.gs == 128) return by_tokens(std::integral_constant<int, 4>());
+    if (p.gs == 64) return by_tokens(std::integral_constant<int, 2>());
+    return by_tokens(std::integral_constant<int, 1>());
 }
 
 }  // namespace l2

@@ -42,7 +42,7 @@ unsigned long long* g_sk_trace = nullptr;
 
 
 template <int W, int NSEG>
-__global__ void __launch_bounds__(SK_THREADS + 32, 1) gemv_sk_kernel(const SkParams* __restrict__ gp) {
+__global__ void __launch_bounds__(SK_THREADS + 32, 1) gemv_sk_kernel(const SkParams* __restrict__ gp, float* out) {
     constexpr int GS = 32 * W;
     constexpr int ROWS = 16 * NSEG;  // rows of a (super) tile
     extern __shared__ __align__(16) uint8_t smem[];
@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(SK_THREADS + 32, 1) gemv_sk_kernel(const SkPar
     if (threadIdx.x < sizeof(SkParams) / 16)
         reinterpret_cast<uint4*>(&sp)[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(gp) + threadIdx.x);
     __syncthreads();
+    if (out && threadIdx.x == 0) sp.job[0].out = out;  // (read behind later barriers)
     const SkParams& P = sp;
     if (P.trace && threadIdx.x == 0) P.trace[blockIdx.x * 8] = t_entry;
 
@@ -302,7 +303,7 @@ size_t sk_smem_fixed(int in, int G, int nseg, int ptiles) {
 size_t sk_slot_bytes(int group_size, int chunk) { return (size_t)chunk * (8 * (size_t)group_size + 80); }
 
 template <int W, int NSEG>
-static cudaError_t launch_sk_t(const SkParams* p, int grid, size_t smem, cudaStream_t st, bool pdl) {
+static cudaError_t launch_sk_t(const SkParams* p, int grid, size_t smem, cudaStream_t st, bool pdl, float* out) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(grid);
@@ -316,19 +317,19 @@ static cudaError_t launch_sk_t(const SkParams* p, int grid, size_t smem, cudaStr
         cfg.numAttrs = 1;
     }
     g_launches++;
-    return cudaLaunchKernelEx(&cfg, gemv_sk_kernel<W, NSEG>, p);
+    return cudaLaunchKernelEx(&cfg, gemv_sk_kernel<W, NSEG>, p, out);
 }
 
-cudaError_t launch_sk(const SkParams* p, int group_size, int nseg, int grid, size_t smem, cudaStream_t st, bool pdl) {
+cudaError_t launch_sk(const SkParams* p, int group_size, int nseg, int grid, size_t smem, cudaStream_t st, bool pdl, float* out) {
     const int w = group_size / 32;
     if (nseg == 1) {
-        if (w == 4) return launch_sk_t<4, 1>(p, grid, smem, st, pdl);
-        if (w == 2) return launch_sk_t<2, 1>(p, grid, smem, st, pdl);
-        return launch_sk_t<1, 1>(p, grid, smem, st, pdl);
+        if (w == 4) return launch_sk_t<4, 1>(p, grid, smem, st, pdl, out);
+        if (w == 2) return launch_sk_t<2, 1>(p, grid, smem, st, pdl, out);
+        return launch_sk_t<1, 1>(p, grid, smem, st, pdl, out);
     }
-    if (w == 4) return launch_sk_t<4, 2>(p, grid, smem, st, pdl);
-    if (w == 2) return launch_sk_t<2, 2>(p, grid, smem, st, pdl);
-    return launch_sk_t<1, 2>(p, grid, smem, st, pdl);
+    if (w == 4) return launch_sk_t<4, 2>(p, grid, smem, st, pdl, out);
+    if (w == 2) return launch_sk_t<2, 2>(p, grid, smem, st, pdl, out);
+    return launch_sk_t<1, 2>(p, grid, smem, st, pdl, out);
 }
 
 cudaError_t sk_init(int max_smem) {

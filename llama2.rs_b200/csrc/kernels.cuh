@@ -96,21 +96,34 @@ struct TcParams {
 struct TcOut {
     const float* out; const float* part;
     int ldo, rows, tile0;  // tile0: tiles of the launch in front of this matrix
-    int ntb, tq, KS, q, tile_rows, M;
+    int ntb, tq, KS, q, M;
+    float rq;              // 1 / q
 };
+constexpr int TC_TILE_ROWS = 256;  // rows of a tile of the launch
+constexpr int TC_MAX_SLICES = 8;   // slices of a tile at most
 #ifdef __CUDACC__
-__device__ __forceinline__ int tc_slices(const TcOut& t, int m, int o) {
-    const int T = t.tile0 + (o / t.tile_rows) * t.ntb + m / t.tq;
-    return (T * t.KS + t.KS - 1) / t.q - (T * t.KS) / t.q + 1;
+__device__ __forceinline__ int tc_cta(const TcOut& t, int x) {  // x / q for x < 2^24
+    int c = (int)((float)x * t.rq);
+    if (c * t.q > x) c--; else if ((c + 1) * t.q <= x) c++;
+    return c;
 }
-__device__ __forceinline__ float4 tc_load4(const TcOut& t, int m, int o) {  // o a multiple of 4
+__device__ __forceinline__ int tc_slices(const TcOut& t, int tb, int o) {  // of output o of a token of block tb
+    const int x = (t.tile0 + (o / TC_TILE_ROWS) * t.ntb + tb) * t.KS;
+    return tc_cta(t, x + t.KS - 1) - tc_cta(t, x) + 1;
+}
+// Outputs o .. o + 3 of token m (block tb): the slices are requested together and added in order.
+__device__ __forceinline__ float4 tc_load4(const TcOut& t, int m, int tb, int o) {
     float4 v = *reinterpret_cast<const float4*>(t.out + (size_t)m * t.ldo + o);
-    const int n = tc_slices(t, m, o);
+    const int n = tc_slices(t, tb, o);
+    if (n == 1) return v;
     const float* p = t.part + (size_t)m * t.rows + o;
-    for (int j = 1; j < n; j++, p += (size_t)t.M * t.rows) {
-        const float4 a = *reinterpret_cast<const float4*>(p);
-        v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
-    }
+    float4 a[TC_MAX_SLICES - 1];
+#pragma unroll
+    for (int j = 0; j < TC_MAX_SLICES - 1; j++)
+        a[j] = j + 1 < n ? *reinterpret_cast<const float4*>(p + (size_t)j * t.M * t.rows) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < TC_MAX_SLICES - 1; j++)
+        if (j + 1 < n) { v.x += a[j].x; v.y += a[j].y; v.z += a[j].z; v.w += a[j].w; }
     return v;
 }
 #endif
@@ -258,7 +271,8 @@ size_t token_gemv_smem(int in, int G, int nseg, int ptiles, bool natural, bool g
 
 void launch_embed(const EmbedParams& p, cudaStream_t st, bool pdl);
 // `p` points to device memory: the kernel copies the record into shared memory with one cooperative load
-cudaError_t launch_sk(const SkParams* p, int group_size, int nseg, int grid, size_t smem, cudaStream_t st, bool pdl);
+// (out: where a launch of a single job puts its result, instead of the record's pointer)
+cudaError_t launch_sk(const SkParams* p, int group_size, int nseg, int grid, size_t smem, cudaStream_t st, bool pdl, float* out = nullptr);
 size_t sk_smem_fixed(int in, int G, int nseg, int ptiles);  // digits, group sums, tile sums
 size_t sk_slot_bytes(int group_size, int chunk);           // one ring slot of one warp
 cudaError_t sk_init(int max_smem);

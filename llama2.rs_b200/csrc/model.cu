@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "host_stage.h"
 #include "model.h"
 
 using namespace l2;
@@ -104,13 +105,23 @@ int upload_qlinear(const PackedQ& p, const int32_t* g_index, DevQ& d, std::vecto
 }
 
 __global__ void permute_kernel(const float* __restrict__ x, const int* __restrict__ perm, float* __restrict__ xp, int n) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) xp[j] = x[perm[j]];
+    const int src = j < n ? perm[j] : 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernels in front may still read xp or write x
+    if (j < n) xp[j] = x[src];
 }
 
-void launch_permute(const float* x, const int* perm, float* xp, int n, cudaStream_t st) {
-    permute_kernel<<<(n + 255) / 256, 256, 0, st>>>(x, perm, xp, n);
+// Launched programmatically, and so is the GEMV behind it: that kernel's weight stream starts while this one runs.
+cudaError_t launch_permute(const float* x, const int* perm, float* xp, int n, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3((n + 255) / 256); cfg.blockDim = dim3(256); cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
     g_launches++;
+    return cudaLaunchKernelEx(&cfg, permute_kernel, x, perm, xp, n);
 }
 
 void sk_set_matrix(SkJob& j, int seg, const DevQ& q, const float* x, const float* nw) {
@@ -178,18 +189,16 @@ void sk_prefetch_next(SkLaunch& L, const DevQ& q) {
     p.next_bytes[p.n_next++] = (size_t)q.tiles * q.G * ((q.gs / 32) * 256 + 80);
 }
 
-int run_gemv_single(const DevQ& q, const float* xp, float* y, int sms, SkParams* d_plan, cudaStream_t st) {
-    SkLaunch L;
+// The launch of one matrix alone; the output is given with each launch, so the record stays on the device.
+int plan_gemv_single(const DevQ& q, const float* xp, int sms, SkLaunch& L) {
+    L = SkLaunch{};
     L.p.njobs = 1;
     L.nseg = 1;
     L.gs = q.gs;
     sk_set_matrix(L.p.job[0], 0, q, xp, nullptr);
-    L.p.job[0].out = y;
     L.p.job[0].epi = EPI_STORE;
     if (int rc = sk_plan(L, sms)) return rc;
     L.p.trace = g_sk_trace;
-    L2_CUDA(cudaMemcpyAsync(d_plan, &L.p, sizeof(SkParams), cudaMemcpyHostToDevice, st));  // pageable source: staged before return
-    L2_CUDA(launch_sk(d_plan, L.gs, 1, L.grid, L.smem, st, false));
     return L2_OK;
 }
 
@@ -319,6 +328,8 @@ static int build_model(const Shape& shape, Source& src, const l2_options* opt, l
                c.dim, c.hidden_dim, c.n_layers, c.n_heads, c.n_kv_heads, c.vocab_size, c.seq_len, c.group_size);
         printf("CUDA device %d, %d SMs, %.2f GB of weights on device\n", m->device, m->sms, m->device_bytes / 1e9);
     }
+    StagePool::retain();
+    m->staged = true;
     *out = m.release();
     return L2_OK;
 }
@@ -911,6 +922,7 @@ extern "C" void l2_model_close(l2_model* m) {
     free_batch(m);
     free_allocs(m->allocs);
     if (m->own_stream) cudaStreamDestroy(m->own_stream);
+    if (m->staged) StagePool::release();
     delete m;
 }
 
@@ -1106,6 +1118,13 @@ static int check_state(l2_model* m, l2_state* s, const char* who) {
 static int check_status(l2_state* s);
 static int report_status(l2_state* s);
 
+// The logits in the caller's array, through pinned memory; returns with the stream drained.
+static int read_logits(l2_state* s, float* logits) {
+    StagePool::Lease stage;
+    if (int rc = stage.take(s->m->device)) return rc;
+    return stage->download(logits, s->logits, sizeof(float) * s->m->shape.c.vocab_size, s->m->stream);
+}
+
 extern "C" int l2_forward(l2_model* m, l2_state* s, const int32_t* tokens, const int32_t* pos, int B, float* logits) {
     clear_error();
     if (int rc = check_state(m, s, "l2_forward")) return rc;
@@ -1131,8 +1150,8 @@ extern "C" int l2_forward(l2_model* m, l2_state* s, const int32_t* tokens, const
     } else if (int rc = forward_batch(s, B, tokens, pos)) {  // all rows stored, then attention over 0..=pos[b]
         return rc;
     }
-    if (B == 1 && logits) L2_CUDA(cudaMemcpyAsync(logits, s->logits, sizeof(float) * c.vocab_size, cudaMemcpyDeviceToHost, m->stream));
     if (B > 1) return check_status(s);
+    if (logits) return read_logits(s, logits);
     L2_CUDA(cudaStreamSynchronize(m->stream));
     return L2_OK;
 }
@@ -1206,8 +1225,8 @@ extern "C" int l2_decode_step(l2_model* m, l2_state* s, int32_t token, int32_t p
     if (int rc = write_ctl(s, pos, token, 0, forced_next < 0 ? -1 : forced_next, temperature, rng_seed ? *rng_seed : 0)) return rc;
     if (int rc = run_forward(s, G_DECODE)) return rc;
     L2_CUDA(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, m->stream));
-    if (logits) L2_CUDA(cudaMemcpyAsync(logits, s->logits, sizeof(float) * c.vocab_size, cudaMemcpyDeviceToHost, m->stream));
-    L2_CUDA(cudaStreamSynchronize(m->stream));
+    if (logits) { if (int rc = read_logits(s, logits)) return rc; }
+    else L2_CUDA(cudaStreamSynchronize(m->stream));
     if (s->h_ctl->status) return report_status(s);
     if (next) *next = s->h_ctl->last_next;
     if (rng_seed) *rng_seed = s->h_ctl->rng;
@@ -1463,18 +1482,28 @@ extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t*
     PackedQ p;
     repack_qlinear(in, out, group_size, qweight, qzeros, scales, nullptr, p);
     if (int rc = upload_qlinear(p, g_index, q->q, q->allocs, nullptr)) { free_allocs(q->allocs); return rc; }
-    if (int rc = dev_alloc(reinterpret_cast<void**>(&q->d_plan), sizeof(SkParams), q->allocs)) { free_allocs(q->allocs); return rc; }
     L2_CUDA(cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking));
+    L2_CUDA(cudaMallocHost(reinterpret_cast<void**>(&q->status), sizeof(int)));
+    *q->status = 0;
+    StagePool::retain();
     *h = q.release();
     return L2_OK;
 }
 
-static int qlinear_reserve(l2_qlinear* h, int B) {
-    if (B <= h->cap_b) return L2_OK;
+static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
     int rc;
-    if ((rc = dev_alloc(reinterpret_cast<void**>(&h->x_dev), sizeof(float) * h->q.in * B, h->allocs))) return rc;
-    if ((rc = dev_alloc(reinterpret_cast<void**>(&h->xp_dev), sizeof(float) * h->q.in, h->allocs))) return rc;
-    if ((rc = dev_alloc(reinterpret_cast<void**>(&h->y_dev), sizeof(float) * h->q.out * B, h->allocs))) return rc;
+    if (host && B > h->cap_host) {  // device copies of the caller's host arrays
+        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->x_dev), sizeof(float) * h->q.in * B, h->allocs))) return rc;
+        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->y_dev), sizeof(float) * h->q.out * B, h->allocs))) return rc;
+        h->cap_host = B;
+    }
+    if (B == 1) {
+        if (h->d_plan) return L2_OK;
+        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->xp_dev), sizeof(float) * h->q.in, h->allocs))) return rc;
+        if ((rc = plan_gemv_single(h->q, h->xp_dev, h->sms, h->plan))) return rc;
+        return dev_upload(&h->d_plan, &h->plan.p, 1, h->allocs);
+    }
+    if (B <= h->cap_b) return L2_OK;
     if (B >= 2) {  // buffers of the batched (tcgen05) path
         const int cap = B <= TC_MAX_TOKENS ? TC_MAX_TOKENS : (int)MAX_BATCH;
         if (cap > h->cap_tc) {
@@ -1484,12 +1513,8 @@ static int qlinear_reserve(l2_qlinear* h, int B) {
             if ((rc = dev_alloc(reinterpret_cast<void**>(&h->kpart), sizeof(float) * part_floats(rows, 1, h->q.in, h->q.gs, cap, h->sms), h->allocs))) return rc;
             h->cap_tc = cap;
         }
-        if (!h->status) {
-            if ((rc = dev_alloc(reinterpret_cast<void**>(&h->status), sizeof(int), h->allocs))) return rc;
-            L2_CUDA(cudaMemset(h->status, 0, sizeof(int)));
-        }
     }
-    h->cap_b = B;
+    if (B >= 2) h->cap_b = B;
     return L2_OK;
 }
 
@@ -1498,7 +1523,7 @@ extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* x
     if (!h || !x_dev || !xout_dev || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec_dev: bad argument");
     L2_CUDA(cudaSetDevice(h->device));
     cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : h->stream;
-    if (int rc = qlinear_reserve(h, B)) return rc;
+    if (int rc = qlinear_reserve(h, B, false)) return rc;
     if (B >= 2) {  // batched: tensor-core GEMM, MAX_BATCH tokens at a time
         for (int b0 = 0; b0 < B; b0 += MAX_BATCH) {
             const int M = std::min<int>(MAX_BATCH, B - b0);
@@ -1506,22 +1531,22 @@ extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* x
         }
         return L2_OK;
     }
-    launch_permute(x_dev, h->q.perm, h->xp_dev, h->q.in, st);
-    return run_gemv_single(h->q, h->xp_dev, xout_dev, h->sms, h->d_plan, st);
+    L2_CUDA(launch_permute(x_dev, h->q.perm, h->xp_dev, h->q.in, st));
+    L2_CUDA(launch_sk(h->d_plan, h->q.gs, 1, h->plan.grid, h->plan.smem, st, true, xout_dev));
+    return L2_OK;
 }
 
 extern "C" int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B) {
     clear_error();
     if (!h || !x || !xout || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec: bad argument");
     L2_CUDA(cudaSetDevice(h->device));
-    if (int rc = qlinear_reserve(h, B)) return rc;
-    L2_CUDA(cudaMemcpyAsync(h->x_dev, x, sizeof(float) * h->q.in * B, cudaMemcpyHostToDevice, h->stream));
+    if (int rc = qlinear_reserve(h, B, true)) return rc;
+    StagePool::Lease stage;
+    if (int rc = stage.take(h->device)) return rc;
+    if (int rc = stage->upload(h->x_dev, x, sizeof(float) * h->q.in * B, h->stream)) return rc;
     if (int rc = l2_qlinear_matvec_dev(h, h->x_dev, h->y_dev, B, h->stream)) return rc;
-    L2_CUDA(cudaMemcpyAsync(xout, h->y_dev, sizeof(float) * h->q.out * B, cudaMemcpyDeviceToHost, h->stream));
-    int status = 0;
-    if (h->status) L2_CUDA(cudaMemcpyAsync(&status, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    L2_CUDA(cudaStreamSynchronize(h->stream));
-    if (status) return fail(L2_ESTATUS, "device status %d", status);
+    if (int rc = stage->download(xout, h->y_dev, sizeof(float) * h->q.out * B, h->stream)) return rc;
+    if (*h->status) return fail(L2_ESTATUS, "device status %d", *h->status);
     return L2_OK;
 }
 
@@ -1529,7 +1554,9 @@ extern "C" void l2_qlinear_free(l2_qlinear* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     free_allocs(h->allocs);
+    if (h->status) cudaFreeHost(h->status);
     if (h->stream) cudaStreamDestroy(h->stream);
+    StagePool::release();
     delete h;
 }
 

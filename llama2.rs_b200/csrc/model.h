@@ -88,6 +88,7 @@ struct l2_model {
     size_t device_bytes = 0;
     l2_state* gen_state = nullptr;  // reused by l2_generate_ids
     l2::BatchBuffers* batch = nullptr;  // activations of the batched forward, allocated on first use
+    bool staged = false;            // holds a share of the pinned staging pool
     bool use_graph = true, use_pdl = true;
     bool use_token_kernel = true;    // B=1 forward as one persistent kernel (single GPU only)
     int tp_rank = 0, tp_world = 1;   // tensor parallelism: this process owns 1/tp_world of every matrix's rows
@@ -144,24 +145,25 @@ struct l2_qlinear {
     int sms = 148;
     int group_size = 128;
     float *x_dev = nullptr, *xp_dev = nullptr, *y_dev = nullptr;
+    l2::SkLaunch plan;                   // B = 1: launch plan and its record on the device
     l2::SkParams* d_plan = nullptr;
     uint8_t* img = nullptr;   // batched path: digit image with the digit sums, and the factors
     float* osc = nullptr;
     float* kpart = nullptr;   // slices of the output beyond the first
-    int* status = nullptr;
-    int cap_b = 0, cap_tc = 0;  // batch sizes the buffers hold
+    int* status = nullptr;    // pinned host word that a kernel whose wait gave up writes: nothing has to be copied to look at it
+    int cap_host = 0, cap_b = 0, cap_tc = 0;  // batch sizes the buffers hold
     cudaStream_t stream = nullptr;
     std::vector<void*> allocs;
 };
 
 namespace l2 {
 int upload_qlinear(const PackedQ& p, const int32_t* g_index, DevQ& d, std::vector<void*>& allocs, size_t* bytes);
-void launch_permute(const float* x, const int* perm, float* xp, int n, cudaStream_t st);
+cudaError_t launch_permute(const float* x, const int* perm, float* xp, int n, cudaStream_t st);
 int check_attention_args(int n_heads, int n_kv_heads, int pos, const void* q, const void* k, const void* v, const void* kc,
                          const void* vc, const void* rc, const void* rs, const void* out);
 int device_sm_count();
 int attention_max_split(int n_kv_heads);
-int run_gemv_single(const DevQ& q, const float* xp, float* y, int sms, SkParams* d_plan, cudaStream_t st);
+int plan_gemv_single(const DevQ& q, const float* xp, int sms, SkLaunch& L);
 int sk_plan(SkLaunch& L, int sms);
 void sk_prefetch_next(SkLaunch& L, const DevQ& q);
 int forward_batch(l2_state* s, int M, const int32_t* tokens, const int32_t* pos);

@@ -24,7 +24,7 @@ TcOut tc_out(const TcParams& t, int i) {
     TcOut o{};
     o.out = t.mat[i].out; o.part = t.mat[i].part; o.ldo = t.mat[i].ldo; o.rows = t.mat[i].rows;
     o.tile0 = i ? t.mat[i - 1].tile_end : 0;
-    o.ntb = t.ntb; o.tq = t.tq; o.KS = t.KS; o.q = t.q; o.tile_rows = 128 * t.rt; o.M = t.M;
+    o.ntb = t.ntb; o.tq = t.tq; o.KS = t.KS; o.q = t.q; o.rq = 1.0f / (float)t.q; o.M = t.M;
     return o;
 }
 

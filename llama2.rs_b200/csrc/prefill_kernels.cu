@@ -54,34 +54,46 @@ __global__ void embed_batch_kernel(const float* __restrict__ table, const int* _
 constexpr int RQ_THREADS = 256;
 constexpr int RQ_MAX_CLUSTER = 8;
 
-__global__ void __launch_bounds__(RQ_THREADS) row_quant_kernel(const __grid_constant__ RowParams P) {
+__global__ void __launch_bounds__(RQ_THREADS, 4) row_quant_kernel(const __grid_constant__ RowParams P) {
     extern __shared__ __align__(16) float xs[];  // the row (times the norm weight), natural order
     __shared__ float red[2][RQ_THREADS / 32];
     __shared__ float stat[RQ_MAX_CLUSTER][2];    // (largest |x nw|, sum of x^2) of every CTA's share
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int C = (int)gridDim.x, r = (int)cluster_rank(), m = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tb = m / P.tq, t = m - tb * P.tq;
+    const int n4 = P.in / 4, i0 = (int)((long long)n4 * r / C), i1 = (int)((long long)n4 * (r + 1) / C);
+    // this CTA's share of the digits: blocks of 8 inputs, whole K steps; an item is a block of one consumer
+    const int b0 = (int)((long long)P.KS * r / C) * 16, nb = min(P.in / 8, (int)((long long)P.KS * (r + 1) / C) * 16) - b0, items = P.nmat * nb;
+    auto perm_of = [&](int item) {
+        const int j = item / nb;
+        const uint16_t* p = j == 0 ? P.perm[0] : j == 1 ? P.perm[1] : P.perm[2];
+        return item < items && p ? __ldg(reinterpret_cast<const uint4*>(p) + b0 + (item - j * nb)) : make_uint4(0, 0, 0, 0);
+    };
+    // what does not depend on the kernel in front is requested before waiting for it
+    const uint4 perm0 = perm_of(tid);
+    float4 w0 = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (P.nw && i0 + tid < i1) w0 = __ldg(reinterpret_cast<const float4*>(P.nw) + i0 + tid);
     if (C > 1) cluster_barrier();  // every CTA of the cluster has started: its shared memory may be written
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int n4 = P.in / 4, i0 = (int)((long long)n4 * r / C), i1 = (int)((long long)n4 * (r + 1) / C);
     float mx = 0.f, sq = 0.f;
     for (int i = i0 + tid; i < i1; i += RQ_THREADS) {
         float4 v;
         if (P.mode == ROW_SWIGLU) {  // src/models.rs:92-98
-            const float4 a = tc_load4(P.a, m, i * 4), b = tc_load4(P.b, m, i * 4);
+            const float4 a = tc_load4(P.a, m, tb, i * 4), b = tc_load4(P.b, m, tb, i * 4);
             v.x = (a.x * (1.0f / (1.0f + expf(-a.x)))) * b.x; v.y = (a.y * (1.0f / (1.0f + expf(-a.y)))) * b.y;
             v.z = (a.z * (1.0f / (1.0f + expf(-a.z)))) * b.z; v.w = (a.w * (1.0f / (1.0f + expf(-a.w)))) * b.w;
         } else {
             float4* xp = reinterpret_cast<float4*>(P.x + (size_t)m * P.ldx) + i;
             v = *xp;
             if (P.mode == ROW_RESID) {  // src/models.rs:47-51
-                const float4 a = tc_load4(P.a, m, i * 4);
+                const float4 a = tc_load4(P.a, m, tb, i * 4);
                 v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
                 *xp = v;
             }
         }
         sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         if (P.nw) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(P.nw) + i);
+            const float4 w = i == i0 + tid ? w0 : __ldg(reinterpret_cast<const float4*>(P.nw) + i);
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
         mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
@@ -114,26 +126,19 @@ __global__ void __launch_bounds__(RQ_THREADS) row_quant_kernel(const __grid_cons
     if (tid == 0 && r == 0) P.osc[m] = rs / scale;
 
     const size_t blk_bytes = (size_t)512 * P.tq;
-    const int tb = m / P.tq, t = m - tb * P.tq;
-    const int b0 = (int)((long long)P.KS * r / C) * 16, b1 = min(P.in / 8, (int)((long long)P.KS * (r + 1) / C) * 16);  // blocks of 8 inputs, whole K steps
+    {
 #pragma unroll 1
-    for (int j = 0; j < P.nmat; j++) {
-        uint8_t* img = P.img[j] + (size_t)tb * P.KS * blk_bytes;
-        const uint4* perm = reinterpret_cast<const uint4*>(P.perm[j]);
-#pragma unroll 1
-        for (int base = b0; base < b1; base += RQ_THREADS) {
-            const int blk = base + tid;
-            if (blk >= b1) break;
+        for (int item = tid; item < items; item += RQ_THREADS) {
+            const int j = item / nb, blk = b0 + (item - j * nb);
+            uint8_t* img = (j == 0 ? P.img[0] : j == 1 ? P.img[1] : P.img[2]) + (size_t)tb * P.KS * blk_bytes;
             float v[8];
-            {
-                if (perm) {
-                    const uint4 ix = __ldg(perm + blk);
-                    v[0] = xs[ix.x & 0xFFFFu]; v[1] = xs[ix.x >> 16]; v[2] = xs[ix.y & 0xFFFFu]; v[3] = xs[ix.y >> 16];
-                    v[4] = xs[ix.z & 0xFFFFu]; v[5] = xs[ix.z >> 16]; v[6] = xs[ix.w & 0xFFFFu]; v[7] = xs[ix.w >> 16];
-                } else {
-                    const float4 a = reinterpret_cast<const float4*>(xs)[2 * blk], b = reinterpret_cast<const float4*>(xs)[2 * blk + 1];
-                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                }
+            if (P.perm[0]) {  // (a launch's rows are all permuted or none is)
+                const uint4 ix = item == tid ? perm0 : perm_of(item);
+                v[0] = xs[ix.x & 0xFFFFu]; v[1] = xs[ix.x >> 16]; v[2] = xs[ix.y & 0xFFFFu]; v[3] = xs[ix.y >> 16];
+                v[4] = xs[ix.z & 0xFFFFu]; v[5] = xs[ix.z >> 16]; v[6] = xs[ix.w & 0xFFFFu]; v[7] = xs[ix.w >> 16];
+            } else {
+                const float4 a = reinterpret_cast<const float4*>(xs)[2 * blk], b = reinterpret_cast<const float4*>(xs)[2 * blk + 1];
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
             }
             uint32_t hi[4], lo[4];
             constexpr int order[8] = {0, 4, 1, 5, 2, 6, 3, 7};
@@ -166,7 +171,7 @@ __device__ __forceinline__ void rotate4(const float4& a, const float4& b, const 
 __global__ void __launch_bounds__(256) rope_append_kernel(const __grid_constant__ RopeParams P) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int m = blockIdx.x, pos = P.pos[m];
+    const int m = blockIdx.x, pos = P.pos[m], tb = m / P.q.tq;
     const int KV = P.kv_stride ? P.kv_stride : P.n_kv_heads * HS;
     const int nq = P.n_heads * (HS / 8), nk = P.n_kv_heads * (HS / 8);  // units of four pairs
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < nq + 2 * nk; i += gridDim.y * blockDim.x) {
@@ -174,14 +179,14 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const __grid_constant_
         if (i < nq + nk) {
             const float4 c = *reinterpret_cast<const float4*>(P.rope_cos + (size_t)pos * (HS / 2) + e), s = *reinterpret_cast<const float4*>(P.rope_sin + (size_t)pos * (HS / 2) + e);
             const TcOut& T = i < nq ? P.q : P.k;
-            const float4 a = tc_load4(T, m, o), b = tc_load4(T, m, o + HS / 2);
+            const float4 a = tc_load4(T, m, tb, o), b = tc_load4(T, m, tb, o + HS / 2);
             float4 na, nb;
             rotate4(a, b, c, s, na, nb);
             float* dst = i < nq ? P.qout + (size_t)m * P.ldq + o : P.kc + (size_t)pos * KV + o;
             *reinterpret_cast<float4*>(dst) = na;
             *reinterpret_cast<float4*>(dst + HS / 2) = nb;
         } else {
-            const float4 a = tc_load4(P.v, m, o), b = tc_load4(P.v, m, o + HS / 2);
+            const float4 a = tc_load4(P.v, m, tb, o), b = tc_load4(P.v, m, tb, o + HS / 2);
             float* dst = P.vc + (size_t)pos * KV + o;
             *reinterpret_cast<float4*>(dst) = a;
             *reinterpret_cast<float4*>(dst + HS / 2) = b;
@@ -454,12 +459,12 @@ void launch_tp_gather(const TpGatherParams& p, cudaStream_t st) {
 __global__ void __launch_bounds__(256) finish_kernel(TcOut a, TcOut b, int pair, float* dst, int ld, int add) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 4, m = blockIdx.y;
+    const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 4, m = blockIdx.y, tb = m / a.tq;
     if (o >= a.rows) return;
-    if (dst == a.out && tc_slices(a, m, o) == 1) return;
-    float4 v = tc_load4(a, m, o);
+    if (dst == a.out && tc_slices(a, tb, o) == 1) return;
+    float4 v = tc_load4(a, m, tb, o);
     if (pair) {  // src/models.rs:92-98
-        const float4 w = tc_load4(b, m, o);
+        const float4 w = tc_load4(b, m, tb, o);
         v.x = (v.x * (1.0f / (1.0f + expf(-v.x)))) * w.x; v.y = (v.y * (1.0f / (1.0f + expf(-v.y)))) * w.y;
         v.z = (v.z * (1.0f / (1.0f + expf(-v.z)))) * w.z; v.w = (v.w * (1.0f / (1.0f + expf(-v.w)))) * w.w;
     }
