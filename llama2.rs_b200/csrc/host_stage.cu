@@ -5,10 +5,11 @@
 
 namespace l2 {
 
-static bool is_pinned(const void* p) {
+// Pinned arrays need no staging; a device pointer is left to the copy, which refuses it.
+static bool direct_copy(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost;
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeDevice;
 }
 
 HostStage::~HostStage() {
@@ -18,13 +19,13 @@ HostStage::~HostStage() {
 
 int HostStage::init(int device) {
     device_ = device;
-    L2_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pin_), CHUNK * SLOTS));
+    L2_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pin_), CHUNK * SLOTS + 64));
     for (cudaEvent_t& e : done_) L2_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return L2_OK;
 }
 
 int HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (is_pinned(src)) {  // the caller's array itself is the staging memory
+    if (direct_copy(src)) {  // the caller's array itself is the staging memory
         L2_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return L2_OK;
     }
@@ -39,10 +40,13 @@ int HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
     return L2_OK;
 }
 
-int HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (is_pinned(dst)) {
+int HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t st, const int* word_dev, int* word) {
+    volatile int* pin_word = reinterpret_cast<int*>(pin_ + CHUNK * SLOTS);  // (in front of the data on the stream: there when the data is)
+    if (word_dev) L2_CUDA(cudaMemcpyAsync(pin_ + CHUNK * SLOTS, word_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (direct_copy(dst)) {
         L2_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         L2_CUDA(cudaStreamSynchronize(st));
+        if (word_dev) *word = *pin_word;
         return L2_OK;
     }
     const int chunks = (int)((bytes + CHUNK - 1) / CHUNK);
@@ -61,6 +65,7 @@ int HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t s
         if (i + SLOTS < chunks)
             if (int rc = request(i + SLOTS)) return rc;
     }
+    if (word_dev) *word = *pin_word;
     return L2_OK;
 }
 
