@@ -396,7 +396,8 @@ __device__ float stage_digits_pair(const SkSeg& sa, const SkSeg& sb, int in, flo
 // Layout in shared memory: digits [4 planes][pstride], plane 0 the most significant digit, a plane holding
 // the K orders of the phase's matrices one after the other; sp [groups] records of four words
 // {256 * S0 + S1, f * 2^16, 256 * S2 + S3, f}: the digit sums of the upper and of the lower digit pair, each
-// followed by the factor its MMA columns are scaled with (f = 2^-(26 - E_g); the upper pair weighs 2^16 more).
+// followed by the factor its MMA columns are scaled with (f = 2^-(26 - E_g); the upper pair weighs 2^16 more).  For groups of 64
+// and 128 the sums are stored times 16 and the factors over 16 (the main loop leaves high nibbles in place).
 
 // Turns 8 values of K-order block `blk` into digits and finishes the group's record.
 template <int W>
@@ -439,8 +440,11 @@ __device__ __forceinline__ void stage_emit8(float (&v)[8], bool valid, int blk, 
         s23 += __shfl_xor_sync(0xffffffffu, s23, o);
     }
     if (valid && (threadIdx.x & (4 * W - 1)) == 0) {
-        const uint32_t f = (254u << 23) - __float_as_uint(P);  // 1 / P, exact (P is a power of two)
-        sp[blk / (4 * W)] = make_uint4((uint32_t)s01, f + (16u << 23), (uint32_t)s23, f);
+        // 1 / P, exact (P is a power of two between 2^-100 and 2^100, so nothing below leaves the range); where the main loop works
+        // with 16 times the integers, the sums and the factor follow
+        constexpr int X16 = W >= 2 ? 4 : 0;
+        const uint32_t f = ((254u - X16) << 23) - __float_as_uint(P);
+        sp[blk / (4 * W)] = make_uint4((uint32_t)s01 << X16, f + (16u << 23), (uint32_t)s23 << X16, f);
     }
 }
 

@@ -271,34 +271,45 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
     // ---- main loop.  In every slot fill this warp owns units 2*warp and 2*warp + 1; unit u of the CTA is group
     // u % Gs of tile u / Gs (the groups of w1 and of w3 of a tile follow one another).  The loop is bound by
     // instruction issue (16 warps run it on 4 schedulers), so it is straight-line code on 32-bit shared-space
-    // addresses: all lanes run the scale / zero-point step (lanes t >= 2 hold the unused MMA columns and are ignored
-    // when the sums are written), lanes r >= 4 read their digits from a block of zeros instead of skipping the load;
-    // in the last, partial fill of a phase the units beyond the end are multiplied all the same (the slot holds older
-    // records there) and only their sums are left out.  Row sums stay in registers while consecutive units belong to
-    // the same (tile, matrix) and go to shared memory when that changes.
-    const int r = lane >> 2, t = lane & 3;
+    // addresses, and the pair shares one set of accumulators: the four digits of the first unit are columns 0-3 of the
+    // MMAs, those of the second columns 4-7 (the other unit's columns multiply a block of zeros), so that lanes t < 2 hold
+    // the first unit's sums and lanes t >= 2 the second's, and the scale / zero-point step runs once for both.  Low and
+    // high nibbles have their own MMAs: a high nibble stays where it is in its byte and counts 16 times, which the
+    // combination makes up for (16 * low + high, 16 times the group's integer; its record carries the digit sums
+    // times 16 and the factors over 16, see stage_emit8).  Per pair that is 110 instructions (group of 128) where a step per unit with
+    // shifted nibbles took 160.  In the last, partial fill of a phase the units beyond the end are multiplied all the same (the
+    // slot holds older records there) and only their sums are left out.  Row sums stay in registers while consecutive units
+    // belong to the same (tile, matrix) and go to shared memory when that changes.
+    const int r = lane >> 2, t = lane & 3, half = t >> 1;  // row (and column of B), column pair, unit of the pair that the sums belong to
     const uint32_t zshift = 4u * (uint32_t)r;
-    const uint32_t w_lane = r_base + (uint32_t)(2 * warp) * UB + (uint32_t)lane * 16u;            // this lane's weights of unit 0 in slot 0
-    const uint32_t m_lane = r_base + (uint32_t)(2 * warp) * UB + 256u * W + 4u * (uint32_t)r;     // its two scales (and, + 64 - 4r, the zero-point words)
-    const uint32_t z_warp = r_base + (uint32_t)(2 * warp) * UB + 256u * W + 64u;
-    const uint32_t dg_lane = r < 4 ? smem_u32(digits) + (uint32_t)(r * pstride + t * (8 * W)) : r_zeros;
-    const uint32_t dstep = r < 4 ? (uint32_t)GS : 0u;
+    const uint32_t w_lane = r_base + (uint32_t)(2 * warp) * UB + (uint32_t)lane * (4u * W);             // this lane's weights of the first unit in slot 0
+    const uint32_t m_lane = r_base + (uint32_t)(2 * warp + half) * UB + 256u * W + 4u * (uint32_t)r;    // its two scales
+    const uint32_t z_lane = r_base + (uint32_t)(2 * warp + half) * UB + 256u * W + 64u;                 // the zero-point words
+    const uint32_t dg_lane = smem_u32(digits) + (uint32_t)((r & 3) * pstride + t * (8 * W));
     const uint32_t sp_lane = smem_u32(sp) + 8u * (uint32_t)(t & 1);
     const uint32_t part_lane = smem_u32(partial) + 4u * (uint32_t)(warp * PROWS + r);
     float tot0 = 0.f, tot1 = 0.f;
     uint32_t cur_dst = 0;  // where the running row sums belong (0: nothing accumulated yet)
-    auto flush = [&]() {   // lanes t = 0 hold digits 0,1 (already scaled by 2^16), lanes t = 1 digits 2,3
+    // lanes t = 0 / 2 hold digits 0,1 (already scaled by 2^16), lanes t = 1 / 3 digits 2,3; the two units' sums of a row are added in that order
+    auto flush = [&](bool go) {
         const float a = tot0 + __shfl_xor_sync(0xffffffffu, tot0, 1), b = tot1 + __shfl_xor_sync(0xffffffffu, tot1, 1);
-        if (t == 0) {
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(cur_dst), "f"(a) : "memory");
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(cur_dst + 32u), "f"(b) : "memory");
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (go && cur_dst && t == 2 * h) {
+                const float p0 = __uint_as_float(lds32(cur_dst)), p1 = __uint_as_float(lds32(cur_dst + 32u));
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(cur_dst), "f"(p0 + a) : "memory");
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(cur_dst + 32u), "f"(p1 + b) : "memory");
+            }
+            __syncwarp();
         }
     };
-    constexpr uint32_t M = 0x0F0F0F0Fu;
-    // position of this warp's first unit of the current fill: group f0 of the tile's Gs, tile tile0
-    int f0 = 2 * warp, tile0 = 0;
-    while (f0 >= Gs) { f0 -= Gs; tile0++; }
-    int rem = n - 2 * warp;  // units of this warp's stride that are left, counted from its first of the current fill
+    constexpr uint32_t M = 0x0F0F0F0Fu, MH = 0xF0F0F0F0u;
+    // groups (of the tile's Gs) of the unit whose digits this lane loads and of the unit whose sums it holds; the latter's tile
+    int fb = 2 * warp + (r >> 2), fs = 2 * warp + half, tile = 0, fstep = SU, tstep = 0;
+    while (fb >= Gs) fb -= Gs;
+    while (fs >= Gs) { fs -= Gs; tile++; }
+    while (fstep >= Gs) { fstep -= Gs; tstep++; }
+    int rem = n - 2 * warp - half;  // units of this lane's stride that are left
     uint32_t fslot = kbase & 0xFFFFu, fpar = kbase >> 16;  // slot and parity of the next fill, carried from phase to phase
     bool ok = true;
 #pragma unroll 1
@@ -314,11 +325,9 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
         }
         if (!(skip & 1)) {
             const uint32_t so = fslot * SLOT_BYTES;
-            int f1 = f0 + 1, tile1 = tile0;
-            if (f1 == Gs) { f1 = 0; tile1++; }
-            // operands of both units: weights (two 16-row halves), digits, scales, zero points, group record
+            // operands of both units: weights (two 16-row halves), digits; scales, zero points and group record of this lane's unit
             uint32_t a0[W], b0[W], a1[W], b1[W], d0[2 * W], d1[2 * W];
-            const uint32_t dg0 = dg_lane + (uint32_t)f0 * dstep, dg1 = dg_lane + (uint32_t)f1 * dstep;
+            const uint32_t dg = dg_lane + (uint32_t)fb * GS, dg0 = r < 4 ? dg : r_zeros, dg1 = r < 4 ? r_zeros : dg;
             if constexpr (W == 4) {
                 const uint4 x0 = lds128(w_lane + so), y0 = lds128(w_lane + so + 512), x1 = lds128(w_lane + so + UB), y1 = lds128(w_lane + so + UB + 512);
                 const uint4 p0 = lds128(dg0), q0 = lds128(dg0 + 16), p1 = lds128(dg1), q1 = lds128(dg1 + 16);
@@ -327,78 +336,67 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
                 d0[0] = p0.x; d0[1] = p0.y; d0[2] = p0.z; d0[3] = p0.w; d0[4] = q0.x; d0[5] = q0.y; d0[6] = q0.z; d0[7] = q0.w;
                 d1[0] = p1.x; d1[1] = p1.y; d1[2] = p1.z; d1[3] = p1.w; d1[4] = q1.x; d1[5] = q1.y; d1[6] = q1.z; d1[7] = q1.w;
             } else if constexpr (W == 2) {
-                const uint32_t wl = w_lane - (uint32_t)lane * 8u;  // 8 bytes per lane and half
-                const uint2 x0 = lds64(wl + so), y0 = lds64(wl + so + 256), x1 = lds64(wl + so + UB), y1 = lds64(wl + so + UB + 256);
+                const uint2 x0 = lds64(w_lane + so), y0 = lds64(w_lane + so + 256), x1 = lds64(w_lane + so + UB), y1 = lds64(w_lane + so + UB + 256);
                 const uint4 p0 = lds128(dg0), p1 = lds128(dg1);
                 a0[0] = x0.x; a0[1] = x0.y; b0[0] = y0.x; b0[1] = y0.y; a1[0] = x1.x; a1[1] = x1.y; b1[0] = y1.x; b1[1] = y1.y;
                 d0[0] = p0.x; d0[1] = p0.y; d0[2] = p0.z; d0[3] = p0.w; d1[0] = p1.x; d1[1] = p1.y; d1[2] = p1.z; d1[3] = p1.w;
             } else {
-                const uint32_t wl = w_lane - (uint32_t)lane * 12u;  // 4 bytes per lane and half
-                a0[0] = lds32(wl + so); b0[0] = lds32(wl + so + 128); a1[0] = lds32(wl + so + UB); b1[0] = lds32(wl + so + UB + 128);
+                a0[0] = lds32(w_lane + so); b0[0] = lds32(w_lane + so + 128); a1[0] = lds32(w_lane + so + UB); b1[0] = lds32(w_lane + so + UB + 128);
                 const uint2 p0 = lds64(dg0), p1 = lds64(dg1);
                 d0[0] = p0.x; d0[1] = p0.y; d1[0] = p1.x; d1[1] = p1.y;
             }
-            const uint32_t s00 = lds32(m_lane + so), s01 = lds32(m_lane + so + 32), s10 = lds32(m_lane + so + UB), s11 = lds32(m_lane + so + UB + 32);
-            const uint2 zz0 = lds64(z_warp + so), zz1 = lds64(z_warp + so + UB);
-            const uint2 g0 = lds64(sp_lane + 16u * (uint32_t)f0), g1 = lds64(sp_lane + 16u * (uint32_t)f1);  // {digit sums of this lane's columns, their factor}
-            // The MMAs of the pair are independent instructions issued back to back (even and odd K steps of a unit have
-            // their own accumulators): an integer mma.sync that depends on the previous one of its warp occupies the
-            // tensor pipe about four times as long as one that follows an independent one.
-            int c0[4], c1[4];
+            const uint32_t s0 = lds32(m_lane + so), s1 = lds32(m_lane + so + 32);
+            const uint2 zz = lds64(z_lane + so);
+            const uint2 g = lds64(sp_lane + 16u * (uint32_t)fs);  // {digit sums of this lane's columns, their factor}
+            // Four independent MMAs, then four that add to them: an integer mma.sync that depends on the previous one of its
+            // warp occupies the tensor pipe about four times as long as one that follows an independent one.
+            int c[4];
             if constexpr (W == 1) {
-                mma_u8s8_first(c0, a0[0] & M, b0[0] & M, (a0[0] >> 4) & M, (b0[0] >> 4) & M, d0[0], d0[1]);
-                mma_u8s8_first(c1, a1[0] & M, b1[0] & M, (a1[0] >> 4) & M, (b1[0] >> 4) & M, d1[0], d1[1]);
+                int e[4];
+                mma_u8s8_first(c, a0[0] & M, b0[0] & M, (a0[0] >> 4) & M, (b0[0] >> 4) & M, d0[0], d0[1]);
+                mma_u8s8_first(e, a1[0] & M, b1[0] & M, (a1[0] >> 4) & M, (b1[0] >> 4) & M, d1[0], d1[1]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) c[j] += e[j];
             } else {
-                int e0[4], e1[4];
-                mma_u8s8_first(c0, a0[0] & M, b0[0] & M, (a0[0] >> 4) & M, (b0[0] >> 4) & M, d0[0], d0[1]);
-                mma_u8s8_first(e0, a0[1] & M, b0[1] & M, (a0[1] >> 4) & M, (b0[1] >> 4) & M, d0[2], d0[3]);
-                mma_u8s8_first(c1, a1[0] & M, b1[0] & M, (a1[0] >> 4) & M, (b1[0] >> 4) & M, d1[0], d1[1]);
-                mma_u8s8_first(e1, a1[1] & M, b1[1] & M, (a1[1] >> 4) & M, (b1[1] >> 4) & M, d1[2], d1[3]);
-#pragma unroll
-                for (int i = 2; i < W; i += 2) {
-                    mma_u8s8(c0, a0[i] & M, b0[i] & M, (a0[i] >> 4) & M, (b0[i] >> 4) & M, d0[2 * i], d0[2 * i + 1]);
-                    mma_u8s8(e0, a0[i + 1] & M, b0[i + 1] & M, (a0[i + 1] >> 4) & M, (b0[i + 1] >> 4) & M, d0[2 * i + 2], d0[2 * i + 3]);
-                    mma_u8s8(c1, a1[i] & M, b1[i] & M, (a1[i] >> 4) & M, (b1[i] >> 4) & M, d1[2 * i], d1[2 * i + 1]);
-                    mma_u8s8(e1, a1[i + 1] & M, b1[i + 1] & M, (a1[i + 1] >> 4) & M, (b1[i + 1] >> 4) & M, d1[2 * i + 2], d1[2 * i + 3]);
+                int l0[4], l1[4], h0[4], h1[4];
+                mma_u8s8_first(l0, a0[0] & M, b0[0] & M, a0[1] & M, b0[1] & M, d0[0], d0[2]);
+                mma_u8s8_first(h0, a0[0] & MH, b0[0] & MH, a0[1] & MH, b0[1] & MH, d0[1], d0[3]);
+                mma_u8s8_first(l1, a1[0] & M, b1[0] & M, a1[1] & M, b1[1] & M, d1[0], d1[2]);
+                mma_u8s8_first(h1, a1[0] & MH, b1[0] & MH, a1[1] & MH, b1[1] & MH, d1[1], d1[3]);
+                if constexpr (W == 4) {
+                    mma_u8s8(l0, a0[2] & M, b0[2] & M, a0[3] & M, b0[3] & M, d0[4], d0[6]);
+                    mma_u8s8(h0, a0[2] & MH, b0[2] & MH, a0[3] & MH, b0[3] & MH, d0[5], d0[7]);
+                    mma_u8s8(l1, a1[2] & M, b1[2] & M, a1[3] & M, b1[3] & M, d1[4], d1[6]);
+                    mma_u8s8(h1, a1[2] & MH, b1[2] & MH, a1[3] & MH, b1[3] & MH, d1[5], d1[7]);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; j++) { c0[j] += e0[j]; c1[j] += e1[j]; }
+                for (int j = 0; j < 4; j++) c[j] = (l0[j] + l1[j]) * 16 + (h0[j] + h1[j]);
             }
-            // scale, zero point and digit sums of the finished units (exact integers up to the final FMA)
-            if (rem > 0) {
-                const uint32_t dst = part_lane + (uint32_t)tile0 * (SK_WARPS * PROWS * 4u) + (f0 >= G ? 64u : 0u);
-                if (dst != cur_dst) {  // warp-uniform
-                    if (cur_dst) flush();
-                    cur_dst = dst;
-                    tot0 = tot1 = 0.f;
-                }
-                const int za = (int)((zz0.x >> zshift) & 15u) + 1, zb = (int)((zz0.y >> zshift) & 15u) + 1;  // src/gptq.rs:148
-                const float pf = __uint_as_float(g0.y);  // a power of two: the products below are exact scalings
-                tot0 = fmaf(__uint_as_float(s00) * pf, (float)(c0[0] * 256 + c0[1] - za * (int)g0.x), tot0);
-                tot1 = fmaf(__uint_as_float(s01) * pf, (float)(c0[2] * 256 + c0[3] - zb * (int)g0.x), tot1);
+            // scale, zero point and digit sums of this lane's unit (exact integers below 2^31 up to the final FMA)
+            const bool live = rem > 0;
+            const uint32_t dst = live ? part_lane + (uint32_t)tile * (SK_WARPS * PROWS * 4u) + (fs >= G ? 64u : 0u) : cur_dst;
+            if (__any_sync(0xffffffffu, dst != cur_dst)) {
+                flush(dst != cur_dst);
+                if (dst != cur_dst) { cur_dst = dst; tot0 = tot1 = 0.f; }
             }
-            if (rem > 1) {
-                const uint32_t dst = part_lane + (uint32_t)tile1 * (SK_WARPS * PROWS * 4u) + (f1 >= G ? 64u : 0u);
-                if (dst != cur_dst) {
-                    if (cur_dst) flush();
-                    cur_dst = dst;
-                    tot0 = tot1 = 0.f;
-                }
-                const int za = (int)((zz1.x >> zshift) & 15u) + 1, zb = (int)((zz1.y >> zshift) & 15u) + 1;
-                const float pf = __uint_as_float(g1.y);
-                tot0 = fmaf(__uint_as_float(s10) * pf, (float)(c1[0] * 256 + c1[1] - za * (int)g1.x), tot0);
-                tot1 = fmaf(__uint_as_float(s11) * pf, (float)(c1[2] * 256 + c1[3] - zb * (int)g1.x), tot1);
+            if (live) {
+                const int za = (int)((zz.x >> zshift) & 15u) + 1, zb = (int)((zz.y >> zshift) & 15u) + 1;  // src/gptq.rs:148
+                const float pf = __uint_as_float(g.y);  // a power of two: the products below are exact scalings
+                tot0 = fmaf(__uint_as_float(s0) * pf, (float)(c[0] * 256 + c[1] - za * (int)g.x), tot0);
+                tot1 = fmaf(__uint_as_float(s1) * pf, (float)(c[2] * 256 + c[3] - zb * (int)g.x), tot1);
             }
         }
         __syncwarp();  // every lane has read the slot
         if (lane == 0) mbar_arrive_u32(r_empty + 8u * fslot);
         rem -= SU;
-        f0 += SU;
-        while (f0 >= Gs) { f0 -= Gs; tile0++; }
+        fb += fstep;
+        if (fb >= Gs) fb -= Gs;
+        fs += fstep; tile += tstep;
+        if (fs >= Gs) { fs -= Gs; tile++; }
         if (++fslot == (uint32_t)NS) { fslot = 0; fpar ^= 1u; }
     }
     kbase = fslot | (fpar << 16);
-    if (cur_dst) flush();
+    flush(true);
     if (stamp && threadIdx.x == 0) { stamp[2] = clock64(); stamp[9] = (unsigned long long)nslots; }
     consumer_sync();
     if (stamp && threadIdx.x == 0) stamp[18] = clock64();
