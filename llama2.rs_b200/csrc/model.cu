@@ -489,9 +489,10 @@ static bool token_path(const l2_state* s) {
 }
 
 // Shared memory in front of the ring (the largest need of any phase) and the ring slots that fit behind it.  The next
-// smaller carve-out (196 KB) leaves 60 KB of L1 instead of 28 KB, which the kernel's local memory (stack, the few spilled
-// registers of 544 threads) and read-only operands need more than a fourth or fifth ring slot (measured: 3 slots of 35 KB beat
-// 5 on the 7B model); the largest carve-out only where the ring would otherwise be shorter than three slots.
+// smaller carve-out (196 KB) leaves 60 KB of L1 instead of 28 KB, which the kernel's read-only operands need more than another ring slot;
+// the largest carve-out only where the ring would otherwise be shorter than three slots.  Within the smaller one every slot counts:
+// the tile sums share memory with the staged vector (token_gemv_smem), which gives the 7B model four slots of 35 KB instead of
+// three (1387 -> 1342 us a token).
 static size_t tk_fixed_bytes(const l2_state* s, bool gather13) {
     const l2_model* m = s->m;
     const l2_config& c = m->shape.c;
@@ -517,9 +518,9 @@ static int tk_slots(const l2_state* s, size_t fixed, int su) {
 }
 // w1 and w3 read one input through two different g_index orders.  Keeping the input once in natural order and gathering each
 // matrix's blocks from it saves 4 * dim bytes of shared memory against two K-ordered copies, at the price of scattered
-// shared-memory reads while the digits are cut.  It is used where it lets three ring slots fit into the smaller carve-out
-// (13B and 70B shapes; measured on the 70B shapes: + 3 %, the same with three slots and 60 KB of L1 as with four slots and
-// 28 KB), or where it buys a slot at all.
+// shared-memory reads while the digits are cut (no difference by itself: 7B with every input gathered 1339 us a token, 70B shapes 0.4 %
+// slower).  It is used where it lets three ring slots fit into the smaller carve-out (13B and 70B shapes: + 3 %), or where it buys a
+// slot (7B).
 static bool tk_gather13(const l2_state* s) {
     const int su = 2 * SK_WARPS;
     if (const char* e = getenv("L2_TK_GATHER13")) return atoi(e) != 0;  // tuning knob

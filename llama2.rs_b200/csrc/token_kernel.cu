@@ -23,6 +23,8 @@
 // free slot or record buffer): a wait that gives up writes a status word, raises the CTA's abort
 // flag, lets copies in flight land and leaves; the other CTAs run into their own limits or see the
 // flag at their next wait and leave too.  The launch is cooperative, so all CTAs are resident together.
+#include <algorithm>
+
 #include "gemv_device.cuh"
 #include "kernels.cuh"
 
@@ -206,9 +208,8 @@ __device__ __forceinline__ void warm_operands(const SkParams& P, int NSEG) {
 size_t token_gemv_smem(int in, int G, int nseg, int ptiles, bool natural, bool gather) {
     size_t b = (size_t)4 * ((size_t)nseg * in + 16);       // digit planes
     b += (size_t)nseg * G * 16;                            // group records
-    if (natural) b += (size_t)(gather ? 1 : nseg) * in * 4;  // the vector as plain floats: in each matrix's K order, or once in natural order
-    b += (size_t)ptiles * SK_WARPS * 32 * 4;               // tile sums per warp
-    return b;
+    // the vector as plain floats (in each matrix's K order, or once in natural order) while it is staged, then the tile sums per warp
+    return b + std::max(natural ? (size_t)(gather ? 1 : nseg) * in * 4 : 0, (size_t)ptiles * SK_WARPS * 32 * 4);
 }
 
 template <int W>
@@ -236,9 +237,8 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
     uint4* sp = reinterpret_cast<uint4*>(smem + (size_t)4 * pstride);    // [nseg * G] group records
     const bool natural = J.seg[0].perm != nullptr;                       // the input arrives in natural order and is gathered into the K order
     float* xs = reinterpret_cast<float*>(sp + Gs);                       // [nseg][in] the vector in each matrix's K order as plain floats (only then)
-    float* partial = xs + (natural ? (J.gather ? 1 : nseg) * J.in : 0);  // [nt][SK_WARPS][PROWS]
+    float* partial = xs;                                                 // [nt][SK_WARPS][PROWS], once the digits are cut
 
-    for (int i = threadIdx.x; i < nt * SK_WARPS * PROWS; i += SK_THREADS) partial[i] = 0.f;
     bool stage_failed = false;  // a poll for a tagged input gave up
     if (stamp && threadIdx.x == 0) stamp[16] = clock64();
     if (n > 0) {
@@ -252,7 +252,9 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
         if (lane == 0) red[warp] = sq;
     }
     if (stage_failed) ring_abort(R, 1010);
-    consumer_sync();  // digits and group records are in place; so are the zeroed tile sums
+    consumer_sync();  // digits and group records are in place, the vector has been used
+    for (int tl = 0; tl < nt; tl++) partial[(tl * SK_WARPS + warp) * PROWS + lane] = 0.f;  // a warp's own sums
+    __syncwarp();
     if (warp == 0) {  // rmsnorm factor of the input (src/models.rs:58-60), read by the epilogue; the digit scaling is already in the sums
         float total = tk_warp_sum(lane < SK_WARPS ? red[lane] : 0.f);
         if (lane == 0) oscale[0] = J.seg[0].nw ? 1.0f / sqrtf(total / (float)J.in + P.eps) : 1.0f;
