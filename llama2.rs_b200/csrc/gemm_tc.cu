@@ -1,5 +1,5 @@
 // Batched QLinear::matvec<B> (src/gptq.rs:94-176) for B >= 2 as a dense contraction on the
-// 5th-generation tensor cores: tcgen05.mma kind::i8 with accumulators in tensor memory.
+// 5th-generation tensor cores: tcgen05.mma kind::f16 on exact integer digits, weights and accumulators in tensor memory.
 //
 //   out[m][o] = f[m] * sum_g scale[o][g] * sum_{k in g} (q[o][k] - z[o][g]) * X[m][k]
 //

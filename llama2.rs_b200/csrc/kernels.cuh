@@ -279,7 +279,7 @@ cudaError_t sk_init(int max_smem);
 void launch_embed_batch(const float* table, const int* tokens, float* x, int dim, int M, cudaStream_t st);
 cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st);
 cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st);
-void launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, cudaStream_t st);
+cudaError_t launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, int sms, cudaStream_t st);
 void launch_tp_gather(const TpGatherParams& p, cudaStream_t st);
 // dst[m][ld] (+)= the output of a GEMM, slices added in order; with b: dst = silu(a) * b
 void launch_finish(const TcOut& a, const TcOut* b, float* dst, int ld, bool add, cudaStream_t st);

@@ -193,7 +193,7 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
         AttnBatchParams a{};
         a.q = b->q; a.kc = r.kc; a.vc = r.vc; a.pos = pos; a.out = b->att + (size_t)R * Dl;
         a.n_kv_heads = kvh_l; a.ag = m->shape.attn_groups(); a.ldq = Dl; a.ldo = D; a.kv_stride = KV;
-        launch_attn_batch(a, heads_l, M, long_context, st);
+        L2_CUDA(launch_attn_batch(a, heads_l, M, long_context, m->sms, st));
         gather(1, D, R * Dl, Dl);
         // wo + residual (:260-264)
         launch({&y.wo}, t);

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 
 #include "kernels.cuh"
@@ -379,32 +380,222 @@ __global__ void __launch_bounds__(32 * AT_WARPS) attn_batch_tiled_kernel(const _
     }
 }
 
-template <int AG, int NQW>
-static void launch_attn_tiled(const AttnBatchParams& p, int M, cudaStream_t st) {
-    constexpr int QB = AT_WARPS * (NQW / AG);
-    const size_t smem = (size_t)(AT_WARPS * NQW * HS + AT_TILE * AT_KPAD + AT_TILE * HS) * sizeof(float);
-    launch_pdl(attn_batch_tiled_kernel<AG, NQW>, dim3(p.n_kv_heads, (M + QB - 1) / QB), dim3(32 * AT_WARPS), smem, 0, st, p, M);
+// ---- the same for many queries: 16 per warp ------------------------------------------------------------------------------
+// What bounds the kernel above is the way from shared memory into registers: 128 bytes per clock, broadcasts included, so a 16-byte load of a warp
+// costs 4 clocks and feeds as many FMA clocks as there are values to combine it with (9 loads per 32 FMAs for the scores, a load and 8
+// shuffles per 32 for the values: 1880 clocks per 8 queries and tile).  Hence register tiles:
+//   scores: lane (pi, qi) has positions pi + 8 j (j < 4) of queries qi + 4 u (u < 4): 8 loads per 64 FMAs;
+//   values: lane (half, dl) has dimensions 4 dl .. + 3 and 64 + 4 dl .. + 3 of 8 queries: 4 loads per 64 FMAs (the probabilities come
+//   from shared memory, where the lanes that computed them put them).
+// Rows of K are padded: the lanes of a load read different banks.  The shared memory is small enough for three CTAs per SM, so that the
+// copies of one tile overlap the arithmetic of others.
+constexpr int AW_WARPS = 4, AW_QW = 16, AW_PP = AW_QW + 4;
+constexpr int AW_FLOATS = AW_WARPS * AW_QW * HS + AT_TILE * (AT_KPAD + HS) + AW_WARPS * AT_TILE * AW_PP;
+static_assert(3 * (AW_FLOATS * 4 + 1024) <= 228 * 1024, "three CTAs per SM");
+
+__device__ __forceinline__ float2 at_fma2(const float2& a, const float2& b, const float2& c) {
+    float2 d;
+    asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ void at_copy16(float* dst, const float4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-// the tiled kernel's shared memory (65 KB at most) is above the default limit: once per device, at start-up
+template <int AG>  // query heads per kv head
+__global__ void __launch_bounds__(32 * AW_WARPS, 3) attn_batch_wide_kernel(const __grid_constant__ AttnBatchParams P, int M) {
+    extern __shared__ __align__(16) float at_smem[];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int TPW = AW_QW / AG, QB = AW_WARPS * TPW;        // tokens per warp, per CTA
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* Qs = at_smem;                                     // [AW_WARPS * 16][HS]
+    float* Ks = Qs + AW_WARPS * AW_QW * HS;                     // [AT_TILE][AT_KPAD]
+    float* Vs = Ks + AT_TILE * AT_KPAD;                     // [AT_TILE][HS]
+    float* Ps = Vs + AT_TILE * HS + warp * AT_TILE * AW_PP;  // [AT_TILE][AW_PP] this warp's probabilities by place; behind them in rows 0-3
+    float* Cs = Ps + AW_QW;                                  // a factor, in rows 4-7 the last position of the query in place 4 row + column
+    int* Ls = reinterpret_cast<int*>(Cs + 4 * AW_PP);
+    const int kvh = blockIdx.x, m0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * QB;  // (the blocks with the longest way start first)
+    const int KV = P.kv_stride ? P.kv_stride : P.n_kv_heads * HS;
+    const float div = sqrtf((float)HS);
+    // queries of this CTA: query i = (token m0 + i / AG, head kvh * AG + i % AG)
+    for (int i = tid; i < AW_WARPS * AW_QW * (HS / 4); i += 32 * AW_WARPS) {
+        const int qi = i / (HS / 4), c = i % (HS / 4), m = m0 + qi / AG;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m < M) v = reinterpret_cast<const float4*>(P.q + (size_t)m * P.ldq + (size_t)(kvh * AG + qi % AG) * HS)[c];
+        *reinterpret_cast<float4*>(Qs + qi * HS + 4 * c) = v;
+    }
+    const int pi = lane & 7, qi = lane >> 3;
+    // last position that query qi + 4 u attends to (-1: no such token); the last and the first of the warp's; the last of the CTA's
+    int last[4], wlast = -1, wfirst = INT_MAX, tmax = -1;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int m = m0 + warp * TPW + (qi + 4 * u) / AG;
+        last[u] = m < M ? P.pos[m] : -1;
+    }
+    if (pi == 0) *reinterpret_cast<int4*>(Ls + qi * AW_PP) = make_int4(last[0], last[1], last[2], last[3]);  // query qi + 4 u has place 4 qi + u
+    for (int m = m0 + warp * TPW; m < min(M, m0 + (warp + 1) * TPW); m++) { wlast = max(wlast, P.pos[m]); wfirst = min(wfirst, P.pos[m]); }
+    for (int m = m0; m < min(M, m0 + QB); m++) tmax = max(tmax, P.pos[m]);
+    float mx[4], l[4];
+    float2 acc[8][4];  // 8 queries x 8 dimensions
+#pragma unroll
+    for (int u = 0; u < 4; u++) { mx[u] = -INFINITY; l[u] = 0.f; }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[q][i] = make_float2(0.f, 0.f);
+    const int half = lane >> 4, dl = lane & 15;
+    const float4* kc = reinterpret_cast<const float4*>(P.kc) + (size_t)kvh * (HS / 4);
+    const float4* vc = reinterpret_cast<const float4*>(P.vc) + (size_t)kvh * (HS / 4);
+    const size_t rs = (size_t)KV / 4;
+    const float* krow = Ks + pi * AT_KPAD;
+    const float* qrow = Qs + (warp * AW_QW + qi) * HS;
+    for (int t0 = 0; t0 <= tmax; t0 += AT_TILE) {
+        __syncthreads();  // the previous tile has been used
+        for (int i = tid; i < AT_TILE * (HS / 4); i += 32 * AW_WARPS) {
+            const int r = i / (HS / 4), c = i % (HS / 4), t = min(t0 + r, tmax);  // (rows beyond the last are not used)
+            at_copy16(Ks + r * AT_KPAD + 4 * c, kc + (size_t)t * rs + c);
+            at_copy16(Vs + r * HS + 4 * c, vc + (size_t)t * rs + c);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (t0 > wlast) continue;
+        float2 s2[4][4];  // [position][query], even and odd dimensions
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) s2[j][u] = make_float2(0.f, 0.f);
+#pragma unroll 2
+        for (int c = 0; c < HS; c += 4) {
+            float4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = *reinterpret_cast<const float4*>(qrow + 4 * u * HS + c);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 k = *reinterpret_cast<const float4*>(krow + 8 * j * AT_KPAD + c);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    s2[j][u] = at_fma2(make_float2(q[u].x, q[u].y), make_float2(k.x, k.y), s2[j][u]);
+                    s2[j][u] = at_fma2(make_float2(q[u].z, q[u].w), make_float2(k.z, k.w), s2[j][u]);
+                }
+            }
+        }
+        // online softmax: one rescale per tile; a query's 32 scores are in 8 lanes
+        float p[4][4], corr[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            float tm = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                p[j][u] = t0 + pi + 8 * j <= last[u] ? __fdiv_rn(s2[j][u].x + s2[j][u].y, div) : -INFINITY;  // src/models.rs:158
+                tm = fmaxf(tm, p[j][u]);
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
+            const float mn = fmaxf(mx[u], tm);
+            corr[u] = mn == -INFINITY ? 1.f : expf(mx[u] - mn);
+            float ps = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                p[j][u] = t0 + pi + 8 * j <= last[u] ? expf(p[j][u] - mn) : 0.f;
+                ps += p[j][u];
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
+            l[u] = l[u] * corr[u] + ps;
+            mx[u] = mn;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) *reinterpret_cast<float4*>(Ps + (pi + 8 * j) * AW_PP + 4 * qi) = make_float4(p[j][0], p[j][1], p[j][2], p[j][3]);
+        if (pi == 0) *reinterpret_cast<float4*>(Cs + qi * AW_PP) = make_float4(corr[0], corr[1], corr[2], corr[3]);
+        __syncwarp();
+        {
+            const float4 c0 = *reinterpret_cast<const float4*>(Cs + 2 * half * AW_PP), c1 = *reinterpret_cast<const float4*>(Cs + (2 * half + 1) * AW_PP);
+            const float f[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) { acc[q][i].x *= f[q]; acc[q][i].y *= f[q]; }
+        }
+        auto values = [&](int t, auto&& attends) {
+            const float4 v0 = *reinterpret_cast<const float4*>(Vs + t * HS + 4 * dl), v1 = *reinterpret_cast<const float4*>(Vs + t * HS + HS / 2 + 4 * dl);
+            const float4 p0 = *reinterpret_cast<const float4*>(Ps + t * AW_PP + 8 * half), p1 = *reinterpret_cast<const float4*>(Ps + t * AW_PP + 8 * half + 4);
+            const float f[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (attends(q)) {
+                    const float2 pp = make_float2(f[q], f[q]);
+                    acc[q][0] = at_fma2(pp, make_float2(v0.x, v0.y), acc[q][0]);
+                    acc[q][1] = at_fma2(pp, make_float2(v0.z, v0.w), acc[q][1]);
+                    acc[q][2] = at_fma2(pp, make_float2(v1.x, v1.y), acc[q][2]);
+                    acc[q][3] = at_fma2(pp, make_float2(v1.z, v1.w), acc[q][3]);
+                }
+        };
+        if (t0 + AT_TILE - 1 <= wfirst) {
+#pragma unroll 2
+            for (int t = 0; t < AT_TILE; t++) values(t, [](int) { return true; });
+        } else {  // a row that a query does not attend to is left out, not multiplied by zero: it may hold anything
+            const int4 l0 = *reinterpret_cast<const int4*>(Ls + 2 * half * AW_PP), l1 = *reinterpret_cast<const int4*>(Ls + (2 * half + 1) * AW_PP);
+            const int lq[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll 1
+            for (int t = 0; t < AT_TILE && t0 + t <= wlast; t++) values(t, [&](int q) { return t0 + t <= lq[q]; });
+        }
+        __syncwarp();  // the probabilities have been read
+    }
+    __syncwarp();
+    if (pi == 0) *reinterpret_cast<float4*>(Cs + qi * AW_PP) = make_float4(l[0], l[1], l[2], l[3]);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int place = 8 * half + q, query = (place >> 2) + 4 * (place & 3), m = m0 + warp * TPW + query / AG;
+        if (m < M) {
+            const float inv = 1.0f / Cs[(place >> 2) * AW_PP + (place & 3)];
+            float* o = P.out + (size_t)m * P.ldo + (size_t)(kvh * AG + query % AG) * HS + 4 * dl;
+            *reinterpret_cast<float4*>(o) = make_float4(acc[q][0].x * inv, acc[q][0].y * inv, acc[q][1].x * inv, acc[q][1].y * inv);
+            *reinterpret_cast<float4*>(o + HS / 2) = make_float4(acc[q][2].x * inv, acc[q][2].y * inv, acc[q][3].x * inv, acc[q][3].y * inv);
+        }
+    }
+}
+
+template <int AG, int NQW>
+static cudaError_t launch_attn_tiled(const AttnBatchParams& p, int M, cudaStream_t st) {
+    constexpr int QB = AT_WARPS * (NQW / AG);
+    const size_t smem = (size_t)(AT_WARPS * NQW * HS + AT_TILE * AT_KPAD + AT_TILE * HS) * sizeof(float);
+    return launch_pdl(attn_batch_tiled_kernel<AG, NQW>, dim3(p.n_kv_heads, (M + QB - 1) / QB), dim3(32 * AT_WARPS), smem, 0, st, p, M);
+}
+template <int AG>
+static cudaError_t launch_attn_wide(const AttnBatchParams& p, int M, cudaStream_t st) {
+    constexpr int QB = AW_WARPS * (AW_QW / AG);
+    return launch_pdl(attn_batch_wide_kernel<AG>, dim3(p.n_kv_heads, (M + QB - 1) / QB), dim3(32 * AW_WARPS), AW_FLOATS * sizeof(float), 0, st, p, M);
+}
+
+// the tiled kernels' shared memory (77 KB at most) is above the default limit: once per device, at start-up
 cudaError_t attn_batch_init() {
     const int smem = (AT_WARPS * 8 * HS + AT_TILE * AT_KPAD + AT_TILE * HS) * (int)sizeof(float);
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(attn_batch_tiled_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(attn_batch_tiled_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(attn_batch_tiled_kernel<4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(attn_batch_tiled_kernel<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+#define L2_AT_ATTR(kernel, bytes) if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return e;
+    L2_AT_ATTR((attn_batch_tiled_kernel<1, 4>), smem) L2_AT_ATTR((attn_batch_tiled_kernel<2, 8>), smem)
+    L2_AT_ATTR((attn_batch_tiled_kernel<4, 8>), smem) L2_AT_ATTR((attn_batch_tiled_kernel<8, 8>), smem)
+    const int wide = AW_FLOATS * (int)sizeof(float);
+    L2_AT_ATTR(attn_batch_wide_kernel<1>, wide) L2_AT_ATTR(attn_batch_wide_kernel<2>, wide)
+    L2_AT_ATTR(attn_batch_wide_kernel<4>, wide) L2_AT_ATTR(attn_batch_wide_kernel<8>, wide)
+#undef L2_AT_ATTR
+    return cudaSuccess;
 }
 
-// tiled: the kernel that shares cache tiles among queries (long contexts); otherwise one CTA per (head, token), which has
-// more CTAs and less set-up (short contexts: the cache is small and sits in the L2 anyway)
-void launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, cudaStream_t st) {
+// Short contexts: one CTA per (head, token), which has more CTAs and less set-up (the cache is small and sits in the L2 anyway).  From
+// `tiled` on (about 200 positions), the kernels that share cache tiles among queries: 16 queries per warp where that still gives the SMs
+// three CTAs for every two of them (a batch of 499 tokens of the 7B shapes, 256 CTAs: 2000-token prompt on 16 layers 69.7 -> 61.5 ms; 70B
+// shapes, 512 CTAs: 1536-token prompt on 4 layers 31.3 -> 29.6 ms; 296 tokens of the 7B shapes, 160 CTAs: 15.2 -> 16.2 ms).
+cudaError_t launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, int sms, cudaStream_t st) {
+    const bool wide = (long long)p.n_kv_heads * ((M * p.ag + AW_WARPS * AW_QW - 1) / (AW_WARPS * AW_QW)) * 2 >= 3 * sms;
     switch (tiled ? p.ag : 0) {
-        case 1: launch_attn_tiled<1, 4>(p, M, st); break;
-        case 2: launch_attn_tiled<2, 8>(p, M, st); break;
-        case 4: launch_attn_tiled<4, 8>(p, M, st); break;
-        case 8: launch_attn_tiled<8, 8>(p, M, st); break;
-        default: launch_pdl(attn_batch_kernel, dim3(n_heads, M), dim3(128), 0, 0, st, p); break;
+        case 1: return wide ? launch_attn_wide<1>(p, M, st) : launch_attn_tiled<1, 4>(p, M, st);
+        case 2: return wide ? launch_attn_wide<2>(p, M, st) : launch_attn_tiled<2, 8>(p, M, st);
+        case 4: return wide ? launch_attn_wide<4>(p, M, st) : launch_attn_tiled<4, 8>(p, M, st);
+        case 8: return wide ? launch_attn_wide<8>(p, M, st) : launch_attn_tiled<8, 8>(p, M, st);
+        default: return launch_pdl(attn_batch_kernel, dim3(n_heads, M), dim3(128), 0, 0, st, p);
     }
 }
 // ---- all-gather of a column slice over peer memory (batched forward under tensor parallelism) ----------------------------

@@ -211,3 +211,19 @@ def test_model_shapes_two_layers(l2, orc, name, gs):
     got = l2.generate_ids(gpu, prompt, 9 + 64, trace_logits=True)
     assert_close(got["logits"], want["logits"], what="%s logits" % name)
     assert np.array_equal(got["tokens"], want["tokens"])
+
+
+# 1, 2, 4, 8 query heads per kv head; prompts that end inside a warp's tokens, inside and at the end of a tile of 32 positions, and with
+# more than one CTA per kv head
+@pytest.mark.parametrize("dim,kvh", [(256, 2), (512, 2), (512, 1), (1024, 1)])
+def test_batched_attention_edges(l2, orc, dim, kvh):
+    cfg = tiny_config(l2, group_size=64, n_kv_heads=kvh, dim=dim, hidden=2 * dim, seq_len=256)
+    gpu, cpu = make_pair(l2, orc, cfg, seed=23)
+    rng = np.random.default_rng(dim * kvh)
+    for n in (3, 15, 34, 65, 131):
+        prompt = rng.integers(0, cfg.vocab_size, n).astype(np.int32)
+        want = cpu.generate_ids(prompt, n + 4, trace_logits=True)
+        got = l2.generate_ids(gpu, prompt, n + 4, trace_logits=True)
+        assert got["pos0"] == want["pos0"]
+        assert_close(got["logits"], want["logits"], what="logits after %d prompt tokens" % n)
+        assert np.array_equal(got["tokens"], want["tokens"])
