@@ -46,7 +46,8 @@ __global__ void embed_batch_kernel(const float* __restrict__ table, const int* _
 // share, multiplies by the rmsnorm weight (linearity: the 1/sqrt(mean(x^2)+eps) factor goes into osc) and puts it into the shared
 // memory of all CTAs of the cluster, with its part of the statistics; then every CTA cuts its share of each consumer's K order into
 // digits, gathering from shared memory.  So the row is read once and the statistics (the same for every K order) are taken
-// once, for up to three consumers.
+// once, for up to three consumers.  A row that is in K order already (SwiGLU for w2, the longest of a layer) needs no gathering: a CTA's
+// share is what it cuts, it keeps that alone and nothing but the statistics crosses.
 //
 // Digits: X = round(x * nw * 2^(22 - E)) with E the exponent of the row's largest |x * nw|, so |X| <= 2^23 (the 24 bits of an f32
 // mantissa for the largest element), X = 4096 hi + lo with hi in -2048..2048 and lo in -2048..2047, both exact in f16.  They go into the
@@ -56,15 +57,18 @@ constexpr int RQ_THREADS = 256;
 constexpr int RQ_MAX_CLUSTER = 8;
 
 __global__ void __launch_bounds__(RQ_THREADS, 4) row_quant_kernel(const __grid_constant__ RowParams P) {
-    extern __shared__ __align__(16) float xs[];  // the row (times the norm weight), natural order
+    extern __shared__ __align__(16) float xs[];  // the row (times the norm weight), natural order; or this CTA's share of it
     __shared__ float red[2][RQ_THREADS / 32];
     __shared__ float stat[RQ_MAX_CLUSTER][2];    // (largest |x nw|, sum of x^2) of every CTA's share
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int C = (int)gridDim.x, r = (int)cluster_rank(), m = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tb = m / P.tq, t = m - tb * P.tq;
-    const int n4 = P.in / 4, i0 = (int)((long long)n4 * r / C), i1 = (int)((long long)n4 * (r + 1) / C);
     // this CTA's share of the digits: blocks of 8 inputs, whole K steps; an item is a block of one consumer
     const int b0 = (int)((long long)P.KS * r / C) * 16, nb = min(P.in / 8, (int)((long long)P.KS * (r + 1) / C) * 16) - b0, items = P.nmat * nb;
+    // and of the row: the same inputs if the row is in K order (a launch's rows are all permuted or none is)
+    const bool own = !P.perm[0];
+    const int n4 = P.in / 4, i0 = own ? 2 * b0 : (int)((long long)n4 * r / C), i1 = own ? 2 * (b0 + nb) : (int)((long long)n4 * (r + 1) / C);
+    float4* xs4 = reinterpret_cast<float4*>(xs) - (own ? i0 : 0);  // element i of the row
     auto perm_of = [&](int item) {
         const int j = item / nb;
         const uint16_t* p = j == 0 ? P.perm[0] : j == 1 ? P.perm[1] : P.perm[2];
@@ -98,8 +102,8 @@ __global__ void __launch_bounds__(RQ_THREADS, 4) row_quant_kernel(const __grid_c
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
         mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        reinterpret_cast<float4*>(xs)[i] = v;
-        for (int c = 0; c < C; c++)
+        xs4[i] = v;
+        for (int c = 0; c < C && !own; c++)
             if (c != r)
                 asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(peer_smem(xs + 4 * i, c)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
     }
@@ -133,12 +137,12 @@ __global__ void __launch_bounds__(RQ_THREADS, 4) row_quant_kernel(const __grid_c
             const int j = item / nb, blk = b0 + (item - j * nb);
             uint8_t* img = (j == 0 ? P.img[0] : j == 1 ? P.img[1] : P.img[2]) + (size_t)tb * P.KS * blk_bytes;
             float v[8];
-            if (P.perm[0]) {  // (a launch's rows are all permuted or none is)
+            if (!own) {
                 const uint4 ix = item == tid ? perm0 : perm_of(item);
                 v[0] = xs[ix.x & 0xFFFFu]; v[1] = xs[ix.x >> 16]; v[2] = xs[ix.y & 0xFFFFu]; v[3] = xs[ix.y >> 16];
                 v[4] = xs[ix.z & 0xFFFFu]; v[5] = xs[ix.z >> 16]; v[6] = xs[ix.w & 0xFFFFu]; v[7] = xs[ix.w >> 16];
             } else {
-                const float4 a = reinterpret_cast<const float4*>(xs)[2 * blk], b = reinterpret_cast<const float4*>(xs)[2 * blk + 1];
+                const float4 a = xs4[2 * blk], b = xs4[2 * blk + 1];
                 v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
             }
             uint32_t hi[4], lo[4];
@@ -260,11 +264,15 @@ static cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, int 
 cudaError_t row_quant_init(int max_smem) { return cudaFuncSetAttribute(row_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem); }
 
 // As many CTAs per token as it takes to cover the SMs about twice with the batch (a row is 16 to 112 KB: one CTA walks it in 2 to
-// 10 us, and nothing else of a small batch would hide that), never more than the K steps of the row.
+// 10 us, and nothing else of a small batch would hide that), never more than the K steps of the row.  Where a CTA holds its share
+// alone, as many as it takes for four CTAs on an SM (a whole row of 28672 fills one; 7B shapes, 16 layers, 30 tokens: 1690 -> 1632 us, 1536
+// tokens of the 70B shapes 29.6 -> 29.3 ms).
 cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st) {
+    const bool own = !p.perm[0];
+    auto share = [&](int C) { return own ? (size_t)((p.KS + C - 1) / C) * 512 : (size_t)p.in * 4; };
     int C = 1;
-    while (C < RQ_MAX_CLUSTER && 2 * C <= p.KS && (long long)p.M * C < sms) C *= 2;
-    return launch_pdl(row_quant_kernel, dim3(C, p.M), dim3(RQ_THREADS), (size_t)p.in * 4, C, st, p);
+    while (C < RQ_MAX_CLUSTER && 2 * C <= p.KS && ((long long)p.M * C < sms || (own && share(C) > 48 * 1024))) C *= 2;
+    return launch_pdl(row_quant_kernel, dim3(C, p.M), dim3(RQ_THREADS), share(C), C, st, p);
 }
 
 cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st) {
