@@ -111,11 +111,11 @@ def visible_gpus():
     return n
 
 
-def prefill_report(model, cfg, positions, ms, tp, hbm_peak, tensor_peak, peak_kind, cls_rows=None):
+def prefill_report(model, cfg, positions, ms, tp, hbm_peak, tensor_peak, peak_kind, cls_rows=None, per_pass=64, digits=3):
     """Batched prefill (the tcgen05 GEMM path) against both rooflines.  Algorithmic flops: 2 * K * N per position and
     QLinear (the classifier is not run in prefill); algorithmic bytes: the QLinear bytes of one pass over the weights per
-    chunk of up to 64 positions.  The integer GEMM executes 3 digit columns per position (balanced base-256 digits of the
-    activations), i.e. 3x the algorithmic multiply-adds on the int8 pipe."""
+    chunk of up to `per_pass` positions.  The GEMM executes `digits` columns per position (exact integer digits of the
+    activations), i.e. that many times the algorithmic multiply-adds."""
     if positions <= 0 or ms <= 0:
         return None
     d, h, L = cfg.dim, cfg.hidden_dim, cfg.n_layers
@@ -123,12 +123,12 @@ def prefill_report(model, cfg, positions, ms, tp, hbm_peak, tensor_peak, peak_ki
     flops_per_pos = 2.0 * L * (2 * d * d + 2 * d * kv + 3 * d * h)
     cls_rows = cfg.vocab_size if cls_rows is None else cls_rows  # classifier rows this process streams per token (a slice under tensor parallelism over peer memory)
     qbytes = float(model.decode_bytes) - 4.0 * cls_rows * d - 4.0 * (2 * L + 1) * d  # qweight + qzeros + scales of this process's rows
-    passes = positions if tp else (positions + 63) // 64  # tp here: tensor parallel over NCCL, which takes the prompt one position at a time
+    passes = positions if tp else (positions + per_pass - 1) // per_pass  # tp here: tensor parallel over NCCL, which takes the prompt one position at a time
     tflops = flops_per_pos * positions / (ms * 1e-3) / 1e12
     gbs = qbytes * passes / (ms * 1e-3) / 1e9
     return {"positions": positions, "ms": ms, "weight_passes": passes, "tflops": tflops, "tensor_peak_tflops": tensor_peak,
             "tensor_frac": tflops / tensor_peak, "weight_gbs": gbs, "hbm_frac": gbs / hbm_peak, "peak_kind": peak_kind,
-            "executed_mma_inflation": 1 if tp else 3}
+            "executed_mma_inflation": 1 if tp else digits}
 
 
 def make_prompt(np, n, vocab):
@@ -381,7 +381,8 @@ def main():
         "scaling": "strong" if tp else "weak", "vs_baseline": None, "dtype": "f32 activations / int4 weights", "data": "synthetic", "config": config,
         "prefill_tok_s": streams * pos0 * args.steps / max(prefill_ms, 1e-9) * 1e3,
         "prefill": prefill_report(model, cfg, pos0, prefill_ms / args.steps, tp and args.tp_nccl, peak, tensor_peak, peak_kind,
-                                  cls_rows=(cfg.vocab_size * (rank + 1) // world - cfg.vocab_size * rank // world) if tp and not args.tp_nccl else None),
+                                  cls_rows=(cfg.vocab_size * (rank + 1) // world - cfg.vocab_size * rank // world) if tp and not args.tp_nccl else None,
+                                  per_pass=64 if tp else 512, digits=2),
         "decode_ms_per_token": decode_ms / (n_loop * args.steps),
         "roofline": roofline,
         "token_roofline": {"bytes_per_token": model.decode_bytes, "achieved_gbs": model.decode_bytes * tok_s / 1e9,
