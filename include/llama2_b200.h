@@ -181,7 +181,9 @@ int l2_generate_ids(l2_model* m, const int32_t* prompt, int n_prompt, int steps,
  * qzeros [OUT/8][GROUPS] i32, scales [OUT][GROUPS] f32, g_index [IN] i32. */
 int l2_qlinear_create(int in, int out, int group_size, const int32_t* qweight, const int32_t* qzeros,
                       const float* scales, const int32_t* g_index, int device, l2_qlinear** h);
-/* x [B][IN] -> xout [B][OUT], host f32 buffers; copies to and from the device inside the call. */
+/* x [B][IN] -> xout [B][OUT], host f32 buffers; copies to and from the device inside the call.
+ * L2_ESTATUS: a bounded wait on the device gave up, in this call or in an earlier l2_qlinear_matvec_dev on the handle
+ * (which cannot report it itself); reported by one call, the next starts clean. */
 int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B);
 /* The same on device buffers, enqueued on cuda_stream (no copies, no synchronisation). */
 int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* xout_dev, int B, void* cuda_stream);
@@ -233,6 +235,9 @@ int l2_debug_trace(int enable, unsigned long long* host_out, int n_ctas);
  * phase end, phase left; SM clock at phase end; the rest are per-phase details.
  * No counterpart in the reference. */
 int l2_debug_token_trace(l2_state* s, int enable, unsigned long long* host_out, size_t count);
+
+/* Debug: writes the word that a batched kernel of this layer writes when a bounded wait gives up, as if one had. */
+int l2_debug_qlinear_status(l2_qlinear* h, int status);
 
 /* ---- sampling helpers (src/util.rs:39-46, 71-113) ----------------------------------- */
 uint32_t l2_random_u32(uint64_t* seed);

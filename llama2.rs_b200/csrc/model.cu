@@ -1486,6 +1486,9 @@ extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t*
     PackedQ p;
     repack_qlinear(in, out, group_size, qweight, qzeros, scales, nullptr, p);
     if (int rc = upload_qlinear(p, g_index, q->q, q->allocs, nullptr)) { free_allocs(q->allocs); return rc; }
+    const int zero = 0;
+    if (int rc = dev_upload(&q->status, &zero, 1, q->allocs)) { free_allocs(q->allocs); return rc; }
+    L2_CUDA(cudaStreamSynchronize(nullptr));  // cudaMemcpy may return before its last bytes are there, and the streams that read them do not wait for it
     L2_CUDA(cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking));
     StagePool::retain();
     *h = q.release();
@@ -1515,13 +1518,10 @@ static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
     const int rows[1] = {h->q.out};
     size_t total = 0;
     auto room = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
-    const size_t status = room(sizeof(int)), img = room(gemm_tc_image_bytes(h->q.in, h->q.gs, cap)), osc = room(sizeof(float) * cap),
+    const size_t img = room(gemm_tc_image_bytes(h->q.in, h->q.gs, cap)), osc = room(sizeof(float) * cap),
                  part = room(sizeof(float) * part_floats(rows, 1, h->q.in, h->q.gs, cap, h->sms));
     char* base = nullptr;
     if ((rc = dev_alloc(reinterpret_cast<void**>(&base), total, h->allocs))) return rc;
-    L2_CUDA(cudaMemset(base + status, 0, sizeof(int)));
-    L2_CUDA(cudaStreamSynchronize(nullptr));
-    h->status = reinterpret_cast<int*>(base + status);
     h->img = reinterpret_cast<uint8_t*>(base + img);
     h->osc = reinterpret_cast<float*>(base + osc);
     h->kpart = reinterpret_cast<float*>(base + part);
@@ -1569,9 +1569,21 @@ extern "C" int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int
     if (int rc = stage.take(h->device)) return rc;
     if (int rc = stage->upload(h->x_dev, x, sizeof(float) * h->q.in * B, h->stream)) return rc;
     if (int rc = l2_qlinear_matvec_dev(h, h->x_dev, h->y_dev, B, h->stream)) return rc;
-    int status = 0;
-    if (int rc = stage->download(xout, h->y_dev, sizeof(float) * h->q.out * B, h->stream, h->status, &status)) return rc;
-    if (status) return fail(L2_ESTATUS, "device status %d", status);
+    int status = 0;  // (only the batched kernels write the word)
+    if (int rc = stage->download(xout, h->y_dev, sizeof(float) * h->q.out * B, h->stream, h->cap_tc ? h->status : nullptr, &status)) return rc;
+    if (status) {  // reported once
+        L2_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+        return fail(L2_ESTATUS, "device status %d (a bounded wait of this call or of an earlier call on device buffers gave up)", status);
+    }
+    return L2_OK;
+}
+
+extern "C" int l2_debug_qlinear_status(l2_qlinear* h, int status) {
+    clear_error();
+    if (!h) return fail(L2_EINVAL, "l2_debug_qlinear_status: null handle");
+    L2_CUDA(cudaSetDevice(h->device));
+    L2_CUDA(cudaMemcpyAsync(h->status, &status, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    L2_CUDA(cudaStreamSynchronize(h->stream));
     return L2_OK;
 }
 

@@ -150,7 +150,7 @@ struct l2_qlinear {
     uint8_t* img = nullptr;   // batched path: digit image with the digit sums, and the factors
     float* osc = nullptr;
     float* kpart = nullptr;   // slices of the output beyond the first
-    int* status = nullptr;    // device word that a kernel whose wait gave up writes (batched path)
+    int* status = nullptr;    // device word that a kernel whose wait gave up writes (batched path); one for the handle's life, cleared when reported
     int cap_host = 0, cap_tc = 0;  // batch sizes the buffers hold
     cudaStream_t stream = nullptr;
     std::vector<void*> allocs;
