@@ -1490,6 +1490,7 @@ extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t*
     if (int rc = dev_upload(&q->status, &zero, 1, q->allocs)) { free_allocs(q->allocs); return rc; }
     L2_CUDA(cudaStreamSynchronize(nullptr));  // cudaMemcpy may return before its last bytes are there, and the streams that read them do not wait for it
     L2_CUDA(cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking));
+    L2_CUDA(cudaEventCreateWithFlags(&q->used, cudaEventDisableTiming));
     StagePool::retain();
     *h = q.release();
     return L2_OK;
@@ -1529,18 +1530,39 @@ static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
     return L2_OK;
 }
 
-extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* xout_dev, int B, void* cuda_stream) {
-    clear_error();
-    if (!h || !x_dev || !xout_dev || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec_dev: bad argument");
-    L2_CUDA(cudaSetDevice(h->device));
-    cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : h->stream;
+// A call's turn on the handle's buffers (x_dev, y_dev, xp_dev, img, osc, kpart), which all calls share: a call on another stream than the last
+// one waits on the device for that one's event.  Streams are told apart by their id, which a later stream does not get again.
+// Calls that a stream capture records take no part: only the caller knows when the graph runs.
+namespace {
+class QlinearTurn {
+public:
+    ~QlinearTurn() { if (h_) cudaEventRecord(h_->used, st_); }  // (whatever the call has enqueued, also where it failed)
+    int begin(l2_qlinear* h, cudaStream_t st) {
+        cudaStreamCaptureStatus capture;
+        L2_CUDA(cudaStreamIsCapturing(st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) return L2_OK;
+        unsigned long long id;
+        L2_CUDA(cudaStreamGetId(st, &id));
+        if (h->used_by && *h->used_by != id) L2_CUDA(cudaStreamWaitEvent(st, h->used, 0));
+        h->used_by = id;
+        h_ = h;
+        st_ = st;
+        return L2_OK;
+    }
+private:
+    l2_qlinear* h_ = nullptr;
+    cudaStream_t st_ = nullptr;
+};
+}  // namespace
+
+static int qlinear_enqueue(l2_qlinear* h, const float* x_dev, float* xout_dev, int B, cudaStream_t st) {
     if (int rc = qlinear_reserve(h, B, false)) return rc;
     if (B >= 2) {  // batched: tensor-core GEMM, MAX_BATCH tokens at a time
         // The kernels around the GEMM read and write rows as 16-byte words; arrays that start elsewhere go through aligned copies.
         if ((reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(xout_dev)) % 16 != 0) {
             if (int rc = qlinear_reserve(h, B, true)) return rc;
             L2_CUDA(cudaMemcpyAsync(h->x_dev, x_dev, sizeof(float) * h->q.in * B, cudaMemcpyDeviceToDevice, st));
-            if (int rc = l2_qlinear_matvec_dev(h, h->x_dev, h->y_dev, B, st)) return rc;
+            if (int rc = qlinear_enqueue(h, h->x_dev, h->y_dev, B, st)) return rc;
             L2_CUDA(cudaMemcpyAsync(xout_dev, h->y_dev, sizeof(float) * h->q.out * B, cudaMemcpyDeviceToDevice, st));
             return L2_OK;
         }
@@ -1560,15 +1582,27 @@ extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* x
     return L2_OK;
 }
 
+extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* xout_dev, int B, void* cuda_stream) {
+    clear_error();
+    if (!h || !x_dev || !xout_dev || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec_dev: bad argument");
+    L2_CUDA(cudaSetDevice(h->device));
+    cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : h->stream;
+    QlinearTurn turn;
+    if (int rc = turn.begin(h, st)) return rc;
+    return qlinear_enqueue(h, x_dev, xout_dev, B, st);
+}
+
 extern "C" int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B) {
     clear_error();
     if (!h || !x || !xout || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec: bad argument");
     L2_CUDA(cudaSetDevice(h->device));
+    QlinearTurn turn;
+    if (int rc = turn.begin(h, h->stream)) return rc;
     if (int rc = qlinear_reserve(h, B, true)) return rc;
     StagePool::Lease stage;
     if (int rc = stage.take(h->device)) return rc;
     if (int rc = stage->upload(h->x_dev, x, sizeof(float) * h->q.in * B, h->stream)) return rc;
-    if (int rc = l2_qlinear_matvec_dev(h, h->x_dev, h->y_dev, B, h->stream)) return rc;
+    if (int rc = qlinear_enqueue(h, h->x_dev, h->y_dev, B, h->stream)) return rc;
     int status = 0;  // (only the batched kernels write the word)
     if (int rc = stage->download(xout, h->y_dev, sizeof(float) * h->q.out * B, h->stream, h->cap_tc ? h->status : nullptr, &status)) return rc;
     if (status) {  // reported once
@@ -1591,6 +1625,7 @@ extern "C" void l2_qlinear_free(l2_qlinear* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     free_allocs(h->allocs);
+    if (h->used) cudaEventDestroy(h->used);
     if (h->stream) cudaStreamDestroy(h->stream);
     StagePool::release();
     delete h;

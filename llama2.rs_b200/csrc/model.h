@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <optional>
 #include <vector>
 
 #include "host_common.h"
@@ -153,6 +154,8 @@ struct l2_qlinear {
     int* status = nullptr;    // device word that a kernel whose wait gave up writes (batched path); one for the handle's life, cleared when reported
     int cap_host = 0, cap_tc = 0;  // batch sizes the buffers hold
     cudaStream_t stream = nullptr;
+    std::optional<unsigned long long> used_by;  // id of the stream whose call has used the buffers last
+    cudaEvent_t used = nullptr;                 // ... and the end of that call
     std::vector<void*> allocs;
 };
 

@@ -1,4 +1,4 @@
-"""What a single layer's handle keeps between calls: the status word of its bounded waits."""
+"""What a single layer's handle keeps between calls: the status word of its bounded waits, buffers that calls on several streams share."""
 import numpy as np
 import pytest
 
@@ -25,3 +25,55 @@ def test_recorded_failure_is_reported_once(l2, B):
         q.matvec(x)
     assert np.array_equal(q.matvec(x), want)
     assert np.array_equal(q.matvec(x[0]), make(l2, 256, 264, 64)[1].matvec(x[0]))
+
+
+# (offset of the device arrays from the 16-byte boundary: batched calls on unaligned arrays go through the arrays of host calls)
+@pytest.mark.parametrize("B,off", [(1, 0), (2, 0), (37, 0), (37, 1), (130, 3)])
+@pytest.mark.parametrize("second", ["host", "stream"])
+def test_calls_on_several_streams_take_turns(l2, B, off, second):
+    import torch
+    K, N = 1024, 776
+    rng, q = make(l2, K, N, 64)
+    xa, xb = rng.standard_normal((2, B, K)).astype(np.float32)
+    want_a, want_b = q.matvec(xa), q.matvec(xb)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    da, db = torch.zeros(B * K + 4, device="cuda"), torch.zeros(B * K + 4, device="cuda")
+    ya, yb = torch.zeros(B * N + 4, device="cuda"), torch.zeros(B * N + 4, device="cuda")
+    da[off:off + B * K] = torch.from_numpy(xa).cuda().flatten()
+    db[off:off + B * K] = torch.from_numpy(xb).cuda().flatten()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        with torch.cuda.stream(s1):
+            torch.cuda._sleep(20_000_000)  # about 10 ms: the first call is still to come when the second is made
+        q.matvec_dev(da.data_ptr() + 4 * off, ya.data_ptr() + 4 * off, B, s1.cuda_stream)
+        if second == "host":
+            got_b = q.matvec(xb)
+        else:
+            q.matvec_dev(db.data_ptr() + 4 * off, yb.data_ptr() + 4 * off, B, s2.cuda_stream)
+        torch.cuda.synchronize()
+        if second == "stream":
+            got_b = yb[off:off + B * N].view(B, N).cpu().numpy()
+        assert np.array_equal(got_b, want_b)
+        assert np.array_equal(ya[off:off + B * N].view(B, N).cpu().numpy(), want_a)
+        ya.zero_(), yb.zero_()
+        torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("B", [1, 37])
+def test_captured_call(l2, B):
+    import torch
+    K, N = 1024, 776
+    rng, q = make(l2, K, N, 64)
+    x = rng.standard_normal((2, B, K)).astype(np.float32)
+    want = [q.matvec(v) for v in x]  # (the first call allocates)
+    xd, yd = torch.zeros(B, K, device="cuda"), torch.zeros(B, N, device="cuda")
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        q.matvec_dev(xd.data_ptr(), yd.data_ptr(), B, s.cuda_stream)
+    for v, w in zip(x, want):
+        xd.copy_(torch.from_numpy(v))
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(yd.cpu().numpy(), w)
+        assert np.array_equal(q.matvec(v), w)
