@@ -1488,8 +1488,9 @@ extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t*
     if (int rc = upload_qlinear(p, g_index, q->q, q->allocs, nullptr)) { free_allocs(q->allocs); return rc; }
     const int zero = 0;
     if (int rc = dev_upload(&q->status, &zero, 1, q->allocs)) { free_allocs(q->allocs); return rc; }
-    L2_CUDA(cudaStreamSynchronize(nullptr));  // cudaMemcpy may return before its last bytes are there, and the streams that read them do not wait for it
+    L2_CUDA(cudaStreamSynchronize(nullptr));  // cudaMemcpy may return before its last bytes are there, and the callers' streams do not wait for it
     L2_CUDA(cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking));
+    L2_CUDA(cudaStreamCreate(&q->stream_default));  // ordered with the default stream: that is what a caller who passes no stream works on
     L2_CUDA(cudaEventCreateWithFlags(&q->used, cudaEventDisableTiming));
     StagePool::retain();
     *h = q.release();
@@ -1586,7 +1587,7 @@ extern "C" int l2_qlinear_matvec_dev(l2_qlinear* h, const float* x_dev, float* x
     clear_error();
     if (!h || !x_dev || !xout_dev || B < 1) return fail(L2_EINVAL, "l2_qlinear_matvec_dev: bad argument");
     L2_CUDA(cudaSetDevice(h->device));
-    cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : h->stream;
+    cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : h->stream_default;
     QlinearTurn turn;
     if (int rc = turn.begin(h, st)) return rc;
     return qlinear_enqueue(h, x_dev, xout_dev, B, st);
@@ -1627,6 +1628,7 @@ extern "C" void l2_qlinear_free(l2_qlinear* h) {
     free_allocs(h->allocs);
     if (h->used) cudaEventDestroy(h->used);
     if (h->stream) cudaStreamDestroy(h->stream);
+    if (h->stream_default) cudaStreamDestroy(h->stream_default);
     StagePool::release();
     delete h;
 }

@@ -153,7 +153,8 @@ struct l2_qlinear {
     float* kpart = nullptr;   // slices of the output beyond the first
     int* status = nullptr;    // device word that a kernel whose wait gave up writes (batched path); one for the handle's life, cleared when reported
     int cap_host = 0, cap_tc = 0;  // batch sizes the buffers hold
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr;          // host arrays
+    cudaStream_t stream_default = nullptr;  // device arrays where the caller gives no stream
     std::optional<unsigned long long> used_by;  // id of the stream whose call has used the buffers last
     cudaEvent_t used = nullptr;                 // ... and the end of that call
     std::vector<void*> allocs;

@@ -1,4 +1,5 @@
-"""What a single layer's handle keeps between calls: the status word of its bounded waits, buffers that calls on several streams share."""
+"""What a single layer's handle keeps between calls: the status word of its bounded waits, buffers that calls on several streams share,
+and the order with the default stream where no stream is given."""
 import numpy as np
 import pytest
 
@@ -77,3 +78,23 @@ def test_captured_call(l2, B):
         torch.cuda.synchronize()
         assert np.array_equal(yd.cpu().numpy(), w)
         assert np.array_equal(q.matvec(v), w)
+
+
+@pytest.mark.parametrize("B,off", [(1, 0), (37, 0), (37, 1)])
+def test_no_stream_is_ordered_with_the_default_stream(l2, B, off):
+    import torch
+    K, N = 1024, 776
+    rng, q = make(l2, K, N, 64)
+    x = rng.standard_normal((B, K)).astype(np.float32)
+    want = q.matvec(x)
+    src = torch.from_numpy(x).cuda().flatten()
+    xd, yd = torch.zeros(B * K + 4, device="cuda"), torch.zeros(B * N + 4, device="cuda")
+    torch.cuda.synchronize()
+    assert torch.cuda.current_stream().cuda_stream == 0
+    for _ in range(3):
+        torch.cuda._sleep(20_000_000)          # the input is not there yet when the call is made ...
+        xd[off:off + B * K] = src
+        q.matvec_dev(xd.data_ptr() + 4 * off, yd.data_ptr() + 4 * off, B)
+        got = yd[off:off + B * N].clone()      # ... and the output is taken and both are overwritten without waiting on the host
+        xd.zero_(), yd.zero_()
+        assert np.array_equal(got.view(B, N).cpu().numpy(), want)
