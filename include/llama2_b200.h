@@ -185,7 +185,9 @@ int l2_qlinear_create(int in, int out, int group_size, const int32_t* qweight, c
  * L2_ESTATUS: a bounded wait on the device gave up, in this call or in an earlier l2_qlinear_matvec_dev on the handle
  * (which cannot report it itself); reported by one call, the next starts clean. */
 int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B);
-/* The same on device buffers, enqueued on cuda_stream (no copies, no synchronisation).  NULL: on a stream of the handle that
+/* The same on device buffers, enqueued on cuda_stream without waiting for it.  The first call with B = 1, and a batched call (B >= 2)
+ * that is larger than any before it, allocate the handle's buffers.  Batched calls read and write rows as 16-byte words: arrays that
+ * do not start on a 16-byte boundary are copied on the device, through buffers of the size of both arrays.  NULL: on a stream of the handle that
  * is ordered with the device's default stream, so that work in front of the call and behind it on that stream needs no
  * synchronisation either.  The handle's buffers serve one call
  * at a time: a call (host buffers or device buffers) on another stream than the call before it waits for that one on the

@@ -1497,6 +1497,14 @@ extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t*
     return L2_OK;
 }
 
+// The B = 1 launch record goes up on the stream of the host calls, which is idle here: neither the caller's stream nor the default stream
+// is waited for.
+static int upload_plan(l2_qlinear* h) {
+    L2_CUDA(cudaMemcpyAsync(h->d_plan, &h->plan.p, sizeof(SkParams), cudaMemcpyHostToDevice, h->stream));
+    L2_CUDA(cudaStreamSynchronize(h->stream));
+    return L2_OK;
+}
+
 static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
     int rc;
     if (host && B > h->cap_host) {  // device copies of the caller's host arrays
@@ -1505,11 +1513,12 @@ static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
         h->cap_host = B;
     }
     if (B == 1) {
-        if (h->d_plan) return L2_OK;
+        if (h->planned) return L2_OK;
         if ((rc = dev_alloc(reinterpret_cast<void**>(&h->xp_dev), sizeof(float) * h->q.in, h->allocs))) return rc;
         if ((rc = plan_gemv_single(h->q, h->xp_dev, h->sms, h->plan))) return rc;
-        if ((rc = dev_upload(&h->d_plan, &h->plan.p, 1, h->allocs))) return rc;
-        L2_CUDA(cudaStreamSynchronize(nullptr));  // the caller's stream need not wait for the copy otherwise
+        if ((rc = dev_alloc(reinterpret_cast<void**>(&h->d_plan), sizeof(SkParams), h->allocs))) return rc;
+        if ((rc = upload_plan(h))) return rc;
+        h->planned = true;
         return L2_OK;
     }
     // Buffers of the batched (tcgen05) path, one allocation: for the tokens of the call, in powers of two so that growing calls do not pile up
@@ -1575,8 +1584,7 @@ static int qlinear_enqueue(l2_qlinear* h, const float* x_dev, float* xout_dev, i
     }
     if (h->plan.p.trace != g_sk_trace) {  // clock stamps were switched on after the record was made
         h->plan.p.trace = g_sk_trace;
-        L2_CUDA(cudaMemcpy(h->d_plan, &h->plan.p, sizeof(SkParams), cudaMemcpyHostToDevice));
-        L2_CUDA(cudaStreamSynchronize(nullptr));
+        if (int rc = upload_plan(h)) return rc;
     }
     L2_CUDA(launch_permute(x_dev, h->q.perm, h->xp_dev, h->q.in, st));
     L2_CUDA(launch_sk(h->d_plan, h->q.gs, 1, h->plan.grid, h->plan.smem, st, true, xout_dev));

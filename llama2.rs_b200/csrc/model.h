@@ -148,6 +148,7 @@ struct l2_qlinear {
     float *x_dev = nullptr, *xp_dev = nullptr, *y_dev = nullptr;
     l2::SkLaunch plan;                   // B = 1: launch plan and its record on the device
     l2::SkParams* d_plan = nullptr;
+    bool planned = false;                // the record is there
     uint8_t* img = nullptr;   // batched path: digit image with the digit sums, and the factors
     float* osc = nullptr;
     float* kpart = nullptr;   // slices of the output beyond the first

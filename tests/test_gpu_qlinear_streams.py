@@ -1,5 +1,7 @@
 """What a single layer's handle keeps between calls: the status word of its bounded waits, buffers that calls on several streams share,
-and the order with the default stream where no stream is given."""
+the order with the default stream where no stream is given, and first calls that wait for nobody."""
+import time
+
 import numpy as np
 import pytest
 
@@ -98,3 +100,27 @@ def test_no_stream_is_ordered_with_the_default_stream(l2, B, off):
         got = yd[off:off + B * N].clone()      # ... and the output is taken and both are overwritten without waiting on the host
         xd.zero_(), yd.zero_()
         assert np.array_equal(got.view(B, N).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("B", [1, 2, 130])
+def test_first_call_does_not_wait_for_other_work(l2, B):
+    import torch
+    K, N = 1024, 776
+    rng, q = make(l2, K, N, 64)
+    x = rng.standard_normal((B, K)).astype(np.float32)
+    want = q.matvec(x)  # (the kernels are loaded)
+    _, fresh = make(l2, K, N, 64)
+    xd, yd = torch.from_numpy(x).cuda(), torch.zeros(B, N, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    for st in (torch.cuda.default_stream(), s):
+        with torch.cuda.stream(st):
+            torch.cuda._sleep(600_000_000)  # about 0.3 s, on the default stream and on the call's
+    busy.record(torch.cuda.default_stream())
+    t = time.perf_counter()
+    fresh.matvec_dev(xd.data_ptr(), yd.data_ptr(), B, s.cuda_stream)
+    took = time.perf_counter() - t
+    assert not busy.query() and took < 0.2
+    torch.cuda.synchronize()
+    assert np.array_equal(yd.cpu().numpy(), want)
