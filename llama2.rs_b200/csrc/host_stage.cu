@@ -25,6 +25,7 @@ int HostStage::init(int device) {
 }
 
 int HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    busy_ = true; busy_on_ = st;
     if (direct_copy(src)) {  // the caller's array itself is the staging memory
         L2_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return L2_OK;
@@ -40,12 +41,19 @@ int HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
     return L2_OK;
 }
 
+void HostStage::drain() {
+    if (busy_) cudaStreamSynchronize(busy_on_);
+    busy_ = false;
+}
+
 int HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t st, const int* word_dev, int* word) {
+    busy_ = true; busy_on_ = st;
     volatile int* pin_word = reinterpret_cast<int*>(pin_ + CHUNK * SLOTS);  // (in front of the data on the stream: there when the data is)
     if (word_dev) L2_CUDA(cudaMemcpyAsync(pin_ + CHUNK * SLOTS, word_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (direct_copy(dst)) {
         L2_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         L2_CUDA(cudaStreamSynchronize(st));
+        busy_ = false;
         if (word_dev) *word = *pin_word;
         return L2_OK;
     }
@@ -65,6 +73,7 @@ int HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t s
         if (i + SLOTS < chunks)
             if (int rc = request(i + SLOTS)) return rc;
     }
+    busy_ = false;  // the last copy has been waited for, and with it everything in front of it on the stream
     if (word_dev) *word = *pin_word;
     return L2_OK;
 }
@@ -99,6 +108,7 @@ int StagePool::Lease::take(int device) {
 }
 StagePool::Lease::~Lease() {
     if (!s_) return;
+    s_->drain();  // a call that ended in an error: the next owner of the ring, and the caller with its array, find nothing in flight
     std::lock_guard<std::mutex> g(mu_);
     if ((int)free_.size() < KEPT && users_ > 0) free_.push_back(std::move(s_));
 }

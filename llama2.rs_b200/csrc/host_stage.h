@@ -23,11 +23,15 @@ public:
     ~HostStage();
     int init(int device);
     int device() const { return device_; }
-    int upload(void* dst, const void* src, size_t bytes, cudaStream_t st);    // src stays as it is until the stream has been waited for
+    // The copies of a call are on one stream.  src stays as it is until a download has returned, or drain.
+    int upload(void* dst, const void* src, size_t bytes, cudaStream_t st);
     // returns when dst holds the data; word_dev (may be null): one more int that comes along
     int download(void* dst, const void* src, size_t bytes, cudaStream_t st, const int* word_dev = nullptr, int* word = nullptr);
+    void drain();  // waits for an upload without a download behind it, or a copy that failed in the middle
 private:
     int device_ = -1;
+    bool busy_ = false;               // copies may be in flight ...
+    cudaStream_t busy_on_ = nullptr;  // ... on this stream
     char* pin_ = nullptr;
     cudaEvent_t done_[SLOTS] = {};
 };
