@@ -286,10 +286,18 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
         float* dst = (sg.slice == 0 ? X.out : X.part + (size_t)(sg.slice - 1) * P.M * X.rows) + (size_t)m0 * ld + orow;
         if (orow < X.rows) {
 #pragma unroll
-            for (int i = 0; i < 8 * NT; i++) {
-                const float2 y = unpack2(acc[i]);
-                if (m0 + 2 * i < P.M) dst[(size_t)(2 * i) * ld] = y.x * __ldg(P.osc + m0 + 2 * i);
-                if (m0 + 2 * i + 1 < P.M) dst[(size_t)(2 * i + 1) * ld] = y.y * __ldg(P.osc + m0 + 2 * i + 1);
+            for (int st = 0; st < NT; st++) {
+                // The factors are the output of the kernel in front, which may run beside this one: no read-only loads.  16 at a time in front of
+                // their stores (a plain load does not move past a store).
+                float f[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) f[i] = m0 + 16 * st + i < P.M ? P.osc[m0 + 16 * st + i] : 0.f;
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const float2 y = unpack2(acc[8 * st + i / 2]);
+                    if (m0 + 16 * st + i < P.M) dst[(size_t)(16 * st + i) * ld] = y.x * f[i];
+                    if (m0 + 16 * st + i + 1 < P.M) dst[(size_t)(16 * st + i + 1) * ld] = y.y * f[i + 1];
+                }
             }
         }
     }

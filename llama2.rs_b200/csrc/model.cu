@@ -104,7 +104,8 @@ int upload_qlinear(const PackedQ& p, const int32_t* g_index, DevQ& d, std::vecto
     return L2_OK;
 }
 
-__global__ void permute_kernel(const float* __restrict__ x, const int* __restrict__ perm, float* __restrict__ xp, int n) {
+// (x may still be written when this kernel starts: it is not declared read-only, and is read behind the wait)
+__global__ void permute_kernel(const float* x, const int* __restrict__ perm, float* xp, int n) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int src = j < n ? perm[j] : 0;

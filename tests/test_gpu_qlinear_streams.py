@@ -1,5 +1,5 @@
 """What a single layer's handle keeps between calls: the status word of its bounded waits, buffers that calls on several streams share,
-the order with the default stream where no stream is given, and first calls that wait for nobody."""
+the order with the default stream where no stream is given, first calls that wait for nobody, and inputs that the kernel in front has just written."""
 import time
 
 import numpy as np
@@ -124,3 +124,24 @@ def test_first_call_does_not_wait_for_other_work(l2, B):
     assert not busy.query() and took < 0.2
     torch.cuda.synchronize()
     assert np.array_equal(yd.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("B", [1, 16, 64, 130])
+def test_inputs_written_by_the_kernel_in_front(l2, B):
+    # call after call on the same arrays, rows and their factors changing each time, nothing waited for in between
+    import torch
+    K, N = 1024, 776
+    rng, q = make(l2, K, N, 64)
+    x = rng.standard_normal((12, B, K)).astype(np.float32) * np.exp(rng.uniform(-6, 6, (12, B, 1))).astype(np.float32)
+    want = np.stack([q.matvec(v) for v in x])
+    s = torch.cuda.Stream()
+    src, xd, yd = torch.from_numpy(x).cuda(), torch.zeros(B, K, device="cuda"), torch.zeros(B, N, device="cuda")
+    got = torch.zeros(12, B, N, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for i in range(12):
+            torch.add(src[i], 0.0, out=xd)
+            q.matvec_dev(xd.data_ptr(), yd.data_ptr(), B, s.cuda_stream)
+            torch.add(yd, 0.0, out=got[i])
+    torch.cuda.synchronize()
+    assert np.array_equal(got.cpu().numpy(), want)
