@@ -1166,20 +1166,22 @@ static int prefill_async(l2_model* m, l2_state* s, const int32_t* prompt, int n_
     // Positions the reference's ladder 64/32/16/8/4/2 covers (src/inference.rs:24, 78-127): the B=1 loop
     // must start where it starts there.  How those positions are cut into batches does not change the
     // cache ("should lead to identical results", src/inference.rs:12-15), so they go in even batches of up to
-    // MAX_BATCH rows (every batch is a pass over the weights).
+    // MAX_BATCH rows (every batch is a pass over the weights), fewer where the device has no room for the buffers.
     static const int ladder[6] = {64, 32, 16, 8, 4, 2};
     int target = 0;
     if (chunk > 0) { while (target + chunk < n_prompt) target += chunk; }
     else for (int a : ladder) while (target + a < n_prompt) target += a;
-    int pos = 0;
+    int pos = 0, limit = TC_MAX_TOKENS;  // (tensor parallel: what the ranks' pools hold)
+    if (m->tp_world == 1 && target > 1)
+        if (int rc = reserve_batch(m, target, &limit)) return rc;
     int32_t tokens[MAX_BATCH], positions[MAX_BATCH];
     while (pos < target) {
         // tensor parallel models run the batched path when the ranks are connected through peer memory (the exchanges are
         // stores into the peers' pools) and this state is the one that works in the pool; otherwise one position at a time
         if (m->tp_direct && !m->tp_pool_owner) m->tp_pool_owner = s;
         const bool batched = m->tp_world == 1 || (m->tp_direct && token_path(s));
-        const int left = target - pos, passes = (left + batch_limit(m) - 1) / batch_limit(m);
-        const int A = batched ? (left + passes - 1) / passes : 1;
+        const int left = target - pos;
+        const int passes = (left + limit - 1) / limit, A = batched ? (left + passes - 1) / passes : 1;
         for (int i = 0; i < A; i++) {
             tokens[i] = pos == 0 ? L2_START : prompt[pos - 1];  // src/inference.rs:29-35
             positions[i] = pos++;

@@ -179,7 +179,7 @@ void tp_rows(int total_rows, int rank, int world, int* row0, int* nrows);
 int gemm_batched(const DevQ& q, const float* x, int M, uint8_t* img, float* osc, float* out, float* part, int* status, int sms, cudaStream_t st);
 size_t part_floats(const int* rows, int n, int in, int gs, int cap, int sms);
 void free_batch(l2_model* m);
-inline int batch_limit(const l2_model* m) { return m->tp_world > 1 ? TC_MAX_TOKENS : MAX_BATCH; }  // tokens of one batched forward (the ranks' pools hold one token block)
+int reserve_batch(l2_model* m, int M, int* limit);
 int dev_alloc_bytes(void** p, size_t bytes, std::vector<void*>& allocs);
 void sk_set_matrix(SkJob& j, int seg, const DevQ& q, const float* x, const float* nw);
 }  // namespace l2

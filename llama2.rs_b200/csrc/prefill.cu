@@ -71,16 +71,9 @@ void free_batch(l2_model* m) {
     m->batch = nullptr;
 }
 
-// The batched forward's buffers belong to the model: its calls run one after another on one stream and every call that uses
-// them ends synchronised, so all run states share them.  They grow once, from the size of a short batch to that of a long one.
-static int ensure_batch(l2_model* m, int M) {
+// The buffers of batches of up to `cap` tokens; cudaErrorMemoryAllocation (and no buffers) where the device does not have the room.
+static cudaError_t alloc_batch(l2_model* m, int cap) {
     const bool tp = m->tp_world > 1;
-    const int cap = M <= TC_MAX_TOKENS || tp ? TC_MAX_TOKENS : MAX_BATCH;
-    if (m->batch && m->batch->cap >= cap) return L2_OK;
-    if (m->batch) {
-        L2_CUDA(cudaStreamSynchronize(m->stream));
-        free_batch(m);
-    }
     const l2_config& c = m->shape.c;
     const int T = m->tp_world, D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim, Dl = D / T, KVl = KV / T, Hl = H / T, gs = c.group_size;
     BatchBuffers* b = m->batch = new BatchBuffers;
@@ -96,7 +89,12 @@ static int ensure_batch(l2_model* m, int M) {
     const size_t img0 = room(gemm_tc_image_bytes(std::max(D, H), gs, cap)), img1 = room(gemm_tc_image_bytes(D, gs, cap)), img2 = room(gemm_tc_image_bytes(D, gs, cap));
     const size_t tok = room(2 * B * sizeof(int)), done = room(256);
     char* base = nullptr;
-    if (int rc = dev_alloc_bytes(reinterpret_cast<void**>(&base), total, b->allocs)) { free_batch(m); return rc; }
+    if (cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base), total)) {
+        cudaGetLastError();  // (an answer here, not an error of a later launch)
+        free_batch(m);
+        return e;
+    }
+    b->allocs.push_back(base);
     auto at = [&](size_t off) { return reinterpret_cast<float*>(base + off); };
     b->x = at(x); b->att = at(att); b->q = at(q); b->y = at(y); b->part = at(part); b->osc = at(osc);
     b->img[0] = reinterpret_cast<uint8_t*>(base + img0); b->img[1] = reinterpret_cast<uint8_t*>(base + img1); b->img[2] = reinterpret_cast<uint8_t*>(base + img2);
@@ -106,9 +104,30 @@ static int ensure_batch(l2_model* m, int M) {
         b->att = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[1]);
         b->hb = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[2]);
         b->tp_done = reinterpret_cast<unsigned*>(base + done);
-        if (cudaMemset(b->tp_done, 0, 256) != cudaSuccess) { free_batch(m); return fail(L2_ECUDA, "cudaMemset failed"); }
+        if (cudaError_t e = cudaMemset(b->tp_done, 0, 256)) { free_batch(m); return e; }
     }
-    if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), sizeof(int) * 2 * B * BATCH_RING) != cudaSuccess) { free_batch(m); return fail(L2_ECUDA, "cudaMallocHost failed"); }
+    if (cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), sizeof(int) * 2 * B * BATCH_RING)) { free_batch(m); return e; }
+    return cudaSuccess;
+}
+
+// The batched forward's buffers belong to the model: its calls run one after another on one stream and every call that uses
+// them ends synchronised, so all run states share them.  They grow once, from the size of a short batch to that of a long one, or to
+// the largest half, quarter ... of it that the device has room for.  *limit: tokens of one batch.
+int reserve_batch(l2_model* m, int M, int* limit) {
+    const int most = m->tp_world > 1 ? TC_MAX_TOKENS : MAX_BATCH;  // (the ranks' pools hold one token block)
+    if (!m->batch || m->batch->cap < std::min(M, most)) {
+        if (m->batch) {
+            L2_CUDA(cudaStreamSynchronize(m->stream));
+            free_batch(m);
+        }
+        for (int cap = M <= TC_MAX_TOKENS ? TC_MAX_TOKENS : most;; cap /= 2) {
+            const cudaError_t e = alloc_batch(m, cap);
+            if (e == cudaSuccess) break;
+            if (e != cudaErrorMemoryAllocation || cap <= TC_MAX_TOKENS)
+                return fail(L2_ECUDA, "buffers of the batched forward (%d tokens): %s", cap, cudaGetErrorString(e));
+        }
+    }
+    *limit = m->batch->cap;
     return L2_OK;
 }
 
@@ -229,8 +248,9 @@ int forward_batch(l2_state* s, int M, const int32_t* tokens, const int32_t* pos)
         if (!m->tp_pool_owner) m->tp_pool_owner = s;
         if (m->tp_pool_owner != s) return fail(L2_EINVAL, "batched forward under tensor parallelism: another run state of this model works in the pool");
     }
-    if (M < 1 || M > batch_limit(m)) return fail(L2_EINVAL, "forward_batch: %d tokens", M);
-    if (int rc = ensure_batch(m, M)) return rc;
+    int limit;
+    if (int rc = reserve_batch(m, M, &limit)) return rc;
+    if (M < 1 || M > limit) return fail(L2_EINVAL, "forward_batch: %d tokens", M);
     BatchBuffers* b = m->batch;
     cudaStream_t st = m->stream;
     // token ids and positions: own pinned slot per call until the copy has run
