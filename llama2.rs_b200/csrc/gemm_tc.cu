@@ -5,7 +5,7 @@
 //
 // X[m][k] is the activation of token m as a 24-bit signed integer, X = 4096 hi + lo with |hi|, |lo| <= 2048 (see row_quant_kernel in
 // prefill_kernels.cu).  Both digits and q - z are small integers, exact in f16, and so are their products and the sums over a
-// quantisation group (below 2^22) in the f32 accumulators: kind::f16 MMAs do exact integer arithmetic here.  f[m] carries the block
+// quantisation group (at most 2^22) in the f32 accumulators: kind::f16 MMAs do exact integer arithmetic here.  f[m] carries the block
 // exponent and the rmsnorm factor.
 // (The alternative, three 8-bit digits on kind::i8, needs 3/4 of the MMA time but a third more accumulator columns, and their way
 // from s32 columns to f32 sums (one multiply-add, two conversions, the zero-point correction) bounded the kernel at 1110 / 1770 clocks

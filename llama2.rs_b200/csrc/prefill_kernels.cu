@@ -50,7 +50,8 @@ __global__ void embed_batch_kernel(const float* __restrict__ table, const int* _
 // share is what it cuts, it keeps that alone and nothing but the statistics crosses.
 //
 // Digits: X = round(x * nw * 2^(22 - E)) with E the exponent of the row's largest |x * nw|, so |X| <= 2^23 (the 24 bits of an f32
-// mantissa for the largest element), X = 4096 hi + lo with hi in -2048..2048 and lo in -2048..2047, both exact in f16.  They go into the
+// mantissa for the largest element), X = 4096 hi + lo with hi and lo in -2048..2048 (halves round to even), both exact in f16.  A NaN or an
+// infinity becomes a digit that is not finite, which makes every output of its token NaN.  The digits go into the
 // K-major, 128-byte-swizzled blocks the GEMM copies into shared memory: per K step two halves of 64 inputs, row digit * tq + token,
 // inside a block of 8 inputs the order (0,4,1,5,2,6,3,7) in which a weight word separates into f16 pairs.
 constexpr int RQ_THREADS = 256;
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 4) row_quant_kernel(const __grid_c
     const float rs = P.nw ? 1.0f / sqrtf(total / (float)P.in + P.eps) : 1.0f;  // src/models.rs:58-60
     int e = 0;
     if (mx > 0.f && mx < INFINITY) e = 22 - (int)((__float_as_uint(mx) >> 23) & 255u) + 127;  // |x| * scale < 2^23
-    e = max(-100, min(100, e));
+    e = min(100, e);  // (at least 22 - 127: every finite row is scaled down far enough)
     const float scale = __uint_as_float((uint32_t)(127 + e) << 23);
     if (tid == 0 && r == 0) P.osc[m] = rs / scale;
 
