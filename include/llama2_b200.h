@@ -243,6 +243,12 @@ int l2_debug_trace(int enable, unsigned long long* host_out, int n_ctas);
  * No counterpart in the reference. */
 int l2_debug_token_trace(l2_state* s, int enable, unsigned long long* host_out, size_t count);
 
+/* Debug: the attention kernels of the batched forward on device buffers: q and out [M][n_heads * 128], caches [SEQ][n_kv_heads][128],
+ * pos [M].  Query row m attends to positions 0 .. pos[m].  kind: 0 one CTA per head and token, 1 and 2 (1, 2, 4 or 8 query heads per
+ * kv head) cache tiles shared by 4 or 8, or by 16 queries per warp; the forward chooses by context and size. */
+int l2_debug_attention_batch(int n_heads, int n_kv_heads, int M, int kind, const float* q, const float* key_cache,
+                             const float* value_cache, const int32_t* pos, float* out, void* cuda_stream);
+
 /* Debug: writes the word that a batched kernel of this layer writes when a bounded wait gives up, as if one had. */
 int l2_debug_qlinear_status(l2_qlinear* h, int status);
 

@@ -280,6 +280,8 @@ void launch_embed_batch(const float* table, const int* tokens, float* x, int dim
 cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st);
 cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st);
 cudaError_t launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, int sms, cudaStream_t st);
+enum : int { ATTN_HEAD = 0, ATTN_TILED = 1, ATTN_WIDE = 2 };  // one CTA per (head, token); cache tiles shared by 4 or 8, or by 16 queries per warp
+cudaError_t launch_attn_kind(const AttnBatchParams& p, int n_heads, int M, int kind, cudaStream_t st);
 void launch_tp_gather(const TpGatherParams& p, cudaStream_t st);
 // dst[m][ld] (+)= the output of a GEMM, slices added in order; with b: dst = silu(a) * b
 void launch_finish(const TcOut& a, const TcOut* b, float* dst, int ld, bool add, cudaStream_t st);

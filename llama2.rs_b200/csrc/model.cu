@@ -1472,6 +1472,22 @@ extern "C" int l2_attention_decode_dev(int n_heads, int n_kv_heads, int pos, con
     return L2_OK;
 }
 
+extern "C" int l2_debug_attention_batch(int n_heads, int n_kv_heads, int M, int kind, const float* q, const float* key_cache,
+                                        const float* value_cache, const int32_t* pos, float* out, void* cuda_stream) {
+    clear_error();
+    if (n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads || M < 1 || kind < ATTN_HEAD || kind > ATTN_WIDE || !q || !key_cache || !value_cache || !pos || !out)
+        return fail(L2_EINVAL, "l2_debug_attention_batch: bad argument");
+    const int ag = n_heads / n_kv_heads;
+    if (kind != ATTN_HEAD && ag != 1 && ag != 2 && ag != 4 && ag != 8) return fail(L2_EINVAL, "l2_debug_attention_batch: %d query heads per kv head", ag);
+    int device, sms;
+    if (int rc = check_device(-1, &device, &sms)) return rc;
+    AttnBatchParams a{};
+    a.q = q; a.kc = key_cache; a.vc = value_cache; a.pos = pos; a.out = out;
+    a.n_kv_heads = n_kv_heads; a.ag = ag; a.ldq = a.ldo = n_heads * HS;
+    L2_CUDA(launch_attn_kind(a, n_heads, M, kind, static_cast<cudaStream_t>(cuda_stream)));
+    return L2_OK;
+}
+
 // ---- C ABI: one QLinear ---------------------------------------------------------------------------
 
 extern "C" int l2_qlinear_create(int in, int out, int group_size, const int32_t* qweight, const int32_t* qzeros,

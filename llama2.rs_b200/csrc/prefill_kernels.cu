@@ -599,7 +599,11 @@ cudaError_t attn_batch_init() {
 // shapes, 512 CTAs: 1536-token prompt on 4 layers 31.3 -> 29.6 ms; 296 tokens of the 7B shapes, 160 CTAs: 15.2 -> 16.2 ms).
 cudaError_t launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, int sms, cudaStream_t st) {
     const bool wide = (long long)p.n_kv_heads * ((M * p.ag + AW_WARPS * AW_QW - 1) / (AW_WARPS * AW_QW)) * 2 >= 3 * sms;
-    switch (tiled ? p.ag : 0) {
+    return launch_attn_kind(p, n_heads, M, !tiled ? ATTN_HEAD : wide ? ATTN_WIDE : ATTN_TILED, st);
+}
+cudaError_t launch_attn_kind(const AttnBatchParams& p, int n_heads, int M, int kind, cudaStream_t st) {
+    const bool wide = kind == ATTN_WIDE;
+    switch (kind == ATTN_HEAD ? 0 : p.ag) {
         case 1: return wide ? launch_attn_wide<1>(p, M, st) : launch_attn_tiled<1, 4>(p, M, st);
         case 2: return wide ? launch_attn_wide<2>(p, M, st) : launch_attn_tiled<2, 8>(p, M, st);
         case 4: return wide ? launch_attn_wide<4>(p, M, st) : launch_attn_tiled<4, 8>(p, M, st);

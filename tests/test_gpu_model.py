@@ -213,14 +213,14 @@ def test_model_shapes_two_layers(l2, orc, name, gs):
     assert np.array_equal(got["tokens"], want["tokens"])
 
 
-# 1, 2, 4, 8 query heads per kv head; prompts that end inside a warp's tokens, inside and at the end of a tile of 32 positions, and with
-# more than one CTA per kv head
+# 1, 2, 4, 8 query heads per kv head; prompts of a few tokens, and with a last position before and behind the line (192) where kernels
+# that share cache tiles take over, inside and at the end of a tile of 32 positions
 @pytest.mark.parametrize("dim,kvh", [(256, 2), (512, 2), (512, 1), (1024, 1)])
 def test_batched_attention_edges(l2, orc, dim, kvh):
     cfg = tiny_config(l2, group_size=64, n_kv_heads=kvh, dim=dim, hidden=2 * dim, seq_len=256)
     gpu, cpu = make_pair(l2, orc, cfg, seed=23)
     rng = np.random.default_rng(dim * kvh)
-    for n in (3, 15, 34, 65, 131):
+    for n in (3, 15, 34, 65, 131, 193, 195, 225, 251):
         prompt = rng.integers(0, cfg.vocab_size, n).astype(np.int32)
         want = cpu.generate_ids(prompt, n + 4, trace_logits=True)
         got = l2.generate_ids(gpu, prompt, n + 4, trace_logits=True)
