@@ -87,6 +87,14 @@ static int dev_upload(T** p, const void* src, size_t count, std::vector<void*>& 
     return L2_OK;
 }
 
+// What a state's kernels find on the device is cleared and uploaded on the stream they run on: the model's stream waits for no other, so
+// work on the default stream could come after them.  (The source may be reused as soon as this returns.)
+static int upload_on(cudaStream_t st, void* dst, const void* src, size_t bytes) {
+    L2_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+    L2_CUDA(cudaStreamSynchronize(st));
+    return L2_OK;
+}
+
 int upload_qlinear(const PackedQ& p, const int32_t* g_index, DevQ& d, std::vector<void*>& allocs, size_t* bytes) {
     d.in = p.in; d.out = p.out; d.tiles = p.tiles; d.G = p.groups; d.gs = p.w * 32;
     if (int rc = dev_upload(&d.rec, p.rec.data(), p.rec.size(), allocs, bytes)) return rc;
@@ -557,7 +565,7 @@ static int plan_token(l2_state* s) {
         L2_CUDA(token_set_poll_limit(lg ? 1u << lg : 0u));
     }
     if (int rc = dev_alloc(reinterpret_cast<void**>(&s->tk.bar), 256, s->allocs)) return rc;
-    L2_CUDA(cudaMemset(s->tk.bar, 0, 256));
+    L2_CUDA(cudaMemsetAsync(s->tk.bar, 0, 256, m->stream));
     {   // tagged activations, zeroed once: tag 0 is never expected
         const TaggedLayout lay = tagged_layout(m);
         char* pool = nullptr;
@@ -565,7 +573,7 @@ static int plan_token(l2_state* s) {
             pool = m->tp_pool;  // made (and zeroed) by l2_model_tp_pool_handle, known to the peers
         } else {
             if (int rc = dev_alloc(reinterpret_cast<void**>(&pool), lay.total, s->allocs)) return rc;
-            L2_CUDA(cudaMemset(pool, 0, lay.total));
+            L2_CUDA(cudaMemsetAsync(pool, 0, lay.total, m->stream));
         }
         if (!pool) return fail(L2_EINVAL, "token kernel: no activation pool");
         unsigned long long** bufs[11] = {&s->t_x, &s->t_xq, &s->t_xk, &s->t_xv, &s->t_q, &s->t_k, &s->t_v, &s->t_att, &s->t_x1, &s->t_x3, &s->t_hb};
@@ -575,7 +583,7 @@ static int plan_token(l2_state* s) {
         s->tk_max_split = std::max(1, std::min(32, m->sms / std::max(1, c.n_kv_heads / m->tp_world)));
         const size_t part_bytes = (size_t)c.n_heads * s->tk_max_split * (HS + 2) * 8;
         if (int rc = dev_alloc(reinterpret_cast<void**>(&s->t_part), part_bytes, s->allocs)) return rc;
-        L2_CUDA(cudaMemset(s->t_part, 0, part_bytes));
+        L2_CUDA(cudaMemsetAsync(s->t_part, 0, part_bytes, m->stream));
         s->tk.world = m->tp_world;
         s->tk.rank = m->tp_rank;
         for (int r = 0; r < 8; r++) s->tk.pool[r] = r < m->tp_world ? (m->tp_world > 1 ? m->tp_peers[r] : pool) : nullptr;
@@ -704,7 +712,7 @@ static int build_phase_table(l2_state* s, int kind) {
     if (bad) return fail(L2_EINVAL, "token kernel: an activation buffer of the launch plan has no tagged counterpart");
     if (t.size() >= 1024) return fail(L2_EINVAL, "token kernel: %zu phases do not fit the 10-bit phase field of a tag", t.size());
     if (int rc = dev_alloc(reinterpret_cast<void**>(&s->d_phases[kind]), sizeof(PhaseRec) * t.size(), s->allocs)) return rc;
-    L2_CUDA(cudaMemcpy(s->d_phases[kind], t.data(), sizeof(PhaseRec) * t.size(), cudaMemcpyHostToDevice));
+    if (int rc = upload_on(m->stream, s->d_phases[kind], t.data(), sizeof(PhaseRec) * t.size())) return rc;
     s->n_phases[kind] = (int)t.size();
     return L2_OK;
 }
@@ -941,7 +949,8 @@ extern "C" int l2_model_tp_pool_handle(l2_model* m, void* handle64) {
     if (!m->tp_pool) {
         const TaggedLayout lay = tagged_layout(m);
         L2_CUDA(cudaMalloc(reinterpret_cast<void**>(&m->tp_pool), lay.total));
-        L2_CUDA(cudaMemset(m->tp_pool, 0, lay.total));
+        L2_CUDA(cudaMemsetAsync(m->tp_pool, 0, lay.total, m->stream));
+        L2_CUDA(cudaStreamSynchronize(m->stream));  // before a peer can write into it
         m->tp_peers[m->tp_rank] = m->tp_pool;
         for (int i = 0; i < 3; i++) m->tp_batch_off[i] = lay.batch_off[i];
         m->tp_flag_off = lay.flag_off;
@@ -1051,10 +1060,7 @@ extern "C" int l2_state_new(l2_model* m, l2_state** out) {
                 if ((rc = plan_layer_gemv(s.get(), l, which, s->plans[(size_t)l * 4 + which]))) { free_allocs(s->allocs); return rc; }
                 host[(size_t)l * 4 + which] = s->plans[(size_t)l * 4 + which].p;
             }
-        if (cudaMemcpy(s->d_plans, host.data(), sizeof(SkParams) * host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-            free_allocs(s->allocs);
-            return fail(L2_ECUDA, "uploading the launch records failed");
-        }
+        if ((rc = upload_on(m->stream, s->d_plans, host.data(), sizeof(SkParams) * host.size()))) { free_allocs(s->allocs); return rc; }
     }
     if (cudaMallocHost(reinterpret_cast<void**>(&s->h_ctl), sizeof(Ctl) * CTL_RING) != cudaSuccess) {
         free_allocs(s->allocs);
@@ -1357,6 +1363,7 @@ extern "C" int l2_debug_trace(int enable, unsigned long long* host_out, int n_ct
     if (enable && !g_sk_trace) {
         L2_CUDA(cudaMalloc(&g_sk_trace, sizeof(unsigned long long) * 8 * 1024));
         L2_CUDA(cudaMemset(g_sk_trace, 0, sizeof(unsigned long long) * 8 * 1024));
+        L2_CUDA(cudaStreamSynchronize(nullptr));
     }
     if (host_out && g_sk_trace) {
         L2_CUDA(cudaDeviceSynchronize());
@@ -1378,7 +1385,7 @@ extern "C" int l2_debug_token_trace(l2_state* s, int enable, unsigned long long*
             if (int rc = dev_alloc(reinterpret_cast<void**>(&s->tk_trace), count * 8, s->allocs)) return rc;
         }
         if (count > s->tk_trace_count) return fail(L2_EINVAL, "l2_debug_token_trace: the buffer holds %zu stamps", s->tk_trace_count);
-        L2_CUDA(cudaMemset(s->tk_trace, 0, s->tk_trace_count * 8));
+        L2_CUDA(cudaMemsetAsync(s->tk_trace, 0, s->tk_trace_count * 8, s->m->stream));
         for (auto& g : s->graphs)  // captured launches carry the old setting
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         return L2_OK;

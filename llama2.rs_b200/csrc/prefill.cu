@@ -104,7 +104,7 @@ static cudaError_t alloc_batch(l2_model* m, int cap) {
         b->att = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[1]);
         b->hb = reinterpret_cast<float*>(m->tp_pool + m->tp_batch_off[2]);
         b->tp_done = reinterpret_cast<unsigned*>(base + done);
-        if (cudaError_t e = cudaMemset(b->tp_done, 0, 256)) { free_batch(m); return e; }
+        if (cudaError_t e = cudaMemsetAsync(b->tp_done, 0, 256, m->stream)) { free_batch(m); return e; }
     }
     if (cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), sizeof(int) * 2 * B * BATCH_RING)) { free_batch(m); return e; }
     return cudaSuccess;

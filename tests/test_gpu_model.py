@@ -227,3 +227,29 @@ def test_batched_attention_edges(l2, orc, dim, kvh):
         assert got["pos0"] == want["pos0"]
         assert_close(got["logits"], want["logits"], what="logits after %d prompt tokens" % n)
         assert np.array_equal(got["tokens"], want["tokens"])
+
+
+def test_first_calls_of_a_state_beside_a_busy_default_stream(l2):
+    # what a state's first calls clear and upload is on the model's own stream: work on the default stream does not come in between
+    import torch
+    cfg = tiny_config(l2, group_size=64, n_kv_heads=1, dim=512, hidden=1024, seq_len=256)
+    model = l2.LlamaModel.synthetic(cfg, 31)
+    prompt = np.random.default_rng(31).integers(0, cfg.vocab_size, 200).astype(np.int32)
+
+    def run(state):
+        at = l2.prefill(model, state, prompt)
+        forced = l2.decode_run(model, state, prompt, at, len(prompt))
+        return at, forced, l2.decode_step(model, state, int(prompt[-1]), len(prompt), want_logits=True)
+
+    at, forced, (token, logits) = run(l2.RunState(model))
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    torch.cuda._sleep(600_000_000)  # about 0.3 s
+    done.record()
+    state = l2.RunState(model)
+    while True:
+        last = done.query()
+        got = run(state)
+        assert got[0] == at and np.array_equal(got[1], forced) and got[2][0] == token and np.array_equal(got[2][1], logits)
+        if last:
+            break
