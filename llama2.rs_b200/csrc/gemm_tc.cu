@@ -230,7 +230,7 @@ __device__ __forceinline__ void add16(const uint32_t (&c)[2][16], unsigned long 
 // index in the CTA modulo 4; the first four drain warps take the first weight tile's accumulator, the others the second's.
 template <int W, int NT>
 __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, Walk& walk) {
-    constexpr int RT = 2, tq = 16 * NT, GPS = 4 / W;
+    constexpr int RT = TC_TILE_ROWS / 128, tq = 16 * NT, GPS = 4 / W;
     using S = TcShape<NT>;
     constexpr uint32_t UB = 256u * W + 80u;
     const int quad = D.warp & 3, rec16 = D.lane & 7, rr = 4 * quad + (D.lane >> 3), rt = (D.warp - TC_LOAD_WARPS) >> 2;
@@ -309,7 +309,7 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
 template <int W, int NT>
 __global__ void __maxnreg__(TcShape<NT>::LAUNCH) gemm_q4_tc_kernel(const __grid_constant__ TcParams P) {
     using S = TcShape<NT>;
-    constexpr int RT = 2, tq = 16 * NT;                      // weight tiles of a tile; tokens of a block
+    constexpr int RT = TC_TILE_ROWS / 128, tq = 16 * NT;     // weight tiles of a tile; tokens of a block
     constexpr int GS = 32 * W, GPS = TC_KSTEP / GS;          // inputs per group, groups per K step
     constexpr uint32_t UB = 256u * W + 80u;                  // bytes of a unit record
     constexpr uint32_t RUN = tc_run_bytes(W);                // room of a record run (16 rows x one K step)
@@ -534,8 +534,7 @@ void gemm_tc_tokens(int M, int* tq, int* ntb) {  // blocks of at most 64 tokens,
     *tq = ((M + *ntb - 1) / *ntb + 15) & ~15;
 }
 
-size_t gemm_tc_image_bytes(int in, int gs, int tokens) {
-    (void)gs;
+size_t gemm_tc_image_bytes(int in, int tokens) {
     return (size_t)((in + TC_KSTEP - 1) / TC_KSTEP) * 512 * ((tokens + TC_MAX_TOKENS - 1) / TC_MAX_TOKENS * TC_MAX_TOKENS);
 }
 
@@ -547,10 +546,9 @@ void gemm_tc_plan(TcParams& p, int gs, int sms) {
     gemm_tc_tokens(p.M, &p.tq, &p.ntb);
     p.gs = gs;
     p.KS = (p.G * gs + TC_KSTEP - 1) / TC_KSTEP;
-    p.rt = 2;
     int tiles = 0;
     for (int i = 0; i < p.nmat; i++) {
-        tiles += (p.mat[i].tiles16 + 8 * p.rt - 1) / (8 * p.rt) * p.ntb;
+        tiles += (p.mat[i].tiles16 + TC_TILE_ROWS / 16 - 1) / (TC_TILE_ROWS / 16) * p.ntb;
         p.mat[i].tile_end = tiles;
     }
     p.total = tiles * p.KS;

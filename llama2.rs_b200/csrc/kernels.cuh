@@ -89,7 +89,7 @@ struct TcParams {
     int* status;
     int nmat, M, tq, ntb;  // tokens, tokens per block (a multiple of 16), token blocks
     int G, gs, KS;         // groups of a row, their size, K steps of 128 inputs
-    int rt, total, q, grid;  // 128-row tiles per tile, (tile, K step) pairs of the launch, pairs per CTA, CTAs
+    int total, q, grid;    // (tile, K step) pairs of the launch, pairs per CTA, CTAs
     int nraw;              // slots of the raw weight ring
 };
 // How the readers of a launch's output find its slices: out plus the parts of slices 1 .. n - 1, in that order.
@@ -136,7 +136,7 @@ struct RowParams {
     TcOut a, b;            // RESID: a is added to x; SWIGLU: silu(a) * b
     const float* nw;       // rmsnorm weight, natural order, or null (no norm)
     float eps;
-    int in, gs, ldx, M, tq, ntb, KS, nmat;
+    int in, ldx, M, tq, KS, nmat;
     const uint16_t* perm[3];  // consumers' K orders (16-bit g_index), or null: the row is in K order
     uint8_t* img[3];       // [token block][K step][half][2 tq][64] f16 digits, swizzled
     float* osc;            // [M] factors
@@ -278,7 +278,7 @@ size_t sk_slot_bytes(int group_size, int chunk);           // one ring slot of o
 cudaError_t sk_init(int max_smem);
 void launch_embed_batch(const float* table, const int* tokens, float* x, int dim, int M, cudaStream_t st);
 cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st);
-cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st);
+cudaError_t launch_rope_append(const RopeParams& p, int M, int sms, cudaStream_t st);
 cudaError_t launch_attn_batch(const AttnBatchParams& p, int n_heads, int M, bool tiled, int sms, cudaStream_t st);
 enum : int { ATTN_HEAD = 0, ATTN_TILED = 1, ATTN_WIDE = 2 };  // one CTA per (head, token); cache tiles shared by 4 or 8, or by 16 queries per warp
 cudaError_t launch_attn_kind(const AttnBatchParams& p, int n_heads, int M, int kind, cudaStream_t st);
@@ -292,7 +292,7 @@ cudaError_t row_quant_init(int max_smem);
 void gemm_tc_plan(TcParams& p, int gs, int sms);         // geometry of a launch whose matrices, G and M are set
 int gemm_tc_slices(const TcParams& p);                   // slices the most divided tile can have
 void gemm_tc_tokens(int M, int* tq, int* ntb);           // token blocks of a batch
-size_t gemm_tc_image_bytes(int in, int gs, int tokens);  // digit image of up to `tokens` activation rows for a matrix with IN = in
+size_t gemm_tc_image_bytes(int in, int tokens);  // digit image of up to `tokens` activation rows for a matrix with IN = in
 extern unsigned long long* g_sk_trace;  // device buffer for SkParams::trace when tracing is on
 void launch_attn(const AttnParams& p, cudaStream_t st, bool pdl);
 void launch_cls(const ClsParams& p, int grid, cudaStream_t st, bool pdl);

@@ -1555,7 +1555,7 @@ static int qlinear_reserve(l2_qlinear* h, int B, bool host) {
     const int rows[1] = {h->q.out};
     size_t total = 0;
     auto room = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
-    const size_t img = room(gemm_tc_image_bytes(h->q.in, h->q.gs, cap)), osc = room(sizeof(float) * cap),
+    const size_t img = room(gemm_tc_image_bytes(h->q.in, cap)), osc = room(sizeof(float) * cap),
                  part = room(sizeof(float) * part_floats(rows, 1, h->q.in, h->q.gs, cap, h->sms));
     char* base = nullptr;
     if ((rc = dev_alloc(reinterpret_cast<void**>(&base), total, h->allocs))) return rc;

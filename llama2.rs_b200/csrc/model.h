@@ -98,7 +98,7 @@ struct l2_model {
     // pools mapped through CUDA IPC; the first run state of the model works in the pool
     char* tp_pool = nullptr;
     char* tp_peers[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    size_t tp_batch_off[3] = {0, 0, 0};   // batched forward under tensor parallelism: x, att, hb ([MAX_BATCH][dim or hidden] f32) inside the pool
+    size_t tp_batch_off[3] = {0, 0, 0};   // batched forward under tensor parallelism: x, att, hb ([TC_MAX_TOKENS][dim or hidden] f32) inside the pool
     size_t tp_flag_off = 0;               // [8] arrival counters of its exchanges; at + 128 bytes this rank's count of exchanges made
     bool tp_peer_borrowed[8] = {false, false, false, false, false, false, false, false};  // attached by pointer: not an IPC mapping to close
     bool tp_direct = false;          // every rank's pool is attached
@@ -149,7 +149,7 @@ struct l2_qlinear {
     l2::SkLaunch plan;                   // B = 1: launch plan and its record on the device
     l2::SkParams* d_plan = nullptr;
     bool planned = false;                // the record is there
-    uint8_t* img = nullptr;   // batched path: digit image with the digit sums, and the factors
+    uint8_t* img = nullptr;   // batched path: digit image, and the tokens' factors
     float* osc = nullptr;
     float* kpart = nullptr;   // slices of the output beyond the first
     int* status = nullptr;    // device word that a kernel whose wait gave up writes (batched path); one for the handle's life, cleared when reported

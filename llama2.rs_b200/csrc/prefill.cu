@@ -28,19 +28,19 @@ TcOut tc_out(const TcParams& t, int i) {
     return o;
 }
 
-static RowParams row_params(int mode, int in, int gs, const TcParams& t) {
+static RowParams row_params(int mode, int in, const TcParams& t) {
     RowParams r{};
-    r.mode = mode; r.in = in; r.gs = gs; r.M = t.M; r.tq = t.tq; r.ntb = t.ntb; r.KS = t.KS;
+    r.mode = mode; r.in = in; r.M = t.M; r.tq = t.tq; r.KS = t.KS;
     return r;
 }
 
-// out[m][:] = QLinear(x[m][:]) for m < M, x in natural order.  part: room for (slices - 1) * M * rows floats (qlinear_part_floats).
+// out[m][:] = QLinear(x[m][:]) for m < M, x in natural order.  part: room for (slices - 1) * M * rows floats (part_floats).
 int gemm_batched(const DevQ& q, const float* x, int M, uint8_t* img, float* osc, float* out, float* part, int* status, int sms, cudaStream_t st) {
     TcParams t{};
     t.nmat = 1; t.M = M; t.osc = osc; t.status = status;
     tc_set_matrix(t, 0, q, img, out, q.out, part);
     gemm_tc_plan(t, q.gs, sms);
-    RowParams r = row_params(ROW_PLAIN, q.in, q.gs, t);
+    RowParams r = row_params(ROW_PLAIN, q.in, t);
     r.x = const_cast<float*>(x); r.ldx = q.in; r.nmat = 1; r.perm[0] = q.perm16; r.img[0] = img; r.osc = osc;
     L2_CUDA(launch_row_quant(r, sms, st));
     L2_CUDA(launch_gemm_tc(t, st));
@@ -86,7 +86,7 @@ static cudaError_t alloc_batch(l2_model* m, int cap) {
     size_t total = 0;
     auto room = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
     const size_t x = tp ? 0 : room(B * D * 4), att = tp ? 0 : room(B * D * 4), q = room(B * Dl * 4), y = room(B * outs * 4), part = room(parts * 4), osc = room(B * 4);
-    const size_t img0 = room(gemm_tc_image_bytes(std::max(D, H), gs, cap)), img1 = room(gemm_tc_image_bytes(D, gs, cap)), img2 = room(gemm_tc_image_bytes(D, gs, cap));
+    const size_t img0 = room(gemm_tc_image_bytes(std::max(D, H), cap)), img1 = room(gemm_tc_image_bytes(D, cap)), img2 = room(gemm_tc_image_bytes(D, cap));
     const size_t tok = room(2 * B * sizeof(int)), done = room(256);
     char* base = nullptr;
     if (cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base), total)) {
@@ -142,7 +142,7 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
     const int D = c.dim, KV = m->shape.kv_dim(), H = c.hidden_dim, gs = c.group_size;
     // this rank's share (everything on one GPU): rows of wq / wo (= heads), of wk / wv (= kv heads), of w1 / w3 / w2's inputs
     const int T = b->tp ? m->tp_world : 1, R = b->tp ? m->tp_rank : 0;
-    const int Dl = D / T, KVl = KV / T, Hl = H / T, heads_l = c.n_heads / T, kvh_l = c.n_kv_heads / T;
+    const int Dl = D / T, KVl = KV / T, heads_l = c.n_heads / T, kvh_l = c.n_kv_heads / T;
     int* status = &s->ctl->status;
     const int* tok = b->tok;
     const int* pos = b->tok + M;
@@ -186,7 +186,7 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
     for (int l = 0; l < c.n_layers; l++) {
         const DevLayer& y = m->layers[l];
         auto with_x = [&](const float* nw) {
-            RowParams r = row_params(pending ? ROW_RESID : ROW_PLAIN, D, gs, t);
+            RowParams r = row_params(pending ? ROW_RESID : ROW_PLAIN, D, t);
             r.x = b->x; r.ldx = D; r.a = resid; r.nw = nw;
             pending = false;
             return r;
@@ -208,7 +208,7 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
         r.kc = s->kc + (size_t)l * ls + (size_t)R * KVl; r.vc = s->vc + (size_t)l * ls + (size_t)R * KVl;
         r.rope_cos = m->rope_cos; r.rope_sin = m->rope_sin; r.pos = pos;
         r.n_heads = heads_l; r.n_kv_heads = kvh_l; r.kv_stride = KV;
-        L2_CUDA(launch_rope_append(r, M, st));
+        L2_CUDA(launch_rope_append(r, M, m->sms, st));
         AttnBatchParams a{};
         a.q = b->q; a.kc = r.kc; a.vc = r.vc; a.pos = pos; a.out = b->att + (size_t)R * Dl;
         a.n_kv_heads = kvh_l; a.ag = m->shape.attn_groups(); a.ldq = Dl; a.ldo = D; a.kv_stride = KV;
@@ -216,7 +216,7 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
         gather(1, D, R * Dl, Dl);
         // wo + residual (:260-264)
         launch({&y.wo}, t);
-        RowParams ra = row_params(ROW_PLAIN, D, gs, t);
+        RowParams ra = row_params(ROW_PLAIN, D, t);
         ra.x = b->att; ra.ldx = D;
         L2_CUDA(quant(ra, {&y.wo}, true));
         L2_CUDA(launch_gemm_tc(t, st));
@@ -228,13 +228,12 @@ static int enqueue_batch(l2_state* s, int M, bool long_context, cudaStream_t st)
         const TcOut h1 = tc_out(t, 0), h3 = tc_out(t, 1);
         // w2 + residual (:279-285)
         launch({&y.w2}, t);
-        RowParams rh = row_params(b->tp ? ROW_PLAIN : ROW_SWIGLU, H, gs, t);
+        RowParams rh = row_params(b->tp ? ROW_PLAIN : ROW_SWIGLU, H, t);
         rh.a = h1; rh.b = h3; rh.x = b->hb; rh.ldx = H;
         if (b->tp) { launch_finish(h1, &h3, b->hb + y.w1.row0, H, false, st); gather(2, H, y.w1.row0, y.w1.out); }
         L2_CUDA(quant(rh, {&y.w2}, false));
         L2_CUDA(launch_gemm_tc(t, st));
         add_to_x(y.w2);
-        (void)Hl;
     }
     L2_CUDA(cudaGetLastError());
     return L2_OK;

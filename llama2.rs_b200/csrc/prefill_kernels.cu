@@ -276,9 +276,9 @@ cudaError_t launch_row_quant(const RowParams& p, int sms, cudaStream_t st) {
     return launch_pdl(row_quant_kernel, dim3(C, p.M), dim3(RQ_THREADS), share(C), C, st, p);
 }
 
-cudaError_t launch_rope_append(const RopeParams& p, int M, cudaStream_t st) {
+cudaError_t launch_rope_append(const RopeParams& p, int M, int sms, cudaStream_t st) {
     const int units = (p.n_heads + 2 * p.n_kv_heads) * (HS / 8);
-    return launch_pdl(rope_append_kernel, dim3(M, std::max(1, std::min((units + 255) / 256, 592 / M))), dim3(256), 0, 0, st, p);
+    return launch_pdl(rope_append_kernel, dim3(M, std::max(1, std::min((units + 255) / 256, 4 * sms / M))), dim3(256), 0, 0, st, p);
 }
 
 // ---- the same attention with the cache rows shared by the queries that need them ---------------------------------------
