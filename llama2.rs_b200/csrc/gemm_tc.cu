@@ -251,6 +251,10 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
         const char* sp = reinterpret_cast<const char*>(X.rec) + ((size_t)min((sg.pair * RT + rt) * 8 + rec16, X.tiles16 - 1) * P.G + g0) * UB + 256 * W + 4 * rr;
         auto scale = [&](int ahead) { return __ldg(reinterpret_cast<const float*>(sp + (size_t)min(ahead, n - 1) * UB)); };
         float s_a = scale(0), s_b = scale(1), s_c = scale(2);
+        // The tokens' factors, one or two per lane, well before they are needed.  They are the output of the kernel in front, which may run beside this
+        // one until the wait above: no read-only loads.
+        const int t0 = sg.tb * tq + D.lane;
+        const float f0 = D.lane < tq && t0 < P.M ? P.osc[t0] : 0.f, f1 = NT > 2 && D.lane + 32 < tq && t0 + 32 < P.M ? P.osc[t0 + 32] : 0.f;
 #pragma unroll
         for (int i = 0; i < 8 * NT; i++) acc[i] = 0ull;
 #pragma unroll 1
@@ -280,25 +284,16 @@ __device__ __forceinline__ bool drain_tiles(const TcParams& P, const Drain& D, W
         }
         w0.next(P, sg);  // (worked out again: the coordinates would take registers from the loop above)
         // ---- this tile's share of the output: slice 0 goes to the output rows, later slices to the part buffers
-        if (*D.failed) return false;
+        if (__any_sync(0xffffffffu, *D.failed)) return false;  // (the whole warp: the factors below are shuffled)
         const int orow = (sg.pair * RT + rt) * 128 + rec16 * 16 + rr, m0 = sg.tb * tq;
         const size_t ld = sg.slice == 0 ? (size_t)X.ldo : (size_t)X.rows;
         float* dst = (sg.slice == 0 ? X.out : X.part + (size_t)(sg.slice - 1) * P.M * X.rows) + (size_t)m0 * ld + orow;
-        if (orow < X.rows) {
 #pragma unroll
-            for (int st = 0; st < NT; st++) {
-                // The factors are the output of the kernel in front, which may run beside this one: no read-only loads.  16 at a time in front of
-                // their stores (a plain load does not move past a store).
-                float f[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) f[i] = m0 + 16 * st + i < P.M ? P.osc[m0 + 16 * st + i] : 0.f;
-#pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    const float2 y = unpack2(acc[8 * st + i / 2]);
-                    if (m0 + 16 * st + i < P.M) dst[(size_t)(16 * st + i) * ld] = y.x * f[i];
-                    if (m0 + 16 * st + i + 1 < P.M) dst[(size_t)(16 * st + i + 1) * ld] = y.y * f[i + 1];
-                }
-            }
+        for (int i = 0; i < 16 * NT; i += 2) {
+            const float2 y = unpack2(acc[i / 2]);
+            const float fa = __shfl_sync(0xffffffffu, i < 32 ? f0 : f1, i & 31), fb = __shfl_sync(0xffffffffu, i < 32 ? f0 : f1, (i + 1) & 31);
+            if (orow < X.rows && m0 + i < P.M) dst[(size_t)i * ld] = y.x * fa;
+            if (orow < X.rows && m0 + i + 1 < P.M) dst[(size_t)(i + 1) * ld] = y.y * fb;
         }
     }
     return true;
