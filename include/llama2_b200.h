@@ -54,7 +54,7 @@ typedef struct l2_options {
     int32_t attn_groups;    /* ATTN_GROUPS when model_size is NULL (1 = no GQA) */
     int32_t device;         /* CUDA device ordinal, -1 = current device */
     int32_t debug;          /* print the configuration, as LlamaModel::from_file(debug=true) does */
-    int32_t max_batch;      /* largest B accepted by l2_forward / prefill chunk (0 = default 64) */
+    int32_t max_batch;      /* largest B accepted by l2_forward (0 = default 64); prefill chooses its own batches */
     int32_t flags;          /* L2_FLAG_* */
     int32_t tp_rank;        /* tensor parallelism: this process's rank ... */
     int32_t tp_world;       /* ... of tp_world processes, one per GPU of the box (0 or 1 = single GPU) */

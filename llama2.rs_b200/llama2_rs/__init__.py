@@ -326,6 +326,7 @@ class QLinear:
         return out[0] if one else out
 
     def matvec_dev(self, x_ptr, out_ptr, B, stream=0):
+        """The same on device arrays, enqueued on `stream` (a cudaStream_t); 0: ordered with the default stream."""
         check(lib.l2_qlinear_matvec_dev(self._h, C.c_void_p(x_ptr), C.c_void_p(out_ptr), B, C.c_void_p(stream)))
 
     def __del__(self):

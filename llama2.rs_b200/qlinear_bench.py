@@ -6,8 +6,8 @@
 Weights have the value distributions of the synthetic checkpoint (nibbles U{0..15}, zero nibbles U{6..9}, scales
 U[0.002, 0.02], act-order g_index from a seeded permutation), activations are N(0,1) f32, resident on the device.
 Per case one line: microseconds per call (CUDA events on the launching stream, warm-up first), the checkpoint bytes of the
-matrix per second, and useful int8 TFLOP/s (2 M K N).  B = 1 runs the GEMV kernel, B >= 2 the tcgen05 GEMM (a call is the
-activation quantiser, the GEMM and, where the groups of a tile are split over CTAs, the kernel that adds the slices).
+matrix per second (read once per pass of 512 rows), and useful TFLOP/s (2 M K N).  B = 1 runs the GEMV kernel, B >= 2 the tcgen05 GEMM (a call is the
+row quantiser, the GEMM and, where a tile's inputs are split over CTAs, the kernel that adds the slices).
 """
 import argparse
 import os
@@ -55,6 +55,7 @@ def main():
                 x = torch.randn(M, K, device="cuda")
                 y = torch.empty(M, N, device="cuda")
                 s = torch.cuda.Stream()
+                torch.cuda.synchronize()
                 with torch.cuda.stream(s):
                     for _ in range(args.warmup):
                         q.matvec_dev(x.data_ptr(), y.data_ptr(), M, s.cuda_stream)
@@ -65,7 +66,7 @@ def main():
                     e1.record(s)
                 torch.cuda.synchronize()
                 us = e0.elapsed_time(e1) / args.iters * 1e3
-                passes = (M + 63) // 64
+                passes = (M + 511) // 512
                 print("K %5d N %5d g%-3d M %3d: %8.1f us/call  %7.1f GB/s of checkpoint bytes (%d pass%s)  %6.1f TFLOP/s" %
                       (K, N, gs, M, us, wbytes * passes / us / 1e3, passes, "" if passes == 1 else "es", 2.0 * M * K * N / us / 1e6), flush=True)
             del q
