@@ -120,11 +120,19 @@ __device__ __forceinline__ void mbar_arrive_u32(uint32_t bar) {
 // barrier of the SK_THREADS consumer threads only (the producer warp runs on its own)
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SK_THREADS) : "memory"); }
 
+// The larger of two values, NaN if either is one (fmaxf drops it): the largest magnitude of a vector taken with this is finite only
+// if every element is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
 __device__ __forceinline__ float block_reduce_2(float& mx, float sq, float* red /* 2*SK_WARPS+2 floats */) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         sq += __shfl_xor_sync(0xffffffffu, sq, o);
     }
     if (lane == 0) { red[warp] = mx; red[SK_WARPS + warp] = sq; }
@@ -134,7 +142,7 @@ __device__ __forceinline__ float block_reduce_2(float& mx, float sq, float* red 
         float s = lane < SK_WARPS ? red[SK_WARPS + lane] : 0.f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
             s += __shfl_xor_sync(0xffffffffu, s, o);
         }
         if (lane == 0) { red[2 * SK_WARPS] = m; red[2 * SK_WARPS + 1] = s; }
@@ -235,8 +243,8 @@ __device__ __forceinline__ void stage_fetch(const SkSeg& sg, int blk, float4& v0
         v1.x *= w1.x; v1.y *= w1.y; v1.z *= w1.z; v1.w *= w1.w;
     }
     if (stats) {
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v0.x), fabsf(v0.y)), fmaxf(fabsf(v0.z), fabsf(v0.w))));
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v1.x), fabsf(v1.y)), fmaxf(fabsf(v1.z), fabsf(v1.w))));
+        mx = max_nan(mx, max_nan(max_nan(fabsf(v0.x), fabsf(v0.y)), max_nan(fabsf(v0.z), fabsf(v0.w))));
+        mx = max_nan(mx, max_nan(max_nan(fabsf(v1.x), fabsf(v1.y)), max_nan(fabsf(v1.z), fabsf(v1.w))));
     }
 }
 
@@ -295,7 +303,8 @@ __device__ __forceinline__ void stage_emit(uint8_t* digits, int* ss, int stride,
 }
 
 // Turns the vector of one segment into digits and per-group digit sums in shared memory.
-// Returns (in every thread) the factor the integer result has to be multiplied with.
+// Returns (in every thread) the factor the integer result has to be multiplied with: NaN for a vector that holds a NaN or an
+// infinity, which has no digits and makes every output NaN.
 template <int W>
 __device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digits, int* ss, float* red, unsigned long long* dbg = nullptr,
                               uint32_t tag = 0, bool* fail = nullptr) {
@@ -340,7 +349,7 @@ __device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digit
         }
     }
     if (dbg && threadIdx.x == 0) dbg[2] = clock64();
-    return rs / P;
+    return mx < INFINITY ? rs / P : NAN;
 }
 
 // Two segments whose vectors are two orderings of the same values (w1 and w3 read the same x, each
