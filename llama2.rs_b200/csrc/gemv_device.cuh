@@ -128,6 +128,16 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     return m;
 }
 
+__device__ __forceinline__ float max_nan(float a, float b, float c) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
+// The largest of the magnitudes of eight values (instructions of three operands: one of two each was 0.3 to 0.5 % of a token slower).
+__device__ __forceinline__ float max_abs8(const float4& a, const float4& b) {
+    return max_nan(max_nan(max_nan(fabsf(a.x), fabsf(a.y), fabsf(a.z)), max_nan(fabsf(a.w), fabsf(b.x), fabsf(b.y)), fabsf(b.z)), fabsf(b.w));
+}
+
 __device__ __forceinline__ float block_reduce_2(float& mx, float sq, float* red /* 2*SK_WARPS+2 floats */) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
@@ -243,17 +253,14 @@ __device__ __forceinline__ void stage_fetch(const SkSeg& sg, int blk, float4& v0
         v1.x *= w1.x; v1.y *= w1.y; v1.z *= w1.z; v1.w *= w1.w;
     }
     if (stats) {
-        mx = max_nan(mx, max_nan(max_nan(fabsf(v0.x), fabsf(v0.y)), max_nan(fabsf(v0.z), fabsf(v0.w))));
-        mx = max_nan(mx, max_nan(max_nan(fabsf(v1.x), fabsf(v1.y)), max_nan(fabsf(v1.z), fabsf(v1.w))));
+        mx = max_nan(mx, max_abs8(v0, v1));
     }
 }
 
-// P = 2^(26 - E) with 2^E <= mx < 2^(E+1): |v * P| < 2^27 for every |v| <= mx
+// P = 2^(26 - E) with 2^E <= mx < 2^(E+1): |v * P| < 2^27 for every |v| <= mx.  At most 2^100: smaller values are rounded to a multiple
+// of 2^-100.  (Where mx is not finite, P is 2^-102 and the caller answers for it.)
 __device__ __forceinline__ float stage_scale(float mx) {
-    int e = 0;
-    if (mx > 0.f && mx < INFINITY) e = 26 - (int)((__float_as_uint(mx) >> 23) & 255u) + 127;
-    e = max(-100, min(100, e));
-    return __uint_as_float((uint32_t)(127 + e) << 23);
+    return __uint_as_float(min(127u + 100u, 127u + 26u + 127u - (__float_as_uint(mx) >> 23)) << 23);
 }
 
 // Writes the digits of block `blk` (8 values v0, v1 scaled by P) and adds them to the group sums.
@@ -405,17 +412,17 @@ __device__ float stage_digits_pair(const SkSeg& sa, const SkSeg& sb, int in, flo
 // Layout in shared memory: digits [4 planes][pstride], plane 0 the most significant digit, a plane holding
 // the K orders of the phase's matrices one after the other; sp [groups] records of four words
 // {256 * S0 + S1, f * 2^16, 256 * S2 + S3, f}: the digit sums of the upper and of the lower digit pair, each
-// followed by the factor its MMA columns are scaled with (f = 2^-(26 - E_g); the upper pair weighs 2^16 more).  For groups of 64
-// and 128 the sums are stored times 16 and the factors over 16 (the main loop leaves high nibbles in place).
+// followed by the factor its MMA columns are scaled with (f = 2^-(26 - E_g); the upper pair weighs 2^16 more).  The second factor of a
+// group that holds a NaN or an infinity is NaN, which makes every output of the vector NaN.  For groups of 64 and 128 the sums are stored
+// times 16 and the factors over 16 (the main loop leaves high nibbles in place).
 
 // Turns 8 values of K-order block `blk` into digits and finishes the group's record.
 template <int W>
 __device__ __forceinline__ void stage_emit8(float (&v)[8], bool valid, int blk, uint8_t* digits, int pstride, uint4* sp) {
-    float mx = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))),
-                     fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
+    float mx = max_abs8(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
     // (a group's 4 * W lanes reduce with shuffles: redux.sync on a part of the warp was measured slower here)
 #pragma unroll
-    for (int o = 1; o < 4 * W; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = 1; o < 4 * W; o <<= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     const float P = stage_scale(mx);
     uint32_t E[8];  // per element: bytes d3, d2, d1, d0 (least significant digit first)
 #pragma unroll
@@ -449,11 +456,11 @@ __device__ __forceinline__ void stage_emit8(float (&v)[8], bool valid, int blk, 
         s23 += __shfl_xor_sync(0xffffffffu, s23, o);
     }
     if (valid && (threadIdx.x & (4 * W - 1)) == 0) {
-        // 1 / P, exact (P is a power of two between 2^-100 and 2^100, so nothing below leaves the range); where the main loop works
-        // with 16 times the integers, the sums and the factor follow
+        // 1 / P, exact (P is a power of two between 2^-102 and 2^100, so nothing below leaves the range); where the main loop works
+        // with 16 times the integers, the sums and the factor follow.  0 * mx is 0, or NaN where mx is not finite.
         constexpr int X16 = W >= 2 ? 4 : 0;
         const uint32_t f = ((254u - X16) << 23) - __float_as_uint(P);
-        sp[blk / (4 * W)] = make_uint4((uint32_t)s01 << X16, f + (16u << 23), (uint32_t)s23 << X16, f);
+        sp[blk / (4 * W)] = make_uint4((uint32_t)s01 << X16, f + (16u << 23), (uint32_t)s23 << X16, __float_as_uint(fmaf(mx, 0.f, __uint_as_float(f))));
     }
 }
 

@@ -48,7 +48,7 @@ def words(cfg):
 @pytest.mark.parametrize("gs", [32, 64, 128])
 @pytest.mark.parametrize("where", ["wv", "w3", "embedding", "wo"])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
-@pytest.mark.parametrize("flags", [8])  # one launch per operator
+@pytest.mark.parametrize("flags", [0, 8])  # the token kernel; one launch per operator
 def test_in_the_forward(l2, orc, gs, where, value, flags):
     cfg = tiny_config(l2, group_size=gs, n_kv_heads=2)
     payload = l2.synth_fill(cfg, 41)
