@@ -239,20 +239,18 @@ __global__ void __launch_bounds__(SK_THREADS + 32, 1) gemv_sk_kernel(const SkPar
         }
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (!P.debug_skip) {
-            const uint8_t* base = ring + (size_t)slot * slot_bytes;
-            for (int j = 2 * warp; j < m; j += 2 * SK_WARPS) {
-                const bool two = j + 1 < m;
-                int tl0, seg0, g0, tl1 = 0, seg1 = 0, g1 = 0;
-                locate(k * SU + j, tl0, seg0, g0);
-                if (two) { g1 = g0 + 1; seg1 = seg0; tl1 = tl0; if (g1 == G) locate(k * SU + j + 1, tl1, seg1, g1); }
-                int c0[4], c1[4];
-                const uint8_t* rec0 = base + (size_t)j * UB;
-                unit_mma(rec0, digits_of(seg0, g0), c0);
-                if (two) unit_mma(rec0 + UB, digits_of(seg1, g1), c1);
-                unit_finish(rec0, tl0, seg0, g0, c0);
-                if (two) unit_finish(rec0 + UB, tl1, seg1, g1, c1);
-            }
+        const uint8_t* base = ring + (size_t)slot * slot_bytes;
+        for (int j = 2 * warp; j < m; j += 2 * SK_WARPS) {
+            const bool two = j + 1 < m;
+            int tl0, seg0, g0, tl1 = 0, seg1 = 0, g1 = 0;
+            locate(k * SU + j, tl0, seg0, g0);
+            if (two) { g1 = g0 + 1; seg1 = seg0; tl1 = tl0; if (g1 == G) locate(k * SU + j + 1, tl1, seg1, g1); }
+            int c0[4], c1[4];
+            const uint8_t* rec0 = base + (size_t)j * UB;
+            unit_mma(rec0, digits_of(seg0, g0), c0);
+            if (two) unit_mma(rec0 + UB, digits_of(seg1, g1), c1);
+            unit_finish(rec0, tl0, seg0, g0, c0);
+            if (two) unit_finish(rec0 + UB, tl1, seg1, g1, c1);
         }
         __syncwarp();  // every lane has read the slot
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(empty + slot)) : "memory");

@@ -69,7 +69,6 @@ struct alignas(16) SkParams {
     unsigned long long* trace;  // debug: 8 clock stamps per CTA, or null
     int* status;                // set non-zero when a bounded wait gives up, or null
     int chunk, slots;           // units per ring slot, ring slots per warp
-    int debug_skip;             // debug: wait for the copies but skip the arithmetic
     int ptiles;                 // tiles the per-CTA sum buffer holds
 };
 
@@ -256,7 +255,7 @@ struct TokenParams {
     unsigned long long* trace;  // debug: [grid][nphases][TK_TRACE_W] stamps, or null
     int chunk, slots;           // ring geometry: unit records per slot, slots
     unsigned fixed_bytes;       // shared memory in front of the ring (digits, sums, scratch of the other phases)
-    int skip;                   // debug: stream the weights but skip the GEMV arithmetic (results are wrong)
+    int skip;                   // builds with L2_TK_TRACE only: bit 0 no GEMV arithmetic, bit 1 no weight copies (results are wrong)
     // tensor parallelism over peer memory: every rank's pool of tagged activations (same layout everywhere, this
     // rank's own at pool[rank]); a phase that broadcasts stores at the same offset into each of them
     char* pool[8];

@@ -182,7 +182,6 @@ int sk_plan(SkLaunch& L, int sms) {
     slots = std::max(2, std::min<int>(slots, (int)((max_units + su - 1) / su)));
     const int chunk = su;
     if (const char* e = getenv("L2_SK_SLOTS")) slots = std::max(2, std::min(slots, atoi(e)));
-    p.debug_skip = getenv("L2_SK_SKIP") ? 1 : 0;
     p.chunk = chunk;
     p.slots = slots;
     p.ptiles = ptiles;
@@ -557,7 +556,9 @@ static int plan_token(l2_state* s) {
     s->tk.fixed_bytes = (unsigned)fixed;
     s->tk.status = &s->ctl->status;
     s->tk.ctl = s->ctl;
-    s->tk.skip = (getenv("L2_SK_SKIP") ? 1 : 0) | (getenv("L2_SK_NOCOPY") ? 2 : 0);  // debugging: no arithmetic / no weight copies (results are wrong)
+#ifdef L2_TK_TRACE  // builds for timing only: no arithmetic / no weight copies (results are wrong)
+    s->tk.skip = (getenv("L2_SK_SKIP") ? 1 : 0) | (getenv("L2_SK_NOCOPY") ? 2 : 0);
+#endif
     s->tk_smem = fixed + (size_t)slots * sk_slot_bytes(c.group_size, su);
     {
         const int lg = m->opt.poll_limit_log2;

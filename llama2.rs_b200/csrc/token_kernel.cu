@@ -90,7 +90,11 @@ struct Ring {
     uint32_t slot_bytes;
     int SU, NS;
     int* status;
-    int skip;  // debug: consume the slot fills without doing the arithmetic
+#ifdef L2_TK_TRACE
+    int skip;  // see TokenParams
+#else
+    static constexpr int skip = 0;
+#endif
 };
 __device__ __forceinline__ bool ring_aborted(const Ring& R) { return lds_volatile_i32(R.abort_flag) != 0; }
 __device__ __forceinline__ void ring_abort(const Ring& R, int code) {
@@ -168,7 +172,7 @@ __device__ __forceinline__ bool produce_units(const SkParams& P, int NSEG, const
         if (!good) return false;
         const int left = min(SU, n - k * SU);
         if (pstamp && lane == 0) { waited += clock64() - w0; if (k == 0) pstamp[11] = clock64(); pstamp[12] = clock64(); pstamp[13] = waited; }
-        if (r_skip & 2) {  // debug: no copies at all, the consumers multiply whatever the slot holds
+        if (r_skip & 2) {  // no copies at all, the consumers multiply whatever the slot holds
             if (lane == 0) mbar_arrive_u32(r_full + 8u * slot);
         } else {
             if (lane == 0) mbar_expect_tx_u32(r_full + 8u * slot, (uint32_t)left * UB);
@@ -982,7 +986,9 @@ __global__ void __launch_bounds__(TK_BLOCK, 1) token_kernel(const __grid_constan
     R.abort_flag = smem_u32(const_cast<int*>(&abort_flag));
     R.status = tk.status;
     R.zeros = smem_u32(zeros);
+#ifdef L2_TK_TRACE
     R.skip = tk.skip;
+#endif
 
     // ================= producer warp ================================================================
     if (warp == SK_WARPS) {
