@@ -40,12 +40,6 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 // Sum of squares of n floats (n % 4 == 0) over the whole block, the same value in every thread.
 __device__ float block_sum_sq(const float* x, int n, float* scratch /* >= 33 floats */) {
     float s = 0.f;
@@ -72,9 +66,7 @@ __device__ float block_sum_sq(const float* x, int n, float* scratch /* >= 33 flo
 __global__ void __launch_bounds__(256) embed_kernel(const __grid_constant__ EmbedParams p) {
     grid_dependency_wait();
     grid_launch_dependents();
-    const int pos = p.ctl->pos;
     int token = p.ctl->token;
-    if (p.feed_prompt) token = pos == 0 ? 1 : p.prompt[pos - 1];
     if (token < 0 || token >= p.vocab) token = 0;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < p.dim) {
@@ -473,19 +465,6 @@ void launch_scatter(const float* src, int n, float* const* dst, const int* const
     cudaLaunchAttribute attr[1];
     launch_cfg(cfg, attr, dim3((n + 255) / 256), dim3(256), 0, st, pdl);
     cudaLaunchKernelEx(&cfg, scatter_kernel, p);
-}
-
-__global__ void advance_kernel(Ctl* ctl) {
-    grid_dependency_wait();
-    grid_launch_dependents();
-    if (threadIdx.x == 0) ctl->pos = ctl->pos + 1;
-}
-
-void launch_advance(Ctl* ctl, cudaStream_t st, bool pdl) {
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    launch_cfg(cfg, attr, dim3(1), dim3(32), 0, st, pdl);
-    cudaLaunchKernelEx(&cfg, advance_kernel, ctl);
 }
 
 cudaError_t kernels_init() {

@@ -164,17 +164,11 @@ __device__ __forceinline__ float block_reduce_2(float& mx, float sq, float* red 
     return total;
 }
 
-__device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
-    return (uint32_t)(a & 255) | ((uint32_t)(b & 255) << 8) | ((uint32_t)(c & 255) << 16) | ((uint32_t)(d & 255) << 24);
-}
-
 // ---- staging of an activation vector as digits ------------------------------------------------------
 // Thread i owns the 8-input blocks i, i + 512, ...; the first SK_KEEP of them stay in registers
 // between the two passes (max / sum of squares, then digits).
 constexpr int SK_KEEP = 3;
 
-// Loads block `blk` of the segment's vector times its norm weight; with `stats` also folds the block
-// into the running max |v| and sum of x^2.
 // Values that travel from CTA to CTA inside one kernel without a barrier in between are stored as
 // (value, tag) pairs, one 64-bit word each: the reader polls until the tag is the one it expects (the
 // tag names the launch and the phase that writes the value), so no fence, flag or barrier has to
@@ -235,17 +229,12 @@ __device__ __forceinline__ bool load_tagged8(const void* base, size_t index, uin
 }
 
 // Loads block `blk` of the segment's vector times its norm weight; with `stats` also folds the block
-// into the running max |v| and sum of x^2.  tag != 0: the vector is stored as tagged pairs.
-__device__ __forceinline__ void stage_fetch(const SkSeg& sg, int blk, float4& v0, float4& v1, bool stats, float& mx, float& sq,
-                                            uint32_t tag = 0, bool* fail = nullptr) {
+// into the running max |v| and sum of x^2.
+__device__ __forceinline__ void stage_fetch(const SkSeg& sg, int blk, float4& v0, float4& v1, bool stats, float& mx, float& sq) {
     const float4* x4 = reinterpret_cast<const float4*>(sg.x);
     const float4* n4 = reinterpret_cast<const float4*>(sg.nw);
-    if (tag) {
-        if (!load_tagged8(sg.x, (size_t)blk * 8, tag, v0, v1) && fail) *fail = true;
-    } else {
-        v0 = __ldcg(x4 + 2 * blk);  // written by other CTAs shortly before: read at the L2, never from a stale L1 line
-        v1 = __ldcg(x4 + 2 * blk + 1);
-    }
+    v0 = __ldcg(x4 + 2 * blk);  // written by other CTAs shortly before: read at the L2, never from a stale L1 line
+    v1 = __ldcg(x4 + 2 * blk + 1);
     if (stats) sq += v0.x * v0.x + v0.y * v0.y + v0.z * v0.z + v0.w * v0.w + v1.x * v1.x + v1.y * v1.y + v1.z * v1.z + v1.w * v1.w;
     if (sg.nw) {
         const float4 w0 = __ldg(n4 + 2 * blk), w1 = __ldg(n4 + 2 * blk + 1);
@@ -313,8 +302,7 @@ __device__ __forceinline__ void stage_emit(uint8_t* digits, int* ss, int stride,
 // Returns (in every thread) the factor the integer result has to be multiplied with: NaN for a vector that holds a NaN or an
 // infinity, which has no digits and makes every output NaN.
 template <int W>
-__device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digits, int* ss, float* red, unsigned long long* dbg = nullptr,
-                              uint32_t tag = 0, bool* fail = nullptr) {
+__device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digits, int* ss, float* red) {
     const int nblk = in / 8;
     float mx = 0.f, sq = 0.f;
     float4 keep[SK_KEEP][2];
@@ -323,15 +311,13 @@ __device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digit
 #pragma unroll
     for (int k = 0; k < SK_KEEP; k++) {
         const int blk = threadIdx.x + k * SK_THREADS;
-        if (blk < nblk) stage_fetch(sg, blk, keep[k][0], keep[k][1], true, mx, sq, tag, fail);
+        if (blk < nblk) stage_fetch(sg, blk, keep[k][0], keep[k][1], true, mx, sq);
     }
     for (int blk = threadIdx.x + SK_KEEP * SK_THREADS; blk < nblk; blk += SK_THREADS) {
         float4 a, b;
-        stage_fetch(sg, blk, a, b, true, mx, sq, tag, fail);
+        stage_fetch(sg, blk, a, b, true, mx, sq);
     }
-    if (dbg && threadIdx.x == 0) dbg[0] = clock64() + (mx > 1e30f ? 1 : 0);
     const float total = block_reduce_2(mx, sq, red);
-    if (dbg && threadIdx.x == 0) dbg[1] = clock64();
     const float rs = sg.nw ? 1.0f / sqrtf(total / (float)in + eps) : 1.0f;  // src/models.rs:58-60
     const float P = stage_scale(mx);
     const int stride = in + 16;
@@ -351,51 +337,11 @@ __device__ float stage_digits(const SkSeg& sg, int in, float eps, uint8_t* digit
             const bool valid = blk < nblk;
             float4 a = zero4, b = zero4;
             float m2 = 0.f, s2 = 0.f;
-            if (valid) stage_fetch(sg, blk, a, b, false, m2, s2, tag, fail);
+            if (valid) stage_fetch(sg, blk, a, b, false, m2, s2);
             stage_emit<W>(digits, ss, stride, blk, a, b, valid, P);
         }
     }
-    if (dbg && threadIdx.x == 0) dbg[2] = clock64();
     return mx < INFINITY ? rs / P : NAN;
-}
-
-// Two segments whose vectors are two orderings of the same values (w1 and w3 read the same x, each
-// in its own K order, with the norm weight ordered alike): the maximum and the sum of squares are
-// taken once, from the first, and both are turned into digits with the same scale.  Needs
-// in <= 2 * 8 * SK_THREADS.  Returns the common output factor.
-template <int W>
-__device__ float stage_digits_pair(const SkSeg& sa, const SkSeg& sb, int in, float eps, uint8_t* da, uint8_t* db, int* ssa, int* ssb, float* red,
-                                   unsigned long long* dbg = nullptr, uint32_t tag = 0, bool* fail = nullptr) {
-    const int nblk = in / 8;
-    float mx = 0.f, sq = 0.f, m2 = 0.f, s2 = 0.f;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 ka[2][2], kb[2][2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        ka[k][0] = ka[k][1] = kb[k][0] = kb[k][1] = zero4;
-        const int blk = threadIdx.x + k * SK_THREADS;
-        if (blk < nblk) {
-            stage_fetch(sa, blk, ka[k][0], ka[k][1], true, mx, sq, tag, fail);
-            stage_fetch(sb, blk, kb[k][0], kb[k][1], false, m2, s2, tag, fail);
-        }
-    }
-    if (dbg && threadIdx.x == 0) dbg[0] = clock64() + (mx > 1e30f ? 1 : 0);
-    const float total = block_reduce_2(mx, sq, red);
-    if (dbg && threadIdx.x == 0) dbg[1] = clock64();
-    const float rs = sa.nw ? 1.0f / sqrtf(total / (float)in + eps) : 1.0f;
-    const float P = stage_scale(mx);
-    const int stride = in + 16;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int blk = threadIdx.x + k * SK_THREADS;
-        if ((blk & ~31) < nblk) {
-            const bool valid = blk < nblk;
-            stage_emit<W>(da, ssa, stride, blk, ka[k][0], ka[k][1], valid, P);
-            stage_emit<W>(db, ssb, stride, blk, kb[k][0], kb[k][1], valid, P);
-        }
-    }
-    if (dbg && threadIdx.x == 0) dbg[2] = clock64();
-    return rs / P;
 }
 
 // ---- one-pass staging with one exponent per quantisation group (token kernel) --------------------

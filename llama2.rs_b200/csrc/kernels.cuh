@@ -174,12 +174,10 @@ struct TpGatherParams {
 struct EmbedParams {
     const float* table;   // [VOCAB][DIM]
     const Ctl* ctl;
-    const int* prompt;    // device copy of the prompt ids
     float* x;             // residual stream, natural order
     float* sdst[3];
     const int* sidx[3];
     int dim, nscatter;
-    int feed_prompt;      // 1: token = START at pos 0 else prompt[pos-1] (src/inference.rs:29-35)
     int vocab;
 };
 
@@ -229,7 +227,7 @@ struct SelectParams {
 // A token is a list of phases; all CTAs run every phase.  A phase polls the tagged values of the
 // phases it depends on; only where barrier_after is set do the CTAs meet at a grid-wide barrier.
 // A phase record is what the stand-alone kernel of the same name takes as parameters.
-enum : int { PH_EMBED = 0, PH_GEMV1, PH_GEMV2, PH_ATTN, PH_CLS, PH_SELECT, PH_ADVANCE };
+enum : int { PH_EMBED = 0, PH_GEMV1, PH_GEMV2, PH_ATTN, PH_CLS, PH_SELECT };
 
 struct alignas(16) PhaseRec {
     int type;
@@ -240,7 +238,7 @@ struct alignas(16) PhaseRec {
         AttnParams at;
         EmbedParams em;
         ClsParams cl;
-        SelectParams se; // PH_SELECT; PH_ADVANCE uses se.ctl only
+        SelectParams se; // PH_SELECT
     } u;
 };
 
@@ -253,7 +251,7 @@ struct TokenParams {
     int* status;                // set non-zero when a bounded wait gives up
     const Ctl* ctl;             // loop state: the position of this token
     unsigned long long* trace;  // debug: [grid][nphases][TK_TRACE_W] stamps, or null
-    int chunk, slots;           // ring geometry: unit records per slot, slots
+    int slots;                  // slots of the weight ring
     unsigned fixed_bytes;       // shared memory in front of the ring (digits, sums, scratch of the other phases)
     int skip;                   // builds with L2_TK_TRACE only: bit 0 no GEMV arithmetic, bit 1 no weight copies (results are wrong)
     // tensor parallelism over peer memory: every rank's pool of tagged activations (same layout everywhere, this
@@ -296,7 +294,6 @@ extern unsigned long long* g_sk_trace;  // device buffer for SkParams::trace whe
 void launch_attn(const AttnParams& p, cudaStream_t st, bool pdl);
 void launch_cls(const ClsParams& p, int grid, cudaStream_t st, bool pdl);
 void launch_select(const SelectParams& p, cudaStream_t st, bool pdl);
-void launch_advance(Ctl* ctl, cudaStream_t st, bool pdl);
 // dst_i[idx_i[j]] = src[j] for j < n and up to three destinations (copies of a vector in consumers' K orders)
 void launch_scatter(const float* src, int n, float* const* dst, const int* const* idx, int ndst, cudaStream_t st, bool pdl);
 cudaError_t kernels_init();  // opt-in shared memory sizes; call once per device

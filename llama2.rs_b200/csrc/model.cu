@@ -456,12 +456,12 @@ static ClsParams classifier_params(l2_state* s) {
 
 static void launch_classifier(l2_state* s, cudaStream_t st, bool pdl) { launch_cls(classifier_params(s), s->m->sms * 2, st, pdl); }
 
-static EmbedParams embed_params(l2_state* s, int kind) {
+static EmbedParams embed_params(l2_state* s) {
     l2_model* m = s->m;
     const l2_config& c = m->shape.c;
     EmbedParams e{};
-    e.table = m->tok_emb; e.ctl = s->ctl; e.prompt = s->prompt; e.x = s->x;
-    e.dim = c.dim; e.vocab = c.vocab_size; e.feed_prompt = kind == G_FEED;
+    e.table = m->tok_emb; e.ctl = s->ctl; e.x = s->x;
+    e.dim = c.dim; e.vocab = c.vocab_size;
     set_scatter3(e.sdst, e.sidx, &e.nscatter, s, &m->layers[0]);
     return e;
 }
@@ -551,7 +551,6 @@ static int plan_token(l2_state* s) {
     if (slots < 2) return fail(L2_EINVAL, "the token kernel needs %zu bytes of shared memory before its weight ring", fixed);
     if (const char* e = getenv("L2_SK_SLOTS")) slots = std::max(2, std::min(slots, atoi(e)));
     s->tk = TokenParams{};
-    s->tk.chunk = su;
     s->tk.slots = slots;
     s->tk.fixed_bytes = (unsigned)fixed;
     s->tk.status = &s->ctl->status;
@@ -616,7 +615,7 @@ static int build_phase_table(l2_state* s, int kind) {
     bool bad = false;
     auto must = [&](float* p) { if (!p) bad = true; return p; };
     {
-        EmbedParams e = embed_params(s, kind);
+        EmbedParams e = embed_params(s);
         e.x = must(tg(e.x));
         e.nscatter = 0;
         add(PH_EMBED).u.em = e;
@@ -707,8 +706,6 @@ static int build_phase_table(l2_state* s, int kind) {
         if (direct && s->t_logits) { sp.tagged = s->t_logits; sp.tagged_phase = cls_phase_index; }
         sp.collect_only = kind == G_FWD_CLS ? 1 : 0;
         add(PH_SELECT).u.se = sp;
-    } else if (kind == G_FEED) {
-        add(PH_ADVANCE).u.se.ctl = s->ctl;
     }
     if (bad) return fail(L2_EINVAL, "token kernel: an activation buffer of the launch plan has no tagged counterpart");
     if (t.size() >= 1024) return fail(L2_EINVAL, "token kernel: %zu phases do not fit the 10-bit phase field of a tag", t.size());
@@ -734,7 +731,7 @@ static int enqueue_forward(l2_state* s, int kind, cudaStream_t st) {
     if (token_path(s)) return enqueue_token(s, kind, st);
     const bool pdl = m->use_pdl;
     const int L = c.n_layers, D = c.dim;
-    launch_embed(embed_params(s, kind), st, false);  // first node of the token: plain stream order
+    launch_embed(embed_params(s), st, false);  // first node of the token: plain stream order
     const int T = m->tp_world;
     for (int l = 0; l < L; l++) {
         const DevLayer& y = m->layers[l];
@@ -773,8 +770,6 @@ static int enqueue_forward(l2_state* s, int kind, cudaStream_t st) {
         SelectParams sp{};
         sp.logits = s->logits; sp.ctl = s->ctl; sp.prompt = s->prompt; sp.out_tokens = s->out_tokens; sp.vocab = c.vocab_size;
         launch_select(sp, st, pdl);
-    } else if (kind == G_FEED) {
-        launch_advance(s->ctl, st, pdl);
     }
     L2_CUDA(cudaGetLastError());
     return L2_OK;
@@ -787,7 +782,7 @@ static int nodes_per_forward(const l2_state* s, int kind) {
     int n = 1 + 5 * L;
     if (m->tp_world > 1) n += 3 * L - 1;  // the copies into the consumers' K orders after each all-gather
     if (kind == G_DECODE) n += 2;
-    if (kind == G_FWD_CLS || kind == G_FEED) n += 1;
+    if (kind == G_FWD_CLS) n += 1;
     return n;
 }
 

@@ -67,7 +67,7 @@ struct BatchBuffers {
     std::vector<void*> allocs;
 };
 
-enum GraphKind : int { G_DECODE = 0, G_FEED, G_FWD_CLS, G_FWD, G_COUNT };
+enum GraphKind : int { G_DECODE = 0, G_FWD_CLS, G_FWD, G_COUNT };
 
 }  // namespace l2
 
@@ -123,8 +123,8 @@ struct l2_state {
     int failed_status = 0;              // device status of a launch that gave up; cleared by l2_state_reset
     std::vector<l2::SkLaunch> plans;     // [layer][4] GEMV launches, planned once
     l2::SkParams* d_plans = nullptr;     // their parameter records on the device
-    l2::PhaseRec* d_phases[l2::G_COUNT] = {nullptr, nullptr, nullptr, nullptr};  // phase tables of the token kernel
-    int n_phases[l2::G_COUNT] = {0, 0, 0, 0};
+    l2::PhaseRec* d_phases[l2::G_COUNT] = {};  // phase tables of the token kernel
+    int n_phases[l2::G_COUNT] = {};
     l2::TokenParams tk{};                // ring geometry and barrier of the token kernel
     size_t tk_smem = 0;
     // activations of the token kernel as (value, tag) pairs, 8 bytes per element (see token_kernel.cu)
@@ -135,8 +135,8 @@ struct l2_state {
     int tk_max_split = 1;
     unsigned long long* tk_trace = nullptr;
     size_t tk_trace_count = 0;
-    cudaGraphExec_t graphs[l2::G_COUNT] = {nullptr, nullptr, nullptr, nullptr};
-    int graph_nodes[l2::G_COUNT] = {0, 0, 0, 0};
+    cudaGraphExec_t graphs[l2::G_COUNT] = {};
+    int graph_nodes[l2::G_COUNT] = {};
     std::vector<void*> allocs;
 };
 
@@ -180,6 +180,5 @@ int gemm_batched(const DevQ& q, const float* x, int M, uint8_t* img, float* osc,
 size_t part_floats(const int* rows, int n, int in, int gs, int cap, int sms);
 void free_batch(l2_model* m);
 int reserve_batch(l2_model* m, int M, int* limit);
-int dev_alloc_bytes(void** p, size_t bytes, std::vector<void*>& allocs);
 void sk_set_matrix(SkJob& j, int seg, const DevQ& q, const float* x, const float* nw);
 }  // namespace l2

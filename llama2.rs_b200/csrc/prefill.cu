@@ -7,12 +7,6 @@
 
 namespace l2 {
 
-int dev_alloc_bytes(void** p, size_t bytes, std::vector<void*>& allocs) {
-    L2_CUDA(cudaMalloc(p, bytes ? bytes : 16));
-    allocs.push_back(*p);
-    return L2_OK;
-}
-
 void tc_set_matrix(TcParams& t, int i, const DevQ& q, const uint8_t* img, float* out, int ldo, float* part) {
     TcMat& m = t.mat[i];
     m.rec = q.rec; m.img = img; m.out = out; m.part = part;
