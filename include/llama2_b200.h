@@ -182,7 +182,8 @@ int l2_generate_ids(l2_model* m, const int32_t* prompt, int n_prompt, int steps,
 int l2_qlinear_create(int in, int out, int group_size, const int32_t* qweight, const int32_t* qzeros,
                       const float* scales, const int32_t* g_index, int device, l2_qlinear** h);
 /* x [B][IN] -> xout [B][OUT], host f32 buffers; copies to and from the device inside the call.
- * A row that holds a NaN or an infinity gives a row of NaN; the other rows are not touched by it.
+ * A row that holds a NaN or an infinity gives a row of NaN; the other rows are not touched by it.  No input is resolved finer than
+ * a multiple of 2^-100.
  * L2_ESTATUS: a bounded wait on the device gave up, in this call or in an earlier l2_qlinear_matvec_dev on the handle
  * (which cannot report it itself); reported by one call, the next starts clean. */
 int l2_qlinear_matvec(l2_qlinear* h, const float* x, float* xout, int B);

@@ -14,9 +14,10 @@
 // pairs that the reader polls (see gemv_device.cuh); one grid barrier per token remains, between the
 // classifier and the selection of the next token, which reads every logit.
 //
-// The kernel is bound by instruction issue and by the latency of each exchange, not by HBM: every
-// phase's code runs once per layer, so it is kept small (one GEMV phase for all four projections,
-// no unrolled polling loops) and each exchange is arranged so that everything that does not depend
+// The kernel is bound by latencies: by each exchange between phases, and in the main loops by what one
+// slot fill takes a warp from its barrier to its last sum (see gemv_phase); HBM adds a fifth to a third to the
+// longer main loops.  Every phase's code runs once per layer, so it is kept small (one GEMV phase for all four
+// projections, no unrolled polling loops) and each exchange is arranged so that everything that does not depend
 // on the awaited values (norm weights, scatter positions, K/V rows) is already in flight.
 //
 // Waits are bounded everywhere (mbarriers, tag polls, the grid barrier, the producer's wait for a
@@ -274,8 +275,10 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
     }
 
     // ---- main loop.  In every slot fill this warp owns units 2*warp and 2*warp + 1; unit u of the CTA is group
-    // u % Gs of tile u / Gs (the groups of w1 and of w3 of a tile follow one another).  The loop is bound by
-    // instruction issue (16 warps run it on 4 schedulers), so it is straight-line code on 32-bit shared-space
+    // u % Gs of tile u / Gs (the groups of w1 and of w3 of a tile follow one another).  Without the weight copies a fill takes 1100
+    // to 1250 clocks, of 35 KB (group of 128) as of 19 KB (64): that is the chain a warp walks through it (barrier, operands,
+    // MMAs, scale step, release; the four warps of a scheduler issue some 440 instructions meanwhile).  With them w1/w3 take 1404 (7B),
+    // 1616 (13B) and 1390 clocks a fill (70B shapes).  So it is straight-line code on 32-bit shared-space
     // addresses, and the pair shares one set of accumulators: the four digits of the first unit are columns 0-3 of the
     // MMAs, those of the second columns 4-7 (the other unit's columns multiply a block of zeros), so that lanes t < 2 hold
     // the first unit's sums and lanes t >= 2 the second's, and the scale / zero-point step runs once for both.  Low and
@@ -353,8 +356,8 @@ __device__ L2_TK_PHASE_INLINE bool gemv_phase(const TokenParams& tk, const SkPar
             const uint32_t s0 = lds32(m_lane + so), s1 = lds32(m_lane + so + 32);
             const uint2 zz = lds64(z_lane + so);
             const uint2 g = lds64(sp_lane + 16u * (uint32_t)fs);  // {digit sums of this lane's columns, their factor}
-            // Four independent MMAs, then four that add to them: an integer mma.sync that depends on the previous one of its
-            // warp occupies the tensor pipe about four times as long as one that follows an independent one.
+            // Four independent MMAs, then four that add to them.  (One warp's dependent MMAs follow each other after 21 clocks instead
+            // of 11; with the four warps that a scheduler has here it is 8.3 clocks an MMA either way.)
             int c[4];
             if constexpr (W == 1) {
                 int e[4];

@@ -3,13 +3,16 @@
 Needs a library built with the stamps compiled in (they cost registers, so the normal build leaves them out):
 
     L2_TK_TRACE=1 python llama2.rs_b200/build.py --force
-    python llama2.rs_b200/token_trace.py [7B|13B|70B] [group size] [context] [layers]
+    python llama2.rs_b200/token_trace.py [7B|13B|70B|dim,hidden,heads,kv heads,vocabulary] [group size] [context] [layers]
     python llama2.rs_b200/build.py --force        # back to the normal build
 
 Runs `context` positions, then one traced token (l2_debug_token_trace), and prints per kind of phase the mean over CTAs
 and layers of: waiting for the tagged inputs, scatter into K order + CTA barrier, digit emission + statistics, main loop,
 epilogue, and the gap to the start of the next phase; for the attention phase: q/k/v wait + RoPE, scores, values, merge.
-Times are SM cycles divided by the SM clock read from the run (globaltimer stamps give the phase spans).
+Times are SM cycles divided by the SM clock read from the run (globaltimer stamps give the phase spans).  A slot fill is 32 unit records.
+
+In that build two variables leave work out of the token kernel, to see what the rest takes (results are wrong): L2_SK_NOCOPY=1 the weight
+copies, L2_SK_SKIP=1 the arithmetic of the main loops.
 """
 import ctypes as C
 import os
@@ -27,7 +30,12 @@ def main():
     name = sys.argv[1] if len(sys.argv) > 1 else "7B"
     gs = int(sys.argv[2]) if len(sys.argv) > 2 else 128
     ctx = int(sys.argv[3]) if len(sys.argv) > 3 else 160
-    cfg = l2.preset_config(name, gs)
+    if "," in name:
+        cfg = l2.Config()
+        cfg.dim, cfg.hidden_dim, cfg.n_heads, cfg.n_kv_heads, cfg.vocab_size = (int(v) for v in name.split(","))
+        cfg.n_layers, cfg.seq_len, cfg.group_size = 8, max(512, ctx + 1), gs
+    else:
+        cfg = l2.preset_config(name, gs)
     if len(sys.argv) > 4:
         cfg.n_layers = int(sys.argv[4])
     import torch
@@ -55,7 +63,7 @@ def main():
     print("%s g%d, %d layers, context %d: token %.1f us, layer %.2f us, classifier %.1f us, SM clock %.0f MHz" %
           (name, gs, L, ctx, total, layer, (t[:, nph - 2, 5].max() - t[:, nph - 2, 4].min()) / 1e3, cyc))
     print("GEMV phases, us (mean over CTAs and layers): span = first CTA's start -> last CTA's end")
-    print("phase   span | wait inputs  scatter+sync  digits+stats  main loop  epilogue  to next phase | start spread  end spread")
+    print("phase   span | wait inputs  scatter+sync  digits+stats  main loop  epilogue  to next phase | start spread  end spread | CTAs  fills  clocks a fill")
     for off, n in ((0, "qkv"), (2, "wo"), (3, "w13"), (4, "w2")):
         rows = []
         for l in range(lo, hi):
@@ -68,9 +76,10 @@ def main():
             emit = (r[:, 1] - r[:, 22]) if natural else (r[:, 1] - r[:, 21])
             rows.append([(r[:, 5].max() - r[:, 4].min()) / 1e3, np.mean(r[:, 16] - r[:, 0] + polled) / cyc, np.mean(sync) / cyc, np.mean(emit) / cyc,
                          np.mean(r[:, 2] - r[:, 1]) / cyc, np.mean(r[:, 7] - r[:, 2]) / cyc, np.mean(nxt[:, 0] - r[:, 7]) / cyc,
-                         (r[:, 4].max() - r[:, 4].min()) / 1e3, (r[:, 5].max() - r[:, 5].min()) / 1e3])
+                         (r[:, 4].max() - r[:, 4].min()) / 1e3, (r[:, 5].max() - r[:, 5].min()) / 1e3,
+                         len(r), np.mean(r[:, 9]), np.sum(r[:, 2] - r[:, 1]) / np.sum(r[:, 9])])
         a = np.mean(np.array(rows), axis=0)
-        print("%-5s %6.2f | %11.2f  %12.2f  %12.2f  %9.2f  %8.2f  %13.2f | %12.2f  %10.2f" % ((n,) + tuple(a)))
+        print("%-5s %6.2f | %11.2f  %12.2f  %12.2f  %9.2f  %8.2f  %13.2f | %12.2f  %10.2f | %4.0f  %5.1f  %13.0f" % ((n,) + tuple(a)))
     print("attention phase, us (CTAs that had an item): span | items | q,k,v wait + RoPE  scores  values  partials + merge")
     rows = []
     for l in range(lo, hi):
