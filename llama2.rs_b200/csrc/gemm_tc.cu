@@ -28,8 +28,9 @@
 //      An accumulator is away from its commit until the drain has read it: with two, that chain bounded the kernel, so the A slots are
 //      one per weight tile and D has three.  Clocks of a step of 256 rows x 64 tokens x 128 inputs (group 64), by stamps in the issuing
 //      warp: 1406 issue (16 MMAs, 1024 of tensor time), 512 waits for an accumulator, 236 for B, 162 for A, 570 between, 2888 in all.
-//      That warp's own work is not the bound: with a second issuing warp, one per weight tile, 8192 x 28672 at 256 tokens took 297 us
-//      instead of 293.
+//      What bounds a step is the hand-overs between the roles (waits, fences, commits, arrivals), not the work between them: with the tensor-memory
+//      stores of A, the loads of D and all MMAs but the first of a group left out together, and every hand-over kept, 8192 x 28672 at 256
+//      tokens takes as long (243 us, back to back), and so it does with each left out alone or with a second issuing warp.
 //
 // Roles (they meet only through mbarriers):
 //   warps 0-7    loaders, four warps per weight tile: a thread turns the 128 weights of one row into f16 (per 8 weights: a shift, four
